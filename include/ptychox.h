@@ -450,6 +450,28 @@ int ptx_reg_upsampled_peak(const float* cross_power, int batch, int rows, int co
                            const int* row_center, const int* col_center, int* peak_rc, double* peak_cc,
                            void* workspace, size_t workspace_bytes, void* stream);
 
+/* The passes around the transforms of the initial estimate (dftregistration.m:90-101), peak of
+ * the cross-correlation upsampled twice.  Images are [batch][rows][cols] complex64 spectra.
+ *   ptx_reg_cross_power    spec1 (batch1 = 1 or batch images) and spec2 -> `padded`
+ *                          [batch][rows][2 cols], spec1 .* conj(spec2) with each row zero-padded
+ *                          (FTpad, :189-224), and `cross_power` [batch][rows][cols], its conjugate
+ *   ptx_reg_pad_transpose  [batch][rows][2 cols] -> [batch][2 cols][2 rows], transposed and
+ *                          zero-padded along the rows
+ *   ptx_reg_estimate       `correlation` [batch][2 cols][2 rows] (unnormalised inverse transform
+ *                          of both axes) -> its first maximum in column-major order: `half_rc`
+ *                          (int32 [batch][2], signed half pixels), the centres round(shift usfac)
+ *                          for ptx_reg_upsampled_peak (int32 [batch] each), and the correlation
+ *                          there (interleaved complex128 [batch])
+ *   ptx_reg_energy         sum |spec|^2 of each image in FP64 */
+int ptx_reg_cross_power(const float* spec1, int batch1, const float* spec2, int batch, int rows, int cols,
+                        float* padded, float* cross_power, void* stream);
+int ptx_reg_pad_transpose(const float* in, int batch, int rows, int cols, float* out, void* stream);
+size_t ptx_reg_estimate_workspace_bytes(int batch, int rows, int cols);
+int ptx_reg_estimate(const float* correlation, int batch, int rows, int cols, int usfac, int* half_rc,
+                     int* row_center, int* col_center, double* peak_cc, void* workspace, size_t workspace_bytes,
+                     void* stream);
+int ptx_reg_energy(const float* spec, int batch, int rows, int cols, double* energy, void* stream);
+
 #ifdef __cplusplus
 }  /* extern "C" */
 #endif

@@ -79,6 +79,11 @@ SIGNATURES: dict[str, tuple] = {
     "ptx_status_code": (_i, [C.c_uint]),
     "ptx_reg_workspace_bytes": (_sz, [_i, _i, _i, _i]),
     "ptx_reg_upsampled_peak": (_i, [_p, _i, _i, _i, _i, _p, _p, _p, _p, _p, _sz, _p]),
+    "ptx_reg_cross_power": (_i, [_p, _i, _p, _i, _i, _i, _p, _p, _p]),
+    "ptx_reg_pad_transpose": (_i, [_p, _i, _i, _i, _p, _p]),
+    "ptx_reg_estimate_workspace_bytes": (_sz, [_i, _i, _i]),
+    "ptx_reg_estimate": (_i, [_p, _i, _i, _i, _i, _p, _p, _p, _p, _p, _sz, _p]),
+    "ptx_reg_energy": (_i, [_p, _i, _i, _i, _p, _p]),
     "ptx_server_create": (_i, [_i, _sz, _i, _p]),
     "ptx_server_submit": (_i, [_p, _p, _p]),
     "ptx_server_poll": (_i, [_p, C.c_longlong, _p, _p, _p, _p, _p]),

@@ -395,6 +395,164 @@ __global__ void __launch_bounds__(32) reg_peak_kernel(const PeakCand* __restrict
   }
 }
 
+// ---- the initial estimate: peak of the twice-upsampled cross-correlation -----------------------
+// Frequency k of a line of n bins in the line zero-padded to 2 n (FTpad,
+// dftregistration.m:189-224): the non-negative ones keep their bins, the negative ones move to
+// the end.
+__device__ __forceinline__ int unpadded_bin(int c, int n) {
+  const int half = n - n / 2;
+  return c < half ? c : (c >= n + half ? c - n : -1);
+}
+
+// One pass from the two spectra to the product spec1 conj(spec2), rows zero-padded to 2 cols
+// (what the row transform reads), and the cross-power conj(spec1) spec2 the refinement reads.
+// HBM-bound: 8 B read (spec1 of a tracked stack is one image, resident in L2), 24 B written.
+__global__ void __launch_bounds__(256) reg_cross_power_kernel(const float2* __restrict__ s1, bool one,
+                                                              const float2* __restrict__ s2, int rows, int cols,
+                                                              float2* __restrict__ padded, float2* __restrict__ q) {
+  const long long row = (long long)blockIdx.y * rows + blockIdx.x;
+  const float2* a = s1 + (one ? (long long)blockIdx.x : row) * cols;
+  const float2* b = s2 + row * cols;
+  for (int c = threadIdx.x; c < 2 * cols; c += blockDim.x) {
+    const int k = unpadded_bin(c, cols);
+    float2 v = make_float2(0.f, 0.f);
+    if (k >= 0) {
+      const float2 z = cmulc(b[k], a[k]);
+      q[row * cols + k] = z;
+      v = cconj(z);
+    }
+    padded[row * 2 * cols + c] = v;
+  }
+}
+
+// [batch][rows][2 cols] -> [batch][2 cols][2 rows]: transposed, the rows zero-padded, so that
+// the second transform again runs along contiguous lines (and the transform along the rows is
+// taken over the rows that are not zero only).  32 x 32 tiles through shared memory.
+__global__ void __launch_bounds__(256) reg_pad_transpose_kernel(const float2* __restrict__ in, int rows, int cols,
+                                                                float2* __restrict__ out) {
+  __shared__ float2 tile[32][33];
+  const int xtiles = (2 * cols + 31) / 32;
+  const int x0 = static_cast<int>(blockIdx.x % xtiles) * 32, y0 = static_cast<int>(blockIdx.x / xtiles) * 32;
+  const int lx = threadIdx.x % 32, ly = threadIdx.x / 32;
+  const float2* ib = in + (size_t)blockIdx.y * rows * 2 * cols;
+  float2* ob = out + (size_t)blockIdx.y * 4 * rows * cols;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int y = y0 + ly + 8 * i, x = x0 + lx;
+    const int r = y < 2 * rows ? unpadded_bin(y, rows) : -1;
+    tile[ly + 8 * i][lx] = r >= 0 && x < 2 * cols ? ib[(size_t)r * 2 * cols + x] : make_float2(0.f, 0.f);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int x = x0 + ly + 8 * i, y = y0 + lx;
+    if (x < 2 * cols && y < 2 * rows) ob[(size_t)x * 2 * rows + y] = tile[lx][ly + 8 * i];
+  }
+}
+
+constexpr int kCorrThreads = 256;
+constexpr int kCorrChunk = 1 << 15;  // correlation values per CTA
+
+// Peak candidates of chunks of |corr[b]|, `count` values in column-major order.  A value with
+// an infinite part has magnitude infinity, and a NaN beats every number (as a maximum over the
+// magnitudes would have it); |.|^2 of FP32 values cannot reach the two stand-ins in FP64.
+__global__ void __launch_bounds__(kCorrThreads) reg_corr_peak_kernel(const float2* __restrict__ corr, long long count,
+                                                                     PeakCand* __restrict__ cand) {
+  constexpr double kInfinite = 1e300, kNan = 1e301;
+  __shared__ PeakCand best_s[kCorrThreads / 32];
+  const float2* cb = corr + (size_t)blockIdx.y * count;
+  const long long l1 = min(count, ((long long)blockIdx.x + 1) * kCorrChunk);
+  PeakCand best = no_peak();
+#pragma unroll 4
+  for (long long l = (long long)blockIdx.x * kCorrChunk + threadIdx.x; l < l1; l += kCorrThreads) {
+    const float2 z = cb[l];
+    const double x = z.x, y = z.y;
+    double m = x * x + y * y;
+    if (!(m < kInfinite)) m = isinf(z.x) || isinf(z.y) ? kInfinite : kNan;
+    if (m > best.m) {  // l increases per thread, so the thread's first maximum is kept
+      best.m = m;
+      best.at = l;
+      best.z = make_double2(x, y);
+    }
+  }
+  best = warp_best(best);
+  if ((threadIdx.x & 31) == 0) best_s[threadIdx.x >> 5] = best;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    best = warp_best(threadIdx.x < kCorrThreads / 32 ? best_s[threadIdx.x] : no_peak());
+    if (threadIdx.x == 0) cand[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = best;
+  }
+}
+
+// From an image's candidates: the peak in half pixels (signed), the refinement's centres
+// round(shift usfac) (halves away from zero, MATLAB's round) and the correlation there.
+__global__ void __launch_bounds__(32) reg_estimate_kernel(const PeakCand* __restrict__ cand, int count, int rows,
+                                                          int cols, int usfac, int* __restrict__ half_rc,
+                                                          int* __restrict__ row_center, int* __restrict__ col_center,
+                                                          double2* __restrict__ peak_cc) {
+  const int b = blockIdx.x;
+  PeakCand best = no_peak();
+  for (int i = threadIdx.x; i < count; i += 32) {
+    const PeakCand x = cand[(size_t)b * count + i];
+    if (better(x, best)) best = x;
+  }
+  best = warp_best(best);
+  if (threadIdx.x == 0) {
+    int r = static_cast<int>(best.at % (2 * rows)), c = static_cast<int>(best.at / (2 * rows));
+    if (r >= rows) r -= 2 * rows;
+    if (c >= cols) c -= 2 * cols;
+    half_rc[2 * b] = r;
+    half_rc[2 * b + 1] = c;
+    auto centre = [&](int half) {
+      const double v = 0.5 * half * usfac, a = floor(fabs(v) + 0.5);
+      return static_cast<int>(v < 0.0 ? -a : a);
+    };
+    row_center[b] = centre(r);
+    col_center[b] = centre(c);
+    peak_cc[b] = best.z;
+  }
+}
+
+// sum |spec[b]|^2 in FP64, one CTA per image (the same order of summation on every call)
+__global__ void __launch_bounds__(1024) reg_energy_kernel(const float2* __restrict__ spec, long long count,
+                                                          double* __restrict__ out) {
+  __shared__ double part[32];
+  const float2* sb = spec + (size_t)blockIdx.x * count;
+  double s = 0.0;
+#pragma unroll 4
+  for (long long i = threadIdx.x; i < count; i += 1024) {
+    const double x = sb[i].x, y = sb[i].y;
+    s = fma(x, x, fma(y, y, s));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    s = part[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) out[blockIdx.x] = s;
+  }
+}
+
+int corr_chunks(int rows, int cols) {
+  return static_cast<int>((4LL * rows * cols + kCorrChunk - 1) / kCorrChunk);
+}
+
+// Shape checks shared by the entry points of the initial estimate.
+int reg_check_stack(int batch, int rows, int cols) {
+  if (batch < 0 || rows <= 0 || cols <= 0) return set_error(PTX_ERR_INVALID_ARGUMENT, "non-positive shape");
+  if (rows > (1 << 29) || cols > (1 << 29)) return set_error(PTX_ERR_UNSUPPORTED_SIZE, "image side above 2^29");
+  return PTX_OK;
+}
+
+// f(first image, images) over slabs of a batch that fit a grid dimension
+template <typename F>
+void for_slabs(int batch, F&& f) {
+  for (int b0 = 0; b0 < batch; b0 += 65535) f((size_t)b0, std::min(65535, batch - b0));
+}
+
 int reg_out_size(int usfac) { return (3 * usfac + 1) / 2; }  // ceil(1.5 usfac)
 
 // Workspace of a call: the shared tables, then per image the phases, its row blocks' shares of M
@@ -493,6 +651,87 @@ int ptx_reg_upsampled_peak(const float* cross_power, int batch, int rows, int co
   reg_peak_kernel<<<batch, 32, 0, s>>>(cand, l.rblocks * splits, n, peak_rc, reinterpret_cast<double2*>(peak_cc));
   prof_end(kMiscKernel, s);
   return cuda_status(cudaGetLastError(), "ptx_reg_upsampled_peak launch");
+}
+
+int ptx_reg_cross_power(const float* spec1, int batch1, const float* spec2, int batch, int rows, int cols,
+                        float* padded, float* cross_power, void* stream) {
+  if (int st = reg_check_stack(batch, rows, cols)) return st;
+  if (batch1 != 1 && batch1 != batch) return set_error(PTX_ERR_INVALID_ARGUMENT, "spec1 holds 1 or %d images", batch);
+  if (batch == 0) return PTX_OK;
+  if (!spec1 || !spec2 || !padded || !cross_power) return set_error(PTX_ERR_INVALID_ARGUMENT, "null pointer argument");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  prof_begin(kMiscKernel, s);
+  const size_t image = (size_t)rows * cols;
+  for_slabs(batch, [&](size_t b0, int nb) {
+    reg_cross_power_kernel<<<dim3(rows, nb), 256, 0, s>>>(
+        reinterpret_cast<const float2*>(spec1) + (batch1 == 1 ? 0 : b0 * image), batch1 == 1,
+        reinterpret_cast<const float2*>(spec2) + b0 * image, rows, cols,
+        reinterpret_cast<float2*>(padded) + 2 * b0 * image, reinterpret_cast<float2*>(cross_power) + b0 * image);
+  });
+  prof_end(kMiscKernel, s);
+  return cuda_status(cudaGetLastError(), "ptx_reg_cross_power launch");
+}
+
+int ptx_reg_pad_transpose(const float* in, int batch, int rows, int cols, float* out, void* stream) {
+  if (int st = reg_check_stack(batch, rows, cols)) return st;
+  if (batch == 0) return PTX_OK;
+  if (!in || !out) return set_error(PTX_ERR_INVALID_ARGUMENT, "null pointer argument");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  prof_begin(kMiscKernel, s);
+  const size_t image = (size_t)rows * cols;
+  const unsigned tiles = static_cast<unsigned>((2LL * cols + 31) / 32 * ((2LL * rows + 31) / 32));
+  for_slabs(batch, [&](size_t b0, int nb) {
+    reg_pad_transpose_kernel<<<dim3(tiles, nb), 256, 0, s>>>(reinterpret_cast<const float2*>(in) + 2 * b0 * image, rows,
+                                                             cols, reinterpret_cast<float2*>(out) + 4 * b0 * image);
+  });
+  prof_end(kMiscKernel, s);
+  return cuda_status(cudaGetLastError(), "ptx_reg_pad_transpose launch");
+}
+
+size_t ptx_reg_estimate_workspace_bytes(int batch, int rows, int cols) {
+  if (batch <= 0 || rows <= 0 || cols <= 0) return 0;
+  return sizeof(PeakCand) * (size_t)batch * corr_chunks(rows, cols);
+}
+
+int ptx_reg_estimate(const float* correlation, int batch, int rows, int cols, int usfac, int* half_rc, int* row_center,
+                     int* col_center, double* peak_cc, void* workspace, size_t workspace_bytes, void* stream) {
+  if (int st = reg_check_stack(batch, rows, cols)) return st;
+  if (usfac < 2 || (long long)std::max(rows, cols) * usfac > (1ll << 30)) {
+    return set_error(PTX_ERR_INVALID_ARGUMENT, "usfac must be at least 2 and usfac times a side at most 2^30");
+  }
+  if (batch == 0) return PTX_OK;
+  if (!correlation || !half_rc || !row_center || !col_center || !peak_cc || !workspace) {
+    return set_error(PTX_ERR_INVALID_ARGUMENT, "null pointer argument");
+  }
+  if (workspace_bytes < ptx_reg_estimate_workspace_bytes(batch, rows, cols)) {
+    return set_error(PTX_ERR_WORKSPACE, "workspace of %zu bytes is smaller than %zu", workspace_bytes,
+                     ptx_reg_estimate_workspace_bytes(batch, rows, cols));
+  }
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  PeakCand* cand = static_cast<PeakCand*>(workspace);
+  const int chunks = corr_chunks(rows, cols);
+  prof_begin(kMiscKernel, s);
+  for_slabs(batch, [&](size_t b0, int nb) {
+    reg_corr_peak_kernel<<<dim3(chunks, nb), kCorrThreads, 0, s>>>(
+        reinterpret_cast<const float2*>(correlation) + 4 * b0 * rows * cols, 4LL * rows * cols, cand + b0 * chunks);
+  });
+  prof_end(kMiscKernel, s);
+  prof_begin(kMiscKernel, s);
+  reg_estimate_kernel<<<batch, 32, 0, s>>>(cand, chunks, rows, cols, usfac, half_rc, row_center, col_center,
+                                           reinterpret_cast<double2*>(peak_cc));
+  prof_end(kMiscKernel, s);
+  return cuda_status(cudaGetLastError(), "ptx_reg_estimate launch");
+}
+
+int ptx_reg_energy(const float* spec, int batch, int rows, int cols, double* energy, void* stream) {
+  if (int st = reg_check_stack(batch, rows, cols)) return st;
+  if (batch == 0) return PTX_OK;
+  if (!spec || !energy) return set_error(PTX_ERR_INVALID_ARGUMENT, "null pointer argument");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  prof_begin(kMiscKernel, s);
+  reg_energy_kernel<<<batch, 1024, 0, s>>>(reinterpret_cast<const float2*>(spec), (long long)rows * cols, energy);
+  prof_end(kMiscKernel, s);
+  return cuda_status(cudaGetLastError(), "ptx_reg_energy launch");
 }
 
 }  // extern "C"

@@ -13,10 +13,10 @@ Mirrors the MATLAB helpers of the reference's near-field example
 
 Stacks are ``[n, h, w]`` (the MATLAB functions take ``[h, w, n]``); shifts are
 ``(row, col)`` as in the reference, and the trackers return ``(locX, locY)`` =
-``(col, row)``.  The plain FFTs of images and the 2x zero-padded cross-correlation run on
-cuFFT (``torch.fft``); the matrix-multiply DFT refinement (``dftups``, ``:150-185``) and
-its peak search run in libptychox (``ptx_reg_upsampled_peak``, summed in FP64).  FP32
-spectra and FFTs, FP64 energy sums.
+``(col, row)``.  The plain FFTs of images and of the 2x zero-padded cross-correlation run on
+cuFFT (``torch.fft``); the passes around them, the matrix-multiply DFT refinement (``dftups``,
+``:150-185``, summed in FP64) and both peak searches run in libptychox (``ptx_reg_*``).
+FP32 spectra and FFTs, FP64 energy sums.
 """
 
 from __future__ import annotations
@@ -46,10 +46,6 @@ def _argmax_colmajor(a: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
     return idx % rows, idx // rows
 
 
-def _round_matlab(x: torch.Tensor) -> torch.Tensor:
-    return torch.sign(x) * torch.floor(x.abs() + 0.5)
-
-
 def _ftpad2(spec: torch.Tensor) -> torch.Tensor:
     """``FTpad(spec, [2 nr, 2 nc])`` (``dftregistration.m:189-224``) for ``[B, nr, nc]``."""
     b, nr, nc = spec.shape
@@ -57,6 +53,42 @@ def _ftpad2(spec: torch.Tensor) -> torch.Tensor:
     r0, c0 = nr - nr // 2, nc - nc // 2
     out[:, r0:r0 + nr, c0:c0 + nc] = torch.fft.fftshift(spec, dim=(-2, -1))
     return torch.fft.ifftshift(out, dim=(-2, -1)) * 4.0
+
+
+def _half_pixel_estimate(b1: torch.Tensor, b2: torch.Tensor, usfac: int):
+    """Peak of the cross-correlation of ``b1`` (one image or as many as ``b2``) and ``b2``
+    upsampled twice (``dftregistration.m:90-101``, ``FTpad`` ``:189-224``): signed half pixels
+    ``[B, 2]``, the centres ``round(shift usfac)``, the unnormalised correlation there, and the
+    cross-power spectrum.  The inverse transform is taken line by line, along the rows before
+    they are padded and along the columns after."""
+    bsz, nr, nc = b2.shape
+    dev = b2.device
+    stream = stream_handle(dev)
+    with torch.cuda.device(dev):
+        rows = torch.empty(bsz, nr, 2 * nc, dtype=torch.complex64, device=dev)
+        q = torch.empty(bsz, nr, nc, dtype=torch.complex64, device=dev)
+        _abi.call("ptx_reg_cross_power", ptr(b1), b1.shape[0], ptr(b2), bsz, nr, nc, ptr(rows), ptr(q), stream)
+        rows = torch.fft.ifft(rows, norm="forward")
+        corr = torch.empty(bsz, 2 * nc, 2 * nr, dtype=torch.complex64, device=dev)
+        _abi.call("ptx_reg_pad_transpose", ptr(rows), bsz, nr, nc, ptr(corr), stream)
+        corr = torch.fft.ifft(corr, norm="forward")
+        half = torch.empty(bsz, 2, dtype=torch.int32, device=dev)
+        centre = torch.empty(2, bsz, dtype=torch.int32, device=dev)
+        value = torch.empty(bsz, dtype=torch.complex128, device=dev)
+        ws = workspace(_abi.query("ptx_reg_estimate_workspace_bytes", bsz, nr, nc), dev)
+        _abi.call("ptx_reg_estimate", ptr(corr), bsz, nr, nc, usfac, ptr(half), ptr(centre[0]), ptr(centre[1]),
+                  ptr(value), ptr(ws), ws.numel(), stream)
+    return half, centre, value, q
+
+
+def _energy(spec: torch.Tensor) -> torch.Tensor:
+    """``sum |spec|^2`` of each image in FP64."""
+    if spec.requires_grad and torch.is_grad_enabled():
+        return (spec.abs().double() ** 2).sum(dim=(-2, -1))
+    out = torch.empty(spec.shape[0], dtype=torch.float64, device=spec.device)
+    with torch.cuda.device(spec.device):
+        _abi.call("ptx_reg_energy", ptr(spec), *spec.shape, ptr(out), stream_handle(spec.device))
+    return out
 
 
 def _refine(q: torch.Tensor, usfac: int, rc: torch.Tensor, cc: torch.Tensor):
@@ -98,10 +130,11 @@ def dftregistration(buf1ft: torch.Tensor, buf2ft: torch.Tensor, usfac: int = 1, 
     b1 = buf1ft.to(torch.complex64).reshape(-1, *buf1ft.shape[-2:])
     b2 = buf2ft.to(torch.complex64).reshape(-1, *buf2ft.shape[-2:])
     bsz = max(b1.shape[0], b2.shape[0])
-    b1, b2 = b1.expand(bsz, -1, -1), b2.expand(bsz, -1, -1)
+    b1, b2 = b1.expand(min(bsz, b1.shape[0]), -1, -1).contiguous(), b2.expand(bsz, -1, -1).contiguous()
+    if b1.shape[0] not in (1, bsz):
+        b1 = b1.expand(bsz, -1, -1)  # raises: the two batches differ
     nr, nc = b2.shape[-2:]
     dev = b2.device
-    ar = torch.arange(bsz, device=dev)
     zeros = torch.zeros(bsz, dtype=torch.float64, device=dev)
     if usfac == 0:
         ccmax = (b1.to(torch.complex128) * b2.to(torch.complex128).conj()).sum(dim=(-2, -1))
@@ -109,30 +142,28 @@ def dftregistration(buf1ft: torch.Tensor, buf2ft: torch.Tensor, usfac: int = 1, 
     elif usfac == 1:
         cc = torch.fft.ifft2(b1 * b2.conj())
         r, c = _argmax_colmajor(cc.abs())
-        ccmax = cc[ar, r, c].to(torch.complex128) * (nr * nc)
+        ccmax = cc[torch.arange(bsz, device=dev), r, c].to(torch.complex128) * (nr * nc)
         row_shift, col_shift = _freq(nr, dev)[r].double(), _freq(nc, dev)[c].double()
-    else:
+    elif usfac == 2 and torch.is_grad_enabled() and (b1.requires_grad or b2.requires_grad):
         cc = torch.fft.ifft2(_ftpad2(b1 * b2.conj()))
         r, c = _argmax_colmajor(cc.abs())
-        ccmax = cc[ar, r, c].to(torch.complex128) * (nr * nc)
-        row_shift = torch.fft.ifftshift(torch.arange(-nr, nr, device=dev))[r].double() / 2.0
-        col_shift = torch.fft.ifftshift(torch.arange(-nc, nc, device=dev))[c].double() / 2.0
+        ccmax = cc[torch.arange(bsz, device=dev), r, c].to(torch.complex128) * (nr * nc)
+        row_shift, col_shift = (torch.fft.ifftshift(torch.arange(-n, n, device=dev))[i].double() / 2.0
+                                for n, i in ((nr, r), (nc, c)))
+    else:
+        half, centre, ccmax, q = _half_pixel_estimate(b1.detach(), b2.detach(), usfac)
+        row_shift, col_shift = half[:, 0].double() / 2.0, half[:, 1].double() / 2.0
         if usfac > 2:
-            rc = _round_matlab(row_shift * usfac)
-            ccn = _round_matlab(col_shift * usfac)
-            q = (b2 * b1.conj()).contiguous()
-            peak, ccmax = _refine(q, usfac, rc.to(torch.int32).contiguous(), ccn.to(torch.int32).contiguous())
+            peak, ccmax = _refine(q, usfac, centre[0], centre[1])
             dftshift = math.ceil(1.5 * usfac) // 2
-            ccmax = ccmax.to(torch.complex128)
-            row_shift = rc / usfac + (peak[:, 0] - dftshift).double() / usfac
-            col_shift = ccn / usfac + (peak[:, 1] - dftshift).double() / usfac
+            row_shift = centre[0].double() / usfac + (peak[:, 0] - dftshift).double() / usfac
+            col_shift = centre[1].double() / usfac + (peak[:, 1] - dftshift).double() / usfac
+    if usfac > 1:
         if nr == 1:
             row_shift = zeros
         if nc == 1:
             col_shift = zeros.clone()
-    rg00 = (b1.abs().double() ** 2).sum(dim=(-2, -1))
-    rf00 = (b2.abs().double() ** 2).sum(dim=(-2, -1))
-    error = torch.sqrt(torch.abs(1.0 - ccmax.abs() ** 2 / (rg00 * rf00)))
+    error = torch.sqrt(torch.abs(1.0 - ccmax.abs() ** 2 / (_energy(b1) * _energy(b2))))
     diffphase = torch.angle(ccmax)
     out = torch.stack([error, diffphase, row_shift, col_shift], dim=1)
     if not return_registered:

@@ -1,6 +1,7 @@
 """The upsampled correlation patch and its peak (``ptx_reg_upsampled_peak``) against the dense
 FP64 transform, at the edges of its tiles: one-line spectra, 32-column and 64-row stages, patches
-one point around a 64-point tile, a single and a shared row block.
+one point around a 64-point tile, a single and a shared row block; and the passes of the initial
+estimate against numpy.
 
 Tolerance: both sides sum ``rows * cols`` FP64 terms of total magnitude ``S = sum |Q|`` in some
 order, each term a product of a few rounded factors, so each is within ``32 eps S`` of the exact
@@ -68,3 +69,37 @@ def test_ties_take_the_first_point_and_nan_the_origin():
               ws.numel(), stream_handle(dev))
     assert peak.cpu().tolist() == [[0, 0], [0, 0]]
     assert complex(value[0].cpu()) == 3.0 and np.isnan(complex(value[1].cpu()).real)
+
+
+@pytest.mark.parametrize("rows, cols", [(1, 1), (1, 40), (33, 1), (16, 31), (48, 64), (45, 51), (97, 130)])
+@pytest.mark.parametrize("single", [True, False])
+def test_half_pixel_estimate(rows, cols, single):
+    """Peak of the twice-upsampled correlation, cross-power and energies.  The correlation is an
+    FP32 transform of ``rows * cols`` products: its values are within ``32 eps32 sum |product|``
+    of the FP64 transform's (a few rounded stages per axis), so the peak is a maximum of it up
+    to twice that."""
+    from ptychox_b200.registration import _energy, _half_pixel_estimate
+
+    rng = np.random.default_rng(rows * 1000 + cols)
+    b, usfac = 3, 7
+    s1 = rng.standard_normal((1 if single else b, rows, cols, 2)).astype(np.float32).view(np.complex64)[..., 0]
+    s2 = rng.standard_normal((b, rows, cols, 2)).astype(np.float32).view(np.complex64)[..., 0]
+    t1, t2 = torch.from_numpy(s1).cuda(), torch.from_numpy(s2).cuda()
+    half, centre, value, q = (t.cpu().numpy() for t in _half_pixel_estimate(t1, t2, usfac))
+    product = s1.astype(np.complex128) * np.conj(s2.astype(np.complex128))
+    assert np.abs(q - np.conj(product)).max() <= 4 * np.finfo(np.float32).eps * np.abs(product).max()
+    full = np.zeros((b, 2 * rows, 2 * cols), np.complex128)
+    full[:, rows - rows // 2:2 * rows - rows // 2, cols - cols // 2:2 * cols - cols // 2] = np.fft.fftshift(
+        product, axes=(1, 2))
+    corr = np.fft.ifft2(np.fft.ifftshift(full, axes=(1, 2))) * (4 * rows * cols)
+    for i in range(b):
+        r, c = half[i]
+        assert -rows <= r < rows and -cols <= c < cols
+        tol = 32 * np.finfo(np.float32).eps * np.abs(product[i]).sum()
+        assert abs(value[i] - corr[i, r, c]) <= tol
+        assert abs(corr[i, r, c]) >= np.abs(corr[i]).max() - 2 * tol
+        want = [np.sign(v) * np.floor(abs(v) * usfac / 2 + 0.5) for v in (r, c)]
+        assert centre[:, i].tolist() == want
+    energy = _energy(t2).cpu().numpy()
+    exact = (np.abs(s2.astype(np.complex128)) ** 2).sum(axis=(1, 2))
+    assert np.abs(energy - exact).max() <= 4 * rows * cols * np.finfo(np.float64).eps * exact.max()
