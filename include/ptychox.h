@@ -86,6 +86,12 @@ int ptx_get_units_per_cta(void);
  * `.to(device)`. */
 int ptx_stage_host_bytes(void* dst, const void* src, size_t bytes, void* stream);
 
+/* out = z * g for two complex64 arrays (n_a and n_b elements; either may be empty) and one FP64
+ * factor g on the device, rounded to FP32: the backward of the fused losses, whose gradients
+ * were computed for a unit loss gradient.  Inputs and outputs do not overlap. */
+int ptx_scale_gradients(const double* factor, const float* a, float* out_a, size_t n_a, const float* b, float* out_b,
+                        size_t n_b, void* stream);
+
 /* Optional per-kernel CUDA-event timing: when enabled every launch is bracketed by an
  * event pair on its stream.  ptx_profile_read synchronises on the recorded events and
  * returns the accumulated device time and timed launches of one kernel kind

@@ -44,6 +44,7 @@ SIGNATURES: dict[str, tuple] = {
     "ptx_set_thread_units_per_cta": (_i, [_i]),
     "ptx_get_units_per_cta": (_i, []),
     "ptx_stage_host_bytes": (_i, [_p, _p, _sz, _p]),
+    "ptx_scale_gradients": (_i, [_p, _p, _p, _sz, _p, _p, _sz, _p]),
     "ptx_profile_enable": (_i, [_i]),
     "ptx_profile_reset": (_i, []),
     "ptx_profile_kinds": (_i, []),

@@ -129,7 +129,17 @@ def upload_small(t: torch.Tensor, device: torch.device, dtype: torch.dtype) -> t
 
 
 def stream_handle(device: torch.device) -> int:
+    """The current stream of `device` as the integer handle the library takes."""
     return torch.cuda.current_stream(device).cuda_stream
+
+
+def call_on(device: torch.device, name: str, *args) -> None:
+    """Library call with the current stream of `device` as its last argument, `device` current."""
+    if torch.cuda.current_device() == device.index:
+        _abi.call(name, *args, stream_handle(device))
+    else:
+        with torch.cuda.device(device):
+            _abi.call(name, *args, stream_handle(device))
 
 
 def workspace(nbytes: int, device: torch.device) -> torch.Tensor:
@@ -150,6 +160,28 @@ def as_u16(measured: torch.Tensor, device: torch.device) -> torch.Tensor:
             raise ValueError("measured counts must lie in [0, 65535].")
         measured = host.to(torch.int32).to(torch.uint16)
     return measured.to(device=device).contiguous()
+
+
+def scaled_gradients(grad_loss: torch.Tensor, first: torch.Tensor, second: torch.Tensor):
+    """``(first * g, second * g)`` for saved unit-loss gradients and the FP64 scalar gradient
+    ``g`` of the loss: one launch, or torch's products where those are needed themselves (a
+    backward that is to be differentiated) or hold what the kernel cannot read (batched or
+    moved saved tensors)."""
+    if not torch.is_grad_enabled():
+        dev = first.device
+        try:
+            args = grad_loss.data_ptr(), first.data_ptr(), second.data_ptr()
+        except RuntimeError:  # a tensor without storage of its own (vmap)
+            args = (0,)
+        if all(args) and dev.type == "cuda" and grad_loss.device == dev == second.device \
+                and grad_loss.dtype == torch.float64 and grad_loss.numel() == 1 \
+                and first.dtype == second.dtype == torch.complex64 and first.is_contiguous() and second.is_contiguous():
+            out = torch.empty_like(first), torch.empty_like(second)
+            call_on(dev, "ptx_scale_gradients", args[0], args[1], out[0].data_ptr(), first.numel(), args[2],
+                    out[1].data_ptr(), second.numel())
+            return out
+    g = grad_loss.to(torch.float32)
+    return first * g, second * g
 
 
 def load_library():

@@ -22,6 +22,7 @@ from ._utils import (
     device_positions_subpixel,
     ptr,
     require_cuda_complex64,
+    scaled_gradients,
     stream_handle,
     workspace,
 )
@@ -165,9 +166,8 @@ class PtychoXBaseLossFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_loss):  # type: ignore[override]
-        gs, gp = ctx.saved_tensors
-        g = grad_loss.to(torch.float32)
-        return gs * g, gp * g, None, None, None
+        gs, gp = scaled_gradients(grad_loss, *ctx.saved_tensors)
+        return gs, gp, None, None, None
 
 
 def ptychoX_base_loss(
@@ -285,9 +285,8 @@ class PtychoXBaseSubpixelLossFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_loss):  # type: ignore[override]
-        gs, gp = ctx.saved_tensors
-        g = grad_loss.to(torch.float32)
-        return gs * g, gp * g, None, None, None
+        gs, gp = scaled_gradients(grad_loss, *ctx.saved_tensors)
+        return gs, gp, None, None, None
 
 
 def ptychoX_base_subpixel(sample: torch.Tensor, probe: torch.Tensor, positions_xy: torch.Tensor) -> torch.Tensor:

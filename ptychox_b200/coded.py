@@ -19,7 +19,7 @@ from __future__ import annotations
 import torch
 
 from . import _abi
-from ._utils import as_u16, ptr, stream_handle, upload_small, workspace
+from ._utils import as_u16, ptr, scaled_gradients, stream_handle, upload_small, workspace
 
 __all__ = [
     "ptychoX_coded",
@@ -231,12 +231,11 @@ class PtychoXCodedLossFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_loss):  # type: ignore[override]
         saved = ctx.saved_tensors
-        go, gm = saved[0], saved[1]
-        g = grad_loss.to(torch.float32)
+        go, gm = scaled_gradients(grad_loss, saved[0], saved[1])
         g_shift = None
         if len(saved) == 3:
             g_shift = (saved[2] * grad_loss.to(torch.float64)).to(device=ctx.shift_device, dtype=ctx.shift_dtype)
-        return go * g, gm * g, None, None, g_shift, None, None, None, None
+        return go, gm, None, None, g_shift, None, None, None, None
 
 
 def ptychoX_coded_loss(object_field, coded_surface, transfer_1, transfer_2, shifts_xy, downsample, measured,

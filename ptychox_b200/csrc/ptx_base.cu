@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(256) base_rows_forward_rt(
     const float2* __restrict__ sample, int H, int W, const float2* __restrict__ probe, int ph, int pw,
     const int64_t* __restrict__ pos, int nframes, int frames_per_cta, float2* __restrict__ scratch,
     LinePlan plan, int lines, unsigned* __restrict__ err) {
+  pdl_wait();
   extern __shared__ float2 sm[];
   const int pitch = line_pitch(pw);
   const int tid = threadIdx.x;
@@ -86,6 +87,7 @@ __global__ void __launch_bounds__(512, 1) base_cols_rt(
     const uint16_t* __restrict__ measured, float scale, float grad_scale, double inv_numel,
     double* __restrict__ loss, float2* __restrict__ far_field, float* __restrict__ amplitude,
     const float* __restrict__ grad_output) {
+  pdl_wait();
   extern __shared__ float2 sm[];
   __shared__ double red[32];
   const int pitch = line_pitch(ph);
@@ -186,6 +188,7 @@ __global__ void __launch_bounds__(256) base_rows_adjoint_rt(
     const float2* __restrict__ probe, int ph, int pw, const int64_t* __restrict__ pos, int nframes,
     int frames_per_cta, float2* __restrict__ grad_sample, float2* __restrict__ grad_probe,
     LinePlan plan, int lines) {
+  pdl_wait();
   extern __shared__ float2 sm[];
   const int pitch = line_pitch(pw);
   const int tid = threadIdx.x;
@@ -377,6 +380,7 @@ __global__ void __launch_bounds__(256, 2) base_cols_reg(
     const uint16_t* __restrict__ measured, const float* __restrict__ lut, float grad_scale, double inv_numel,
     double* __restrict__ loss, float2* __restrict__ far_field, float* __restrict__ amplitude,
     const float* __restrict__ grad_output) {
+  pdl_wait();
   using S = RegShape<N>;
   constexpr int LP = ColCfg<N>::LP;
   extern __shared__ float2 sm[];
@@ -776,6 +780,7 @@ struct RegLaunch {
 // entry point, whose row passes skip such windows without flagging them.
 static __global__ void window_check_kernel(const int64_t* __restrict__ pos, int n, int ph, int pw, int H, int W,
                                            unsigned* __restrict__ err) {
+  pdl_wait();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b < n && !window_ok(pos[2 * b], pos[2 * b + 1], ph, pw, H, W)) atomicOr(err, 1u);
 }
@@ -877,8 +882,8 @@ void launch_rows_forward(const BaseGeom& g, const float2* sample, const float2* 
       const int rowgroups = (g.ph + lines - 1) / lines;
       const int threads = lines * L::T, smem = FwdCfg<N>::smem(lines);
       const int grid = persistent_grid((const void*)base_rows_forward_reg<N>, threads, smem, (long long)rowgroups * nframes);
-      launch_pdl(base_rows_forward_reg<N>, grid, threads, smem, s, sample, g.H, g.W, probe, g.ph, pos, nframes, rowgroups,
-                                                           g.scratch, g.row.tw, lines, g.err);
+      launch_pdl(base_rows_forward_reg<N>, grid, threads, smem, s, sample, g.H, g.W, probe, g.ph, pos, nframes,
+                 rowgroups, g.scratch, g.row.tw, lines, g.err);
     } else if (const MixOps* mo = mix_ops(g.pw)) {
       MixRowsArgs a{sample, g.H, g.W, probe, g.ph, g.pw, pos, nframes, g.scratch, g.row.mix_twt, g.row.mix_twi,
                     g.err, nullptr, nullptr};
@@ -886,8 +891,8 @@ void launch_rows_forward(const BaseGeom& g, const float2* sample, const float2* 
     } else {
       const int rowgroups = (g.ph + g.rs.lines - 1) / g.rs.lines;
       dim3 grid(rowgroups, nframes);
-      base_rows_forward_rt<0><<<grid, g.rs.threads, g.rs.smem, s>>>(sample, g.H, g.W, probe, g.ph, g.pw, pos,
-                                                                    nframes, 1, g.scratch, g.row, g.rs.lines, g.err);
+      launch_pdl(base_rows_forward_rt<0>, grid, g.rs.threads, g.rs.smem, s, sample, g.H, g.W, probe, g.ph, g.pw,
+                 pos, nframes, 1, g.scratch, g.row, g.rs.lines, g.err);
     }
   });
   prof_end(kBaseRowsForward, s);
@@ -905,8 +910,8 @@ void launch_rows_adjoint(const BaseGeom& g, const float2* sample, const float2* 
       const int threads = lines * L::T, smem = L::adj_smem(lines);
       const long long units = (long long)rowgroups * nframes;
       const int grid = persistent_grid((const void*)base_rows_adjoint_reg<N>, threads, smem, units);
-      launch_pdl(base_rows_adjoint_reg<N>, grid, threads, smem, s, g.scratch, sample, g.H, g.W, probe, g.ph, pos, nframes,
-                                                           rowgroups, grad_sample, grad_probe, g.row.tw, lines);
+      launch_pdl(base_rows_adjoint_reg<N>, grid, threads, smem, s, g.scratch, sample, g.H, g.W, probe, g.ph, pos,
+                 nframes, rowgroups, grad_sample, grad_probe, g.row.tw, lines);
     } else if (const MixOps* mo = mix_ops(g.pw)) {
       MixRowsArgs a{sample, g.H, g.W, probe, g.ph, g.pw, pos, nframes, g.scratch, g.row.mix_twt, g.row.mix_twi,
                     g.err, grad_sample, grad_probe};
@@ -915,9 +920,8 @@ void launch_rows_adjoint(const BaseGeom& g, const float2* sample, const float2* 
       const int rowgroups = (g.ph + g.rs.lines - 1) / g.rs.lines;
       const int fpc = frames_per_cta_for(rowgroups, nframes, sm_count() * 8);
       dim3 grid(rowgroups, (nframes + fpc - 1) / fpc);
-      base_rows_adjoint_rt<0><<<grid, g.rs.threads, g.rs.smem, s>>>(g.scratch, sample, g.H, g.W, probe, g.ph,
-                                                                    g.pw, pos, nframes, fpc, grad_sample,
-                                                                    grad_probe, g.row, g.rs.lines);
+      launch_pdl(base_rows_adjoint_rt<0>, grid, g.rs.threads, g.rs.smem, s, g.scratch, sample, g.H, g.W, probe,
+                 g.ph, g.pw, pos, nframes, fpc, grad_sample, grad_probe, g.row, g.rs.lines);
     }
   });
   prof_end(kBaseRowsAdjoint, s);
@@ -945,19 +949,16 @@ void launch_cols(const BaseGeom& g, int frame0, int nframes, const uint16_t* mea
         return;
       }
       dim3 grid(num_tiles(g.pw) * (kTile / kColsReg), nframes);
-      base_cols_reg<MODE, N><<<grid, L::col_threads(), L::col_smem(), s>>>(
-          g.scratch, g.pw, frame0, g.col.tw, measured, g.lut, grad_scale, inv_numel, loss, far_field, amplitude,
-          grad_output);
+      launch_pdl(base_cols_reg<MODE, N>, grid, L::col_threads(), L::col_smem(), s, g.scratch, g.pw, frame0,
+                 g.col.tw, measured, g.lut, grad_scale, inv_numel, loss, far_field, amplitude, grad_output);
     } else if (const MixOps* mo = mix_ops(g.ph)) {
       MixColsArgs a{g.scratch, g.ph, g.pw, frame0, nframes, g.col.mix_twt, g.col.mix_twi, measured, g.lut,
                     grad_scale, inv_numel, loss, far_field, amplitude, grad_output};
       mo->cols(MODE == kColSweep ? kMixColSweep : MODE == kColForward ? kMixColForward : kMixColBackward, a, s);
     } else {
       dim3 grid(num_tiles(g.pw) * (kTile / g.cs.cols), nframes);
-      base_cols_rt<MODE, 0><<<grid, g.cs.threads, g.cs.smem, s>>>(g.scratch, g.ph, g.pw, frame0, g.col,
-                                                                  g.cs.cols, measured, scale, grad_scale,
-                                                                  inv_numel, loss, far_field, amplitude,
-                                                                  grad_output);
+      launch_pdl(base_cols_rt<MODE, 0>, grid, g.cs.threads, g.cs.smem, s, g.scratch, g.ph, g.pw, frame0, g.col,
+                 g.cs.cols, measured, scale, grad_scale, inv_numel, loss, far_field, amplitude, grad_output);
     }
   });
   prof_end(kBaseCols, s);
@@ -1050,13 +1051,11 @@ int ptx_base_backward(const float* grad_output, const float* far_field, const fl
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   float2* GS = reinterpret_cast<float2*>(grad_sample);
   float2* GP = reinterpret_cast<float2*>(grad_probe);
-  cudaMemsetAsync(GS, 0, sizeof(float2) * (size_t)sample_h * sample_w, s);
-  cudaMemsetAsync(GP, 0, sizeof(float2) * (size_t)probe_h * probe_w, s);
-  cudaMemsetAsync(g.err, 0, sizeof(unsigned), s);
+  launch_prologue(s, GS, (size_t)sample_h * sample_w, GP, (size_t)probe_h * probe_w, nullptr, g.err, nullptr, 0.f);
   if (batch > 0) {
     prof_begin(kMiscKernel, s);
-    window_check_kernel<<<(batch + 255) / 256, 256, 0, s>>>(positions_xy, batch, probe_h, probe_w, sample_h, sample_w,
-                                                            g.err);
+    launch_pdl(window_check_kernel, (batch + 255) / 256, 256, 0, s, positions_xy, batch, probe_h, probe_w, sample_h,
+               sample_w, g.err);
     prof_end(kMiscKernel, s);
   }
   const float2* S = reinterpret_cast<const float2*>(sample);
@@ -1088,12 +1087,7 @@ int ptx_base_sweep(const float* sample, int sample_h, int sample_w, const float*
   float2* GP = reinterpret_cast<float2*>(grad_probe);
   const double numel = (double)batch * probe_h * probe_w;
   const float grad_scale = static_cast<float>(2.0 / std::max(numel, 1.0));
-  {
-    const size_t ns = (size_t)sample_h * sample_w, np = (size_t)probe_h * probe_w;
-    prof_begin(kMiscKernel, s);
-    launch_pdl(sweep_prologue_kernel, prologue_blocks(ns, sm_count()), 256, 0, s, GS, ns, GP, np, loss, g.err, g.lut, scale);
-    prof_end(kMiscKernel, s);
-  }
+  launch_prologue(s, GS, (size_t)sample_h * sample_w, GP, (size_t)probe_h * probe_w, loss, g.err, g.lut, scale);
   const float2* S = reinterpret_cast<const float2*>(sample);
   const float2* P = reinterpret_cast<const float2*>(probe);
   for (int b0 = 0; b0 < batch; b0 += g.chunk) {
@@ -1141,12 +1135,7 @@ int ptx_base_sweep_small(const float* sample, int sample_h, int sample_w, const 
   float2* GP = reinterpret_cast<float2*>(grad_probe);
   const double numel = (double)batch * probe_h * probe_w;
   const float grad_scale = static_cast<float>(2.0 / std::max(numel, 1.0));
-  {
-    const size_t ns = (size_t)sample_h * sample_w, np = (size_t)probe_h * probe_w;
-    prof_begin(kMiscKernel, s);
-    launch_pdl(sweep_prologue_kernel, prologue_blocks(ns, sm_count()), 256, 0, s, GS, ns, GP, np, loss, g.err, g.lut, scale);
-    prof_end(kMiscKernel, s);
-  }
+  launch_prologue(s, GS, (size_t)sample_h * sample_w, GP, (size_t)probe_h * probe_w, loss, g.err, g.lut, scale);
   if (batch == 0) return cuda_status(cudaGetLastError(), "ptx_base_sweep_small launch");
   const float2* S = reinterpret_cast<const float2*>(sample);
   const float2* P = reinterpret_cast<const float2*>(probe);

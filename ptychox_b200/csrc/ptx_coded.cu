@@ -61,6 +61,7 @@ __global__ void __launch_bounds__(256, 2) coded_cols(
     float2* __restrict__ scratch, const float2* __restrict__ ospec, const float2* __restrict__ t1,
     const float2* __restrict__ t2, const float* __restrict__ shifts, float inv_n, float2* __restrict__ grad_ospec,
     const float2* __restrict__ tw, double* __restrict__ grad_shifts) {
+  pdl_wait();
   using S = RegShape<N>;
   using CP = ColPass<N>;
   extern __shared__ float2 sm[];
@@ -149,6 +150,7 @@ __global__ void __launch_bounds__(256, 2) coded_cols(
 template <bool CONJ, int N>
 __global__ void __launch_bounds__(ColPairCfg<N>::kThreads, ColPairCfg<N>::kThreads <= 128 ? 2 : 1) coded_cols_filter_pair(
     float2* __restrict__ scratch, const float2* __restrict__ t2, float inv_n, const float2* __restrict__ tw) {
+  pdl_wait();
   using S = RegShape<N>;
   using Cfg = ColPairCfg<N>;
   constexpr int kTiles = (N + kTile - 1) / kTile;
@@ -275,6 +277,7 @@ __global__ void __launch_bounds__(128, 3) coded_rows_mask(float2* __restrict__ s
                                                           const float2* __restrict__ mask,
                                                           float2* __restrict__ xstore, float inv_n, int nframes,
                                                           int rowgroups, const float2* __restrict__ tw, int lines) {
+  pdl_wait();
   using S = RegShape<N>;
   using Cfg = CodedRowCfg<N>;
   extern __shared__ float2 sm[];
@@ -345,6 +348,7 @@ __global__ void __launch_bounds__(256, 2) coded_rows_pool(
     float scale, float grad_scale, double inv_numel, double* __restrict__ loss, float2* __restrict__ sensor,
     float* __restrict__ amplitude, const float* __restrict__ grad_output, const float2* __restrict__ tw,
     int lines) {
+  pdl_wait();
   using S = RegShape<N>;
   extern __shared__ float2 sm[];
   float* pool = reinterpret_cast<float*>(sm + lines * RowPass<N>::LP);  // [lines][N] |s|^2, then factors
@@ -422,6 +426,7 @@ template <int N>
 __global__ void __launch_bounds__(128, 2) coded_rows_grad_mask(
     float2* __restrict__ scratch, const float2* __restrict__ mask, const float2* __restrict__ xstore, int nframes,
     int rowgroups, float2* __restrict__ grad_mask, const float2* __restrict__ tw, int lines) {
+  pdl_wait();
   using S = RegShape<N>;
   extern __shared__ float2 sm[];
   const int tid = threadIdx.x;
@@ -531,6 +536,7 @@ __device__ __forceinline__ void fd_unit(float dx, float dy, bool isotropic, floa
 __global__ void __launch_bounds__(256) fd_loss_kernel(const float* __restrict__ amp, const uint16_t* __restrict__ meas,
                                                       float scale, long long total, int h, int w, int isotropic,
                                                       float* __restrict__ grad_amp, double* __restrict__ loss) {
+  pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   double part = 0.0;
   if (i < total) {
@@ -694,12 +700,12 @@ void launch_fft2(const CodedGeom& g, const float2* in, int n, float2* out, float
     constexpr int N = decltype(NT)::value;
     const int lines = RowPass<N>::lines(256, N);
     prof_begin(kFft2Rows, s);
-    fft2_rows_kernel<N, INV><<<(N + lines - 1) / lines, lines * RowPass<N>::T, RowPass<N>::smem(lines), s>>>(
-        in, N, tmp, p.tw, lines);
+    launch_pdl(fft2_rows_kernel<N, INV>, (N + lines - 1) / lines, lines * RowPass<N>::T, RowPass<N>::smem(lines), s,
+                in, N, tmp, p.tw, lines);
     prof_end(kFft2Rows, s);
     prof_begin(kFft2Cols, s);
-    fft2_cols_kernel<N, INV><<<num_tiles(N) * (kTile / kColsPerCta), ColPass<N>::kThreads,
-                               kColsPerCta * ColPass<N>::LP * (int)sizeof(float2), s>>>(tmp, N, out, 1.0f, p.tw);
+    launch_pdl(fft2_cols_kernel<N, INV>, num_tiles(N) * (kTile / kColsPerCta), ColPass<N>::kThreads,
+               kColsPerCta * ColPass<N>::LP * (int)sizeof(float2), s, tmp, N, out, 1.0f, p.tw);
     prof_end(kFft2Cols, s);
   });
 }
@@ -726,14 +732,15 @@ void launch_cols(const CodedGeom& g, int nf, const float2* t1, const float2* t2,
       if ((reinterpret_cast<uintptr_t>(t2) & 15) == 0) {
         using C = ColPairCfg<N>;
         dim3 grid(num_tiles(N), nf);
-        coded_cols_filter_pair<CONJ, N><<<grid, C::kThreads, C::kExchBytes + C::kTwBytes, s>>>(g.frames, t2, inv_n,
-                                                                                             g.plan.tw);
+        launch_pdl(coded_cols_filter_pair<CONJ, N>, grid, C::kThreads, C::kExchBytes + C::kTwBytes, s, g.frames, t2,
+                   inv_n, g.plan.tw);
         return;
       }
     }
     dim3 grid(num_tiles(N) * (kTile / kColsPerCta), nf);
-    coded_cols<STAGE, CONJ, N><<<grid, ColPass<N>::kThreads, kColsPerCta * ColPass<N>::LP * (int)sizeof(float2), s>>>(
-        g.frames, g.ospec, t1, t2, shifts, inv_n, g.gospec, g.plan.tw, STAGE == 7 ? grad_shifts : nullptr);
+    launch_pdl(coded_cols<STAGE, CONJ, N>, grid, ColPass<N>::kThreads,
+               kColsPerCta * ColPass<N>::LP * (int)sizeof(float2), s, g.frames, g.ospec, t1, t2, shifts, inv_n,
+               g.gospec, g.plan.tw, STAGE == 7 ? grad_shifts : nullptr);
   });
   prof_end(kCodedCols, s);
 }
@@ -755,7 +762,8 @@ void launch_rows_mask(const CodedGeom& g, int nf, const float2* mask, float2* xs
     const int rowgroups = (N + lines - 1) / lines;
     const int threads = lines * RowPass<N>::T, smem = CodedRowCfg<N>::smem(lines, 1);
     const int grid = persistent_grid((const void*)coded_rows_mask<N>, threads, smem, (long long)rowgroups * nf);
-    coded_rows_mask<N><<<grid, threads, smem, s>>>(g.frames, mask, xstore, inv_n, nf, rowgroups, g.plan.tw, lines);
+    launch_pdl(coded_rows_mask<N>, grid, threads, smem, s, g.frames, mask, xstore, inv_n, nf, rowgroups, g.plan.tw,
+               lines);
   });
   prof_end(kCodedRows, s);
 }
@@ -787,9 +795,8 @@ void launch_rows_pool(const CodedGeom& g, int frame0, int nf, const uint16_t* me
     const int lines = RowPass<N>::lines(256, N);
     dim3 grid((N + lines - 1) / lines, nf);
     const int smem = RowPass<N>::smem(lines) + lines * N * (int)sizeof(float) + N * (int)sizeof(float2);
-    coded_rows_pool<MODE, N><<<grid, lines * RowPass<N>::T, smem, s>>>(g.frames, g.ds, frame0, inv_n, measured, scale,
-                                                                       grad_scale, inv_numel, loss, sensor, amplitude,
-                                                                       grad_output, g.plan.tw, lines);
+    launch_pdl(coded_rows_pool<MODE, N>, grid, lines * RowPass<N>::T, smem, s, g.frames, g.ds, frame0, inv_n,
+               measured, scale, grad_scale, inv_numel, loss, sensor, amplitude, grad_output, g.plan.tw, lines);
   });
   prof_end(kCodedRows, s);
 }
@@ -812,8 +819,8 @@ void launch_rows_grad_mask(const CodedGeom& g, int nf, const float2* mask, const
     const int rowgroups = (N + lines - 1) / lines;
     const int threads = lines * RowPass<N>::T, smem = CodedRowCfg<N>::smem(lines, 2);
     const int grid = persistent_grid((const void*)coded_rows_grad_mask<N>, threads, smem, (long long)rowgroups * nf);
-    coded_rows_grad_mask<N><<<grid, threads, smem, s>>>(g.frames, mask, xstore, nf, rowgroups, grad_mask, g.plan.tw,
-                                                        lines);
+    launch_pdl(coded_rows_grad_mask<N>, grid, threads, smem, s, g.frames, mask, xstore, nf, rowgroups, grad_mask,
+               g.plan.tw, lines);
   });
   prof_end(kCodedRows, s);
 }
@@ -837,7 +844,7 @@ namespace {
 int coded_backward_impl(const float* grad_output, const float* x_forward, const float* sensor, const float* amplitude,
                         const float* coded_surface, const float* transfer_1, const float* transfer_2, int n,
                         const float* shifts_xy, int batch, int downsample, float* grad_object, float* grad_coded,
-                        void* workspace, size_t workspace_bytes, void* stream, double* grad_shifts) {
+                        void* workspace, size_t workspace_bytes, void* stream, double* grad_shifts, bool zero) {
   CodedGeom g;
   if (int st = coded_check(n, downsample, coded_surface, coded_surface, transfer_2, shifts_xy, batch, workspace,
                            workspace_bytes, false, &g)) {
@@ -853,8 +860,10 @@ int coded_backward_impl(const float* grad_output, const float* x_forward, const 
   const float2* T1 = reinterpret_cast<const float2*>(transfer_1);
   const float2* T2 = reinterpret_cast<const float2*>(transfer_2);
   const float2* M = reinterpret_cast<const float2*>(coded_surface);
-  cudaMemsetAsync(g.gospec, 0, g.field_bytes, s);
-  cudaMemsetAsync(grad_coded, 0, g.field_bytes, s);
+  if (zero) {
+    const size_t field = g.field_bytes / sizeof(float2);
+    launch_prologue(s, g.gospec, field, reinterpret_cast<float2*>(grad_coded), field, nullptr, nullptr, nullptr, 0.f);
+  }
   for (int b0 = 0; b0 < batch; b0 += g.chunk) {
     const int nf = std::min(g.chunk, batch - b0);
     launch_rows_pool<kCodedBackward>(g, b0, nf, nullptr, 0.f, 0.f, 0.0, nullptr,
@@ -912,7 +921,7 @@ int ptx_coded_backward(const float* grad_output, const float* x_forward, const f
                        void* workspace, size_t workspace_bytes, void* stream) {
   return coded_backward_impl(grad_output, x_forward, sensor, amplitude, coded_surface, transfer_1, transfer_2, n,
                              shifts_xy, batch, downsample, grad_object, grad_coded, workspace, workspace_bytes, stream,
-                             nullptr);
+                             nullptr, true);
 }
 
 static int coded_sweep_mse(const float* object, const float* coded_surface, const float* transfer_1,
@@ -932,14 +941,9 @@ static int coded_sweep_mse(const float* object, const float* coded_surface, cons
   const float2* T1 = reinterpret_cast<const float2*>(transfer_1);
   const float2* T2 = reinterpret_cast<const float2*>(transfer_2);
   const float2* M = reinterpret_cast<const float2*>(coded_surface);
-  {
-    const size_t nf = g.field_bytes / sizeof(float2);
-    prof_begin(kMiscKernel, s);
-    sweep_prologue_kernel<<<prologue_blocks(nf, sm_count()), 256, 0, s>>>(
-        g.gospec, nf, reinterpret_cast<float2*>(grad_coded), nf, loss, nullptr, nullptr, 0.f);
-    if (grad_shifts) cudaMemsetAsync(grad_shifts, 0, sizeof(double) * 2 * (size_t)batch, s);
-    prof_end(kMiscKernel, s);
-  }
+  const size_t field = g.field_bytes / sizeof(float2);
+  launch_prologue(s, g.gospec, field, reinterpret_cast<float2*>(grad_coded), field, loss, nullptr, nullptr, 0.f,
+                  grad_shifts, grad_shifts ? 2 * (size_t)batch : 0);
   const int lw = n / downsample;
   const double numel = (double)batch * lw * lw;
   const float grad_scale = static_cast<float>(2.0 / std::max(numel, 1.0));
@@ -1012,23 +1016,28 @@ static int coded_sweep_fd(const float* object, const float* coded_surface, const
   p += up(b * pooled);
   const size_t inner = workspace_bytes - static_cast<size_t>(p - static_cast<char*>(workspace));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  // the adjoint accumulates into its object-spectrum gradient in the frames' region; the shift
+  // gradient reads the object spectrum the forward leaves there
+  CodedGeom g;
+  if (int st = coded_check(n, downsample, object, coded_surface, transfer_2, shifts_xy, batch, p, inner, false, &g)) {
+    return st;
+  }
+  launch_prologue(s, g.gospec, g.field_bytes / sizeof(float2), reinterpret_cast<float2*>(grad_coded),
+                  g.field_bytes / sizeof(float2), loss, nullptr, nullptr, 0.f, grad_shifts,
+                  grad_shifts ? 2 * (size_t)batch : 0);
   if (int st = ptx_coded_forward(object, coded_surface, transfer_1, transfer_2, n, shifts_xy, batch, downsample, xf,
                                  sensor, amp, p, inner, stream)) {
     return st;
   }
-  cudaMemsetAsync(loss, 0, sizeof(double), s);
   const long long total = (long long)batch * h * h;
   if (total > 0) {
     prof_begin(kMiscKernel, s);
-    fd_loss_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, s>>>(amp, measured, scale, total, h, h,
-                                                                            isotropic, gamp, loss);
+    launch_pdl(fd_loss_kernel, static_cast<unsigned>((total + 255) / 256), 256, 0, s, amp, measured, scale, total,
+               h, h, isotropic, gamp, loss);
     prof_end(kMiscKernel, s);
   }
-  // the backward reuses the forward's region of the workspace, whose object spectrum the
-  // shift gradient reads
-  if (grad_shifts) cudaMemsetAsync(grad_shifts, 0, sizeof(double) * 2 * (size_t)batch, s);
   return coded_backward_impl(gamp, xf, sensor, amp, coded_surface, transfer_1, transfer_2, n, shifts_xy, batch,
-                             downsample, grad_object, grad_coded, p, inner, stream, grad_shifts);
+                             downsample, grad_object, grad_coded, p, inner, stream, grad_shifts, false);
 }
 
 int ptx_coded_sweep_fd(const float* object, const float* coded_surface, const float* transfer_1,

@@ -141,6 +141,7 @@ __global__ void __launch_bounds__(256, 2) fpm_cols(
     double inv_numel,
     double* __restrict__ loss, float2* __restrict__ image_out, float* __restrict__ amplitude,
     const float* __restrict__ grad_output) {
+  pdl_wait();
   using S = RegShape<NH>;
   using CP = ColPass<NH>;
   extern __shared__ float2 sm[];
@@ -480,8 +481,8 @@ void launch_rows_forward(const FpmGeom& g, const float2* spec, const float2* pup
     const int rowgroups = (g.lh + lines - 1) / lines;
     const int threads = lines * RowPass<N>::T, smem = FpmRowCfg<N>::smem(lines);
     const int grid = persistent_grid((const void*)fpm_rows_forward<N>, threads, smem, (long long)rowgroups * nf);
-    launch_pdl(fpm_rows_forward<N>, grid, threads, smem, s, spec, g.oh, g.ow, pupil, g.lh, led, nf, rowgroups, g.frames,
-                                                    g.p_lw.tw, lines);
+    launch_pdl(fpm_rows_forward<N>, grid, threads, smem, s, spec, g.oh, g.ow, pupil, g.lh, led, nf, rowgroups,
+               g.frames, g.p_lw.tw, lines);
   });
   prof_end(kFpmRowsForward, s);
 }
@@ -514,9 +515,8 @@ void launch_cols(const FpmGeom& g, int frame0, int nf, const uint16_t* measured,
       return;
     }
     dim3 grid(num_tiles(g.lw) * (kTile / kColsPerCta), nf);
-    fpm_cols<MODE, N><<<grid, ColPass<N>::kThreads, ColPass<N>::kSmemBytes, s>>>(
-        g.frames, g.lw, frame0, g.p_lh.tw, measured, g.lut, norm, grad_scale, inv_numel, loss, image, amplitude,
-        grad_output);
+    launch_pdl(fpm_cols<MODE, N>, grid, ColPass<N>::kThreads, ColPass<N>::kSmemBytes, s, g.frames, g.lw, frame0,
+               g.p_lh.tw, measured, g.lut, norm, grad_scale, inv_numel, loss, image, amplitude, grad_output);
   });
   prof_end(kFpmCols, s);
 }
@@ -538,8 +538,8 @@ void launch_rows_adjoint(const FpmGeom& g, const float2* spec, const float2* pup
     const int rowgroups = (g.lh + lines - 1) / lines;
     const int threads = lines * RowPass<N>::T, smem = FpmRowCfg<N>::smem(lines);
     const int grid = persistent_grid((const void*)fpm_rows_adjoint<N>, threads, smem, (long long)rowgroups * nf);
-    launch_pdl(fpm_rows_adjoint<N>, grid, threads, smem, s, g.frames, spec, g.oh, g.ow, pupil, g.lh, led, nf, rowgroups,
-                                                    norm, grad_spec, grad_pupil, g.p_lw.tw, lines);
+    launch_pdl(fpm_rows_adjoint<N>, grid, threads, smem, s, g.frames, spec, g.oh, g.ow, pupil, g.lh, led, nf,
+               rowgroups, norm, grad_spec, grad_pupil, g.p_lw.tw, lines);
   });
   prof_end(kFpmRowsAdjoint, s);
 }
@@ -593,8 +593,8 @@ int ptx_fpm_backward(const float* grad_output, const float* image, const float* 
     return set_error(PTX_ERR_INVALID_ARGUMENT, "null pointer argument");
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  cudaMemsetAsync(g.gspec, 0, g.spec_bytes, s);
-  cudaMemsetAsync(grad_pupil, 0, sizeof(float2) * (size_t)low_h * low_w, s);
+  launch_prologue(s, g.gspec, g.spec_bytes / sizeof(float2), reinterpret_cast<float2*>(grad_pupil),
+                  (size_t)low_h * low_w, nullptr, nullptr, nullptr, 0.f);
   const float2* spec = reinterpret_cast<const float2*>(spectrum);
   const float2* P = reinterpret_cast<const float2*>(pupil);
   float2* GP = reinterpret_cast<float2*>(grad_pupil);
@@ -624,13 +624,8 @@ int ptx_fpm_sweep(const float* object, int object_h, int object_w, const float* 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const double numel = (double)batch * low_h * low_w;
   const float grad_scale = static_cast<float>(2.0 / std::max(numel, 1.0));
-  {
-    const size_t ns = g.spec_bytes / sizeof(float2), np = (size_t)low_h * low_w;
-    prof_begin(kMiscKernel, s);
-    launch_pdl(sweep_prologue_kernel, prologue_blocks(ns, sm_count()), 256, 0, s,
-        g.gspec, ns, reinterpret_cast<float2*>(grad_pupil), np, loss, nullptr, g.lut, scale);
-    prof_end(kMiscKernel, s);
-  }
+  launch_prologue(s, g.gspec, g.spec_bytes / sizeof(float2), reinterpret_cast<float2*>(grad_pupil),
+                  (size_t)low_h * low_w, loss, nullptr, g.lut, scale);
   launch_fft2<false>(g, reinterpret_cast<const float2*>(object), object_h, object_w, g.spec, 1.0f, g.tmp, g.p_ow, g.p_oh,
                      s);
   const float2* P = reinterpret_cast<const float2*>(pupil);

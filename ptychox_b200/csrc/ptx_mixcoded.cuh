@@ -54,6 +54,7 @@ __device__ __forceinline__ size_t frame_elem(int f, int r, int c) {
 // (float2 atomics) and, with grad_shifts, dL/d(dx, dy) += -2 pi sum (fx, fy) Im(conj(G) u).
 template <int STAGE, bool CONJ, int N>
 __global__ void __launch_bounds__(ColCfg<N>::THREADS) mix_coded_cols(MixCodedArgs a) {
+  pdl_wait();
   using Cfg = ColCfg<N>;
   constexpr int A = Cfg::A, B = Cfg::B, C = Cfg::C;
   extern __shared__ float2 sm[];
@@ -153,6 +154,7 @@ __global__ void __launch_bounds__(ColCfg<N>::THREADS) mix_coded_cols(MixCodedArg
 // inverse row DFT, x = . / n (stored to xstore), a = x M, forward row DFT.
 template <int N>
 __global__ void __launch_bounds__(RowCfg<N>::THREADS) mix_coded_rows_mask(MixCodedArgs a, int lines) {
+  pdl_wait();
   using Cfg = RowCfg<N>;
   constexpr int A = Cfg::A, B = Cfg::B;
   extern __shared__ float2 sm[];
@@ -196,6 +198,7 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS) mix_coded_rows_mask(MixCod
 // amplitude.  kMixColBackward: g_s from the saved s, amplitude and grad_output, forward DFT.
 template <int MODE, int N>
 __global__ void __launch_bounds__(512) mix_coded_rows_pool(MixCodedArgs a, int lines) {
+  pdl_wait();
   using Cfg = RowCfg<N>;
   constexpr int A = Cfg::A, B = Cfg::B;
   extern __shared__ float2 sm[];
@@ -292,6 +295,7 @@ __global__ void __launch_bounds__(512) mix_coded_rows_pool(MixCodedArgs a, int l
 // inverse row DFT (g_a), grad_M += g_a conj(x) (float2 atomics), g_a conj(M), forward DFT.
 template <int N>
 __global__ void __launch_bounds__(RowCfg<N>::THREADS) mix_coded_rows_grad_mask(MixCodedArgs a, int lines) {
+  pdl_wait();
   using Cfg = RowCfg<N>;
   constexpr int A = Cfg::A, B = Cfg::B;
   extern __shared__ float2 sm[];
@@ -362,28 +366,28 @@ struct Ops {
     if (a.nframes <= 0) return;
     dim3 grid(num_tiles(N) * (kTile / CC::C), a.nframes);
     if (stage == 1) {
-      mix_coded_cols<1, false, N><<<grid, CC::THREADS, CC::SMEM, s>>>(a);
+      launch_pdl(mix_coded_cols<1, false, N>, grid, CC::THREADS, CC::SMEM, s, a);
     } else if (stage == 3) {
       if (conj) {
-        mix_coded_cols<3, true, N><<<grid, CC::THREADS, CC::SMEM, s>>>(a);
+        launch_pdl(mix_coded_cols<3, true, N>, grid, CC::THREADS, CC::SMEM, s, a);
       } else {
-        mix_coded_cols<3, false, N><<<grid, CC::THREADS, CC::SMEM, s>>>(a);
+        launch_pdl(mix_coded_cols<3, false, N>, grid, CC::THREADS, CC::SMEM, s, a);
       }
     } else {
-      mix_coded_cols<7, false, N><<<grid, CC::THREADS, CC::SMEM, s>>>(a);
+      launch_pdl(mix_coded_cols<7, false, N>, grid, CC::THREADS, CC::SMEM, s, a);
     }
   }
   static void rows_mask(const MixCodedArgs& a, cudaStream_t s) {
     if (a.nframes <= 0) return;
     const int lines = row_lines();
     dim3 grid(a.nframes, (N + lines - 1) / lines);
-    mix_coded_rows_mask<N><<<grid, lines * RC::B, RC::smem_forward(lines), s>>>(a, lines);
+    launch_pdl(mix_coded_rows_mask<N>, grid, lines * RC::B, RC::smem_forward(lines), s, a, lines);
   }
   static void rows_grad_mask(const MixCodedArgs& a, cudaStream_t s) {
     if (a.nframes <= 0) return;
     const int lines = row_lines();
     dim3 grid(a.nframes, (N + lines - 1) / lines);
-    mix_coded_rows_grad_mask<N><<<grid, lines * RC::B, RC::smem_forward(lines), s>>>(a, lines);
+    launch_pdl(mix_coded_rows_grad_mask<N>, grid, lines * RC::B, RC::smem_forward(lines), s, a, lines);
   }
   static void rows_pool(int mode, const MixCodedArgs& a, cudaStream_t s) {
     if (a.nframes <= 0) return;
@@ -391,11 +395,11 @@ struct Ops {
     dim3 grid((N + lines - 1) / lines, a.nframes);
     const int threads = lines * RC::B, smem = pool_smem(lines);
     if (mode == kMixColSweep) {
-      mix_coded_rows_pool<kMixColSweep, N><<<grid, threads, smem, s>>>(a, lines);
+      launch_pdl(mix_coded_rows_pool<kMixColSweep, N>, grid, threads, smem, s, a, lines);
     } else if (mode == kMixColForward) {
-      mix_coded_rows_pool<kMixColForward, N><<<grid, threads, smem, s>>>(a, lines);
+      launch_pdl(mix_coded_rows_pool<kMixColForward, N>, grid, threads, smem, s, a, lines);
     } else {
-      mix_coded_rows_pool<kMixColBackward, N><<<grid, threads, smem, s>>>(a, lines);
+      launch_pdl(mix_coded_rows_pool<kMixColBackward, N>, grid, threads, smem, s, a, lines);
     }
   }
   static const MixCodedOps* table() {

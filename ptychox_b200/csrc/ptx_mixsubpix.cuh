@@ -54,6 +54,7 @@ struct RowCfg {
 // windows outside the object are skipped).
 template <int N, bool GATHER>
 __global__ void __launch_bounds__(ColCfg<N>::THREADS) mix_subpix_cols(MixSubpixArgs a) {
+  pdl_wait();
   using Cfg = ColCfg<N>;
   constexpr int A = Cfg::A, B = Cfg::B, C = Cfg::C;
   extern __shared__ float2 sm[];
@@ -117,6 +118,7 @@ __global__ void __launch_bounds__(ColCfg<N>::THREADS) mix_subpix_cols(MixSubpixA
 // element per CTA at the end), G conj(P), row DFT, x conj(ramp_x), inverse DFT, stored.
 template <int M, bool FORWARD, bool STORE_S, bool STORE_OUT>
 __global__ void __launch_bounds__(RowCfg<M>::THREADS) mix_subpix_rows(MixSubpixArgs a, int lines, int fpc) {
+  pdl_wait();
   using Cfg = RowCfg<M>;
   constexpr int A = Cfg::A, B = Cfg::B, P = Cfg::P;
   extern __shared__ float2 sm[];
@@ -235,7 +237,7 @@ struct Ops {
     int fpc = static_cast<int>(std::max<long long>(1, ((long long)rowgroups * a.nframes) / target));
     fpc = std::min(fpc, std::max(a.nframes, 1));
     dim3 grid(rowgroups, (a.nframes + fpc - 1) / fpc);
-    mix_subpix_rows<N, F, S, O><<<grid, lines * RC::B, RC::smem(lines, !F), s>>>(a, lines, fpc);
+    launch_pdl(mix_subpix_rows<N, F, S, O>, grid, lines * RC::B, RC::smem(lines, !F), s, a, lines, fpc);
   }
   static int prepare() {
     const int rs = RC::smem(RC::LINES, true);
@@ -251,9 +253,9 @@ struct Ops {
     if (a.nframes <= 0) return;
     dim3 grid(num_tiles(a.pw) * (kTile / CC::C), a.nframes);
     if (gather) {
-      mix_subpix_cols<N, true><<<grid, CC::THREADS, CC::SMEM, s>>>(a);
+      launch_pdl(mix_subpix_cols<N, true>, grid, CC::THREADS, CC::SMEM, s, a);
     } else {
-      mix_subpix_cols<N, false><<<grid, CC::THREADS, CC::SMEM, s>>>(a);
+      launch_pdl(mix_subpix_cols<N, false>, grid, CC::THREADS, CC::SMEM, s, a);
     }
   }
   static void rows(int variant, const MixSubpixArgs& a, cudaStream_t s) {

@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <stdint.h>
 
+#include "ptx_internal.h"
 #include "ptx_pairfft.cuh"
 #include "ptx_regfft.cuh"
 
@@ -84,18 +85,21 @@ static __global__ void decode_lut_kernel(float* __restrict__ lut, float scale) {
   if (c < kLutEntries) lut[c] = sqrtf(static_cast<float>(c) * scale);
 }
 
-// One launch for everything a sweep resets before its passes: zero two gradient arrays
-// (n_a and n_b complex elements), the FP64 loss and the error word, and (lut non-null)
-// build the count-decode table.  Grid-stride; any grid size works.
+// One launch for everything a sweep (or an adjoint: no loss, no table) resets before its
+// passes: zero two gradient arrays (n_a and n_b complex elements), the FP64 loss, the error word
+// and n_c doubles, and (lut non-null) build the count-decode table.  Grid-stride; any grid size
+// works.
 static __global__ void sweep_prologue_kernel(float2* __restrict__ zero_a, size_t n_a, float2* __restrict__ zero_b,
                                              size_t n_b, double* __restrict__ loss, unsigned* __restrict__ err,
-                                             float* __restrict__ lut, float scale) {
+                                             float* __restrict__ lut, float scale, double* __restrict__ zero_c,
+                                             size_t n_c) {
   pdl_wait();
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const float2 z = make_float2(0.f, 0.f);
   for (size_t i = i0; i < n_a; i += stride) zero_a[i] = z;
   for (size_t i = i0; i < n_b; i += stride) zero_b[i] = z;
+  for (size_t i = i0; i < n_c; i += stride) zero_c[i] = 0.0;
   if (lut) {
     for (size_t c = i0; c < (size_t)kLutEntries; c += stride) lut[c] = sqrtf(static_cast<float>(c) * scale);
   }
@@ -109,6 +113,14 @@ static __global__ void sweep_prologue_kernel(float2* __restrict__ zero_a, size_t
 inline unsigned prologue_blocks(size_t elements, int sms) {
   const size_t want = (elements / 8 + 255) / 256;
   return static_cast<unsigned>(std::max<size_t>(1, std::min<size_t>(want, (size_t)sms * 8 * 4)));
+}
+
+inline void launch_prologue(cudaStream_t s, float2* zero_a, size_t n_a, float2* zero_b, size_t n_b, double* loss,
+                            unsigned* err, float* lut, float scale, double* zero_c = nullptr, size_t n_c = 0) {
+  prof_begin(kMiscKernel, s);
+  launch_pdl(sweep_prologue_kernel, prologue_blocks(std::max(n_a, n_b), sm_count()), 256, 0, s, zero_a, n_a, zero_b, n_b,
+             loss, err, lut, scale, zero_c, n_c);
+  prof_end(kMiscKernel, s);
 }
 
 // 1/sqrt(s), s > 0: the rsqrtf estimate refined by one Newton-Raphson step for the

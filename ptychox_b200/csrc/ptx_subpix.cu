@@ -51,6 +51,7 @@ __device__ __forceinline__ bool sp_window_ok(long long x0, long long y0, int ph,
 // (bit 0 of *err) every window that leaves the object.
 __global__ void subpix_ramp_kernel(const double* __restrict__ pos, int nframes, int ph, int pw, int H, int W,
                                    float2* __restrict__ rx, float2* __restrict__ ry, unsigned* __restrict__ err) {
+  pdl_wait();
   const long long per = (long long)pw + ph;
   const long long total = per * nframes;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -90,6 +91,7 @@ __global__ void __launch_bounds__(kSpCols * RegShape<N>::T) subpix_cols_kernel(
     const float2* __restrict__ sample, float2* __restrict__ grad_sample, int H, int W, int pw,
     const double* __restrict__ pos, int frame0, float2* __restrict__ scratch, const float2* __restrict__ ry_all,
     const float2* __restrict__ tw) {
+  pdl_wait();
   using S = RegShape<N>;
   constexpr int LP = col_line_pitch<N>();
   extern __shared__ float2 sm[];
@@ -152,6 +154,7 @@ __global__ void __launch_bounds__(kSpRowThreads) subpix_rows_kernel(
     float2* __restrict__ scratch, float2* __restrict__ sbuf, int ph, const float2* __restrict__ probe, int nframes,
     int frame0, int frames_per_cta, const float2* __restrict__ rx_all, float2* __restrict__ grad_probe,
     const float2* __restrict__ tw, int lines) {
+  pdl_wait();
   using S = RegShape<M>;
   constexpr int LP = row_line_pitch<M>();
   constexpr int kTiles = M / kTile;
@@ -306,7 +309,7 @@ void sp_launch_ramps(const SpGeom& g, const double* pos, cudaStream_t s) {
   const long long total = (long long)g.batch * (g.ph + g.pw);
   const int blocks = static_cast<int>(std::min<long long>((total + 255) / 256, (long long)sm_count() * 8));
   prof_begin(kMiscKernel, s);
-  subpix_ramp_kernel<<<blocks, 256, 0, s>>>(pos, g.batch, g.ph, g.pw, g.H, g.W, g.rx, g.ry, g.err);
+  launch_pdl(subpix_ramp_kernel, blocks, 256, 0, s, pos, g.batch, g.ph, g.pw, g.H, g.W, g.rx, g.ry, g.err);
   prof_end(kMiscKernel, s);
 }
 
@@ -352,8 +355,8 @@ int sp_launch_cols(const SpGeom& g, const float2* sample, float2* grad_sample, c
       if (st) return;
       dim3 grid(num_tiles(g.pw) * (kTile / kSpCols), nf);
       prof_begin(kSubpixCols, s);
-      subpix_cols_kernel<N, GATHER><<<grid, threads, smem, s>>>(sample, grad_sample, g.H, g.W, g.pw, pos, frame0,
-                                                                g.scratch, g.ry, g.col.tw);
+      launch_pdl(subpix_cols_kernel<N, GATHER>, grid, threads, smem, s, sample, grad_sample, g.H, g.W, g.pw, pos,
+                 frame0, g.scratch, g.ry, g.col.tw);
       prof_end(kSubpixCols, s);
     }
   });
@@ -391,8 +394,8 @@ int sp_launch_rows(const SpGeom& g, const float2* probe, float2* grad_probe, int
       fpc = std::min(fpc, std::max(nf, 1));
       dim3 grid(rowgroups, (nf + fpc - 1) / fpc);
       prof_begin(kSubpixRows, s);
-      kern<<<grid, lines * RegShape<M>::T, smem, s>>>(g.scratch, g.sbuf, g.ph, probe, nf, frame0, fpc, g.rx,
-                                                      grad_probe, g.row.tw, lines);
+      launch_pdl(kern, grid, lines * RegShape<M>::T, smem, s, g.scratch, g.sbuf, g.ph, probe, nf, frame0, fpc, g.rx,
+                 grad_probe, g.row.tw, lines);
       prof_end(kSubpixRows, s);
     }
   });
@@ -419,9 +422,8 @@ int sp_launch_cols_sweep(const SpGeom& g, int frame0, int nf, const uint16_t* me
       if (st) return;
       dim3 grid(num_tiles(g.pw), nf);
       prof_begin(kBaseCols, s);
-      kern<<<grid, ColPairCfg<N>::kThreads, ColPairCfg<N>::kSmemBytes, s>>>(g.scratch, g.pw, frame0, g.col.tw,
-                                                                            measured, g.lut, 1.0f, grad_scale,
-                                                                            inv_numel, loss);
+      launch_pdl(kern, grid, ColPairCfg<N>::kThreads, ColPairCfg<N>::kSmemBytes, s, g.scratch, g.pw, frame0,
+                 g.col.tw, measured, g.lut, 1.0f, grad_scale, inv_numel, loss);
       prof_end(kBaseCols, s);
     }
   });
@@ -463,12 +465,7 @@ int ptx_base_subpix_sweep(const float* sample, int sample_h, int sample_w, const
   const float2* P = reinterpret_cast<const float2*>(probe);
   const double numel = (double)batch * probe_h * probe_w;
   const float grad_scale = static_cast<float>(2.0 / std::max(numel, 1.0));
-  {
-    const size_t ns = (size_t)sample_h * sample_w, np = (size_t)probe_h * probe_w;
-    prof_begin(kMiscKernel, s);
-    sweep_prologue_kernel<<<prologue_blocks(ns, sm_count()), 256, 0, s>>>(GS, ns, GP, np, loss, g.err, g.lut, scale);
-    prof_end(kMiscKernel, s);
-  }
+  launch_prologue(s, GS, (size_t)sample_h * sample_w, GP, (size_t)probe_h * probe_w, loss, g.err, g.lut, scale);
   sp_launch_ramps(g, positions_xy, s);
   for (int b0 = 0; b0 < batch; b0 += g.chunk) {
     const int nf = std::min(g.chunk, batch - b0);
@@ -524,9 +521,7 @@ int ptx_base_subpix_backward(const float* grad_output, const float* far_field, c
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   float2* GS = reinterpret_cast<float2*>(grad_sample);
   float2* GP = reinterpret_cast<float2*>(grad_probe);
-  cudaMemsetAsync(GS, 0, sizeof(float2) * (size_t)sample_h * sample_w, s);
-  cudaMemsetAsync(GP, 0, sizeof(float2) * (size_t)probe_h * probe_w, s);
-  cudaMemsetAsync(g.err, 0, sizeof(unsigned), s);
+  launch_prologue(s, GS, (size_t)sample_h * sample_w, GP, (size_t)probe_h * probe_w, nullptr, g.err, nullptr, 0.f);
   sp_launch_ramps(g, positions_xy, s);
   const float2* S = reinterpret_cast<const float2*>(sample);
   const float2* P = reinterpret_cast<const float2*>(probe);

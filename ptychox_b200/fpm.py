@@ -13,8 +13,8 @@ from __future__ import annotations
 import torch
 
 from . import _abi
-from ._utils import (as_u16, check_complex_scan_inputs, ptr, require_cuda_complex64, stream_handle, upload_small,
-                     workspace)
+from ._utils import (as_u16, check_complex_scan_inputs, ptr, require_cuda_complex64, scaled_gradients, stream_handle,
+                     upload_small, workspace)
 
 __all__ = [
     "ptychoX_fourier",
@@ -120,9 +120,8 @@ class PtychoXFPMLossFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_loss):  # type: ignore[override]
-        go, gp = ctx.saved_tensors
-        g = grad_loss.to(torch.float32)
-        return go * g, gp * g, None, None, None
+        go, gp = scaled_gradients(grad_loss, *ctx.saved_tensors)
+        return go, gp, None, None, None
 
 
 def ptychoX_fourier_loss(object_field, pupil, led_indices_xy, measured, scale) -> torch.Tensor:
