@@ -180,6 +180,16 @@ int ptx_base_sweep_small(const float* sample, int sample_h, int sample_w,
  * with device-resident positions learns of a bad window without copying the positions to
  * the host.  Read it after the stream has reached the copy and map it with ptx_status_code. */
 int ptx_workspace_status(const void* workspace, unsigned* status, void* stream);
+
+/* The same check deferred and without a host synchronisation: ptx_status_track copies the status
+ * word of `workspace` (of the call just queued on `stream`, current device) in stream order into
+ * a page-locked word of the library and records an event behind it; ptx_status_poll retires the
+ * tracked calls of `device` (all devices if negative) whose copies have completed, or waits for
+ * all of them with `block`.  Both put the `tag` (>= 0) of the first retired call with a window
+ * outside the object, or -1, into *failed (ptx_status_track retires calls only when 255 of them
+ * are pending).  Calls on a capturing stream are not tracked. */
+int ptx_status_track(const void* workspace, int tag, int* failed, void* stream);
+int ptx_status_poll(int device, int block, int* failed);
 /* PTX_ERR_OUT_OF_BOUNDS when bit 0 of a status word is set, else PTX_OK. */
 int ptx_status_code(unsigned status);
 

@@ -77,6 +77,8 @@ SIGNATURES: dict[str, tuple] = {
     "ptx_adam_step": (_i, [_p, _p, _p, _p, _sz, _p, _f, _f, _f, _f, _i, _p]),
     "ptx_base_sweep_noalloc": (_i, [_p, _i, _i, _p, _i, _i, _p, _i, _p, _f, _p, _p, _p, _p]),
     "ptx_workspace_status": (_i, [_p, _p, _p]),
+    "ptx_status_track": (_i, [_p, _i, C.POINTER(_i), _p]),
+    "ptx_status_poll": (_i, [_i, _i, C.POINTER(_i)]),
     "ptx_status_code": (_i, [C.c_uint]),
     "ptx_reg_workspace_bytes": (_sz, [_i, _i, _i, _i]),
     "ptx_reg_upsampled_peak": (_i, [_p, _i, _i, _i, _i, _p, _p, _p, _p, _p, _sz, _p]),
@@ -141,13 +143,22 @@ def check(status: int, what: str) -> None:
     raise PtychoXError(msg)
 
 
+_functions: dict[str, object] = {}  # looked up once: an attribute of a CDLL costs a dictionary miss
+
+
+def _function(name: str):
+    fn = _functions[name] = getattr(load(), name)
+    return fn
+
+
 def call(name: str, *args) -> None:
-    fn = getattr(load(), name)
-    check(fn(*args), name)
+    status = (_functions.get(name) or _function(name))(*args)
+    if status != PTX_OK:
+        check(status, name)
 
 
 def query(name: str, *args):
-    return getattr(load(), name)(*args)
+    return (_functions.get(name) or _function(name))(*args)
 
 
 def profile_read() -> dict[str, tuple[float, int]]:

@@ -19,20 +19,17 @@ Calls made while a stream is being captured into a CUDA graph are not tracked.
 
 from __future__ import annotations
 
-import threading
-from collections import deque
+import ctypes
 
 import torch
 
 from . import _abi
+from ._utils import stream_handle
 
 _MODES = ("deferred", "sync", "host")
 _mode = "deferred"
-_lock = threading.Lock()
-_pending: deque = deque()  # (device index, event, slot index, what)
-_slots: dict[int, torch.Tensor] = {}  # device -> pinned uint32 ring
-_next_slot: dict[int, int] = {}
-_RING = 256
+_calls: list[str] = []  # names of the tracked operators; a tracked call's tag is its index here
+_tags: dict[str, int] = {}
 
 
 def set_bounds_check(mode: str) -> None:
@@ -53,69 +50,38 @@ def _raise_for(what: str) -> None:
                      "positions must satisfy 0 <= x <= W - pw and 0 <= y <= H - ph.")
 
 
-def _slot(dev: int) -> tuple[torch.Tensor, int]:
-    ring = _slots.get(dev)
-    if ring is None:
-        ring = torch.zeros(_RING, dtype=torch.int32).pin_memory()
-        _slots[dev] = ring
-        _next_slot[dev] = 0
-    k = _next_slot[dev]
-    _next_slot[dev] = (k + 1) % _RING
-    return ring, k
-
-
-def _drain(block: bool, device: int | None = None) -> None:
-    """Retire pending checks in order (all, or those of `device`); raise for the first failure.
-    With block=False stop at the first check whose copy has not completed."""
-    failed = None
-    with _lock:
-        keep = deque()
-        while _pending:
-            dev, ev, k, what = _pending.popleft()
-            if device is not None and dev != device:
-                keep.append((dev, ev, k, what))
-                continue
-            if not ev.query():
-                if not block:
-                    keep.append((dev, ev, k, what))
-                    keep.extend(e for e in _pending)
-                    _pending.clear()
-                    break
-                ev.synchronize()
-            if failed is None and int(_slots[dev][k]) & 1:
-                failed = what
-        _pending.extend(keep)
-    if failed is not None:
-        _raise_for(failed)
+def _poll(device: int, block: bool) -> None:
+    """Retire tracked calls of `device` (all when negative); raise for the first failure."""
+    if not _calls:
+        return
+    failed = ctypes.c_int(-1)
+    _abi.call("ptx_status_poll", device, int(block), failed)
+    if failed.value >= 0:
+        _raise_for(_calls[failed.value])
 
 
 def check_errors(block: bool = True) -> None:
     """Raise ``ValueError`` if an earlier conventional call with device positions met a window
     outside the object (waits for their status copies when ``block``)."""
-    _drain(block)
+    _poll(-1, block)
 
 
 def before_call(device: torch.device) -> None:
     """Report completed failures of earlier calls on `device` (non-blocking)."""
-    if _pending:
-        _drain(False, device.index)
+    if _calls and device.index is not None:
+        _poll(device.index, False)
 
 
 def after_call(workspace: torch.Tensor, device: torch.device, what: str) -> None:
-    """Queue the status copy of the call that just used `workspace` (device positions only)."""
-    stream = torch.cuda.current_stream(device)
-    with torch.cuda.device(device):
-        if torch.cuda.is_current_stream_capturing():
-            return
-    dev = device.index if device.index is not None else torch.cuda.current_device()
-    if len(_pending) >= _RING - 1:
-        _drain(True)
-    with _lock:
-        ring, k = _slot(dev)
-        ring[k] = 0
-        _abi.call("ptx_workspace_status", workspace.data_ptr(), ring.data_ptr() + 4 * k, stream.cuda_stream)
-        ev = torch.cuda.Event()
-        ev.record(stream)
-        _pending.append((dev, ev, k, what))
+    """Queue the status copy of the call that just used `workspace` (device positions only);
+    `device` is current."""
+    tag = _tags.get(what)
+    if tag is None:
+        _calls.append(what)
+        tag = _tags[what] = _calls.index(what)
+    failed = ctypes.c_int(-1)
+    _abi.call("ptx_status_track", workspace.data_ptr(), tag, failed, stream_handle(device))
+    if failed.value >= 0:
+        _raise_for(_calls[failed.value])
     if _mode == "sync":
-        _drain(True, dev)
+        _poll(device.index if device.index is not None else torch.cuda.current_device(), True)

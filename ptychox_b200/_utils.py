@@ -8,6 +8,8 @@ validated against the object bounds, stream and workspace plumbing.
 
 from __future__ import annotations
 
+import contextlib
+
 import torch
 
 from . import _abi
@@ -119,27 +121,33 @@ def upload_small(t: torch.Tensor, device: torch.device, dtype: torch.dtype) -> t
     host = t.detach().to(dtype=dtype).contiguous()
     out = torch.empty(host.shape, dtype=dtype, device=device)
     if host.numel():
-        args = (out.data_ptr(), host.data_ptr(), host.numel() * host.element_size())
-        if out.device.index == torch.cuda.current_device():
-            _abi.call("ptx_stage_host_bytes", *args, stream_handle(out.device))
-        else:
-            with torch.cuda.device(out.device):
-                _abi.call("ptx_stage_host_bytes", *args, stream_handle(out.device))
+        call_on(out.device, "ptx_stage_host_bytes", out.data_ptr(), host.data_ptr(), host.numel() * host.element_size())
     return out
+
+
+# the current stream's handle without a Stream object around it, where torch has that call
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 def stream_handle(device: torch.device) -> int:
     """The current stream of `device` as the integer handle the library takes."""
-    return torch.cuda.current_stream(device).cuda_stream
+    if _raw_stream is None or device.index is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    return _raw_stream(device.index)
+
+
+_already_there = contextlib.nullcontext()
+
+
+def on_device(device: torch.device):
+    """Context with `device` current; costs nothing to speak of where it already is."""
+    return _already_there if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
 def call_on(device: torch.device, name: str, *args) -> None:
     """Library call with the current stream of `device` as its last argument, `device` current."""
-    if torch.cuda.current_device() == device.index:
+    with on_device(device):
         _abi.call(name, *args, stream_handle(device))
-    else:
-        with torch.cuda.device(device):
-            _abi.call(name, *args, stream_handle(device))
 
 
 def workspace(nbytes: int, device: torch.device) -> torch.Tensor:

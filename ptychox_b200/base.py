@@ -20,6 +20,7 @@ from ._utils import (
     check_complex_scan_inputs,
     device_positions,
     device_positions_subpixel,
+    on_device,
     ptr,
     require_cuda_complex64,
     scaled_gradients,
@@ -87,7 +88,7 @@ class PtychoXBaseFunction(torch.autograd.Function):
         amp = torch.empty((batch, ph, pw), dtype=torch.float32, device=dev)
         ws_bytes = _abi.query("ptx_base_workspace_bytes", ph, pw, batch)
         ws = workspace(ws_bytes, dev)
-        with torch.cuda.device(dev):
+        with on_device(dev):
             _abi.call("ptx_base_forward", ptr(sample), sample.shape[0], sample.shape[1], ptr(probe), ph, pw,
                       ptr(pos), batch, ptr(far), ptr(amp), ptr(ws), ws_bytes, stream_handle(dev))
             if track and batch:
@@ -106,7 +107,7 @@ class PtychoXBaseFunction(torch.autograd.Function):
         grad_probe = torch.empty_like(probe)
         ws_bytes = _abi.query("ptx_base_workspace_bytes", ph, pw, batch)
         ws = workspace(ws_bytes, dev)
-        with torch.cuda.device(dev):
+        with on_device(dev):
             _abi.call("ptx_base_backward", ptr(grad_output), ptr(far), ptr(sample), sample.shape[0],
                       sample.shape[1], ptr(probe), ph, pw, ptr(pos), batch, ptr(grad_sample), ptr(grad_probe),
                       ptr(ws), ws_bytes, stream_handle(dev))
@@ -141,7 +142,7 @@ def base_sweep(sample, probe, positions, measured, scale, ws=None):
         ws = workspace(_abi.query("ptx_base_workspace_bytes", ph, pw, batch), dev)
     # square 32 / 64 / 128 probes: the one-CTA-per-frame sweep (frame resident in shared memory)
     entry = "ptx_base_sweep_small" if use_small_sweep(ph, pw, batch) else "ptx_base_sweep"
-    with torch.cuda.device(dev):
+    with on_device(dev):
         _abi.call(entry, ptr(sample), sample.shape[0], sample.shape[1], ptr(probe), ph, pw,
                   ptr(positions), batch, ptr(measured), float(scale), ptr(loss), ptr(gs), ptr(gp), ptr(ws),
                   ws.numel(), stream_handle(dev))
@@ -159,7 +160,7 @@ class PtychoXBaseLossFunction(torch.autograd.Function):
         ws = workspace(_abi.query("ptx_base_workspace_bytes", probe.shape[0], probe.shape[1], pos.shape[0]), dev)
         loss, gs, gp = base_sweep(sample, probe, pos, meas, scale, ws=ws)
         if track and pos.shape[0]:
-            with torch.cuda.device(dev):
+            with on_device(dev):
                 _status.after_call(ws, dev, "ptychoX_base_loss")
         ctx.save_for_backward(gs, gp)
         return loss
@@ -222,7 +223,7 @@ def base_subpixel_sweep(sample, probe, positions, measured, scale, ws=None):
     gp = torch.empty_like(probe)
     if ws is None:
         ws = workspace(_subpixel_ws_bytes(ph, pw, batch), dev)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         _abi.call("ptx_base_subpix_sweep", ptr(sample), sample.shape[0], sample.shape[1], ptr(probe), ph, pw,
                   ptr(positions), batch, ptr(measured), float(scale), ptr(loss), ptr(gs), ptr(gp), ptr(ws), ws.numel(),
                   stream_handle(dev))
@@ -240,7 +241,7 @@ class PtychoXBaseSubpixelFunction(torch.autograd.Function):
         amp = torch.empty((batch, ph, pw), dtype=torch.float32, device=dev)
         ws_bytes = _subpixel_ws_bytes(ph, pw, batch)
         ws = workspace(ws_bytes, dev)
-        with torch.cuda.device(dev):
+        with on_device(dev):
             _abi.call("ptx_base_subpix_forward", ptr(sample), sample.shape[0], sample.shape[1], ptr(probe), ph, pw,
                       ptr(pos), batch, ptr(far), ptr(amp), ptr(ws), ws_bytes, stream_handle(dev))
             if track and batch:
@@ -259,7 +260,7 @@ class PtychoXBaseSubpixelFunction(torch.autograd.Function):
         grad_probe = torch.empty_like(probe)
         ws_bytes = _subpixel_ws_bytes(ph, pw, batch)
         ws = workspace(ws_bytes, dev)
-        with torch.cuda.device(dev):
+        with on_device(dev):
             _abi.call("ptx_base_subpix_backward", ptr(grad_output), ptr(far), ptr(sample), sample.shape[0],
                       sample.shape[1], ptr(probe), ph, pw, ptr(pos), batch, ptr(grad_sample), ptr(grad_probe),
                       ptr(ws), ws_bytes, stream_handle(dev))
@@ -278,7 +279,7 @@ class PtychoXBaseSubpixelLossFunction(torch.autograd.Function):
         ws = workspace(_subpixel_ws_bytes(ph, pw, pos.shape[0]), dev)
         loss, gs, gp = base_subpixel_sweep(sample, probe, pos, meas, scale, ws=ws)
         if track and pos.shape[0]:
-            with torch.cuda.device(dev):
+            with on_device(dev):
                 _status.after_call(ws, dev, "ptychoX_base_subpixel_loss")
         ctx.save_for_backward(gs, gp)
         return loss

@@ -19,7 +19,7 @@ from __future__ import annotations
 import torch
 
 from . import _abi
-from ._utils import as_u16, ptr, scaled_gradients, stream_handle, upload_small, workspace
+from ._utils import as_u16, on_device, ptr, scaled_gradients, stream_handle, upload_small, workspace
 
 __all__ = [
     "ptychoX_coded",
@@ -96,7 +96,7 @@ class PtychoXCodedFunction(torch.autograd.Function):
         sensor = torch.empty_like(xf)
         amp = torch.empty((batch, n // ds, n // ds), dtype=torch.float32, device=dev)
         ws, nb = _ws(n, batch, dev)
-        with torch.cuda.device(dev):
+        with on_device(dev):
             _abi.call("ptx_coded_forward", ptr(obj), ptr(mask), ptr(t1), ptr(t2), n, ptr(shifts), batch, ds,
                       ptr(xf), ptr(sensor), ptr(amp), ptr(ws), nb, stream_handle(dev))
         ctx.save_for_backward(xf, sensor, amp, mask, t2, shifts, *(() if t1 is None else (t1,)))
@@ -115,7 +115,7 @@ class PtychoXCodedFunction(torch.autograd.Function):
         grad_object = torch.empty_like(mask)
         grad_coded = torch.empty_like(mask)
         ws, nb = _ws(n, batch, dev)
-        with torch.cuda.device(dev):
+        with on_device(dev):
             _abi.call("ptx_coded_backward", ptr(grad_output), ptr(xf), ptr(sensor), ptr(amp), ptr(mask), ptr(t1),
                       ptr(t2), n, ptr(shifts), batch, ctx.downsample, ptr(grad_object), ptr(grad_coded), ptr(ws), nb,
                       stream_handle(dev))
@@ -186,12 +186,12 @@ def coded_sweep(obj, mask, t1, t2, shifts, downsample, measured, scale, ws=None,
         gs = torch.empty((batch, 2), dtype=torch.float64, device=dev)
         if ws is None:
             ws = workspace(_abi.query("ptx_coded_sweep_ex_workspace_bytes", n, batch, int(downsample), kind), dev)
-        with torch.cuda.device(dev):
+        with on_device(dev):
             _abi.call("ptx_coded_sweep_ex", ptr(obj), ptr(mask), ptr(t1), ptr(t2), n, ptr(shifts), batch,
                       int(downsample), ptr(measured), float(scale), kind, ptr(out), ptr(go), ptr(gm), ptr(gs),
                       ptr(ws), ws.numel(), stream_handle(dev))
         return out, go, gm, gs
-    with torch.cuda.device(dev):
+    with on_device(dev):
         if loss == "mse":
             if ws is None:
                 ws, _ = _ws(n, batch, dev)

@@ -334,6 +334,42 @@ int persistent_grid(const void* kernel, int threads, int smem, long long units) 
   return static_cast<int>(std::max<long long>(1, std::min<long long>(grid, std::max<long long>(units, 1))));
 }
 
+// Deferred window checks: one page-locked ring of status words per device, each filled by a copy
+// in stream order after the call it belongs to and retired, oldest first, once the event behind
+// the copy has completed.  Words and events live as long as the process (kStatusSlots of each per
+// device at most); everything runs under one lock.
+constexpr int kStatusSlots = 256;
+struct StatusRing {
+  unsigned* words = nullptr;
+  int next = 0;
+  struct Call {
+    cudaEvent_t done;
+    int slot, tag;
+  };
+  std::deque<Call> pending;
+  std::vector<cudaEvent_t> spare;
+};
+std::mutex g_status_mutex;
+std::map<int, StatusRing> g_status;
+
+// Retire the ring's completed calls (all of them, waiting, with `block`); the tag of the first
+// one whose window check failed goes to *failed if that is still negative.
+int retire_status(StatusRing& r, bool block, int* failed) {
+  while (!r.pending.empty()) {
+    const StatusRing::Call c = r.pending.front();
+    const cudaError_t e = block ? cudaEventSynchronize(c.done) : cudaEventQuery(c.done);
+    if (e == cudaErrorNotReady) {
+      cudaGetLastError();
+      return PTX_OK;
+    }
+    if (e != cudaSuccess) return cuda_status(e, "status event");
+    if (*failed < 0 && (r.words[c.slot] & 1u)) *failed = c.tag;
+    r.spare.push_back(c.done);
+    r.pending.pop_front();
+  }
+  return PTX_OK;
+}
+
 // out = z g for the complex arrays a and b and one real factor g of the device (the gradient of
 // the loss), rounded to FP32 first, with the complex product's handling of infinities and NaN.
 // One launch where a cast and one product per array were three; 16-byte accesses when both ends
@@ -607,6 +643,58 @@ int ptx_scale_gradients(const double* factor, const float* a, float* out_a, size
                   reinterpret_cast<float2*>(out_b), n_b);
   ptx::prof_end(ptx::kMiscKernel, s);
   return ptx::cuda_status(cudaGetLastError(), "ptx_scale_gradients launch");
+}
+
+int ptx_status_track(const void* workspace, int tag, int* failed, void* stream) {
+  if (!workspace || !failed || tag < 0) return ptx::set_error(PTX_ERR_INVALID_ARGUMENT, "invalid argument");
+  *failed = -1;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaError_t e = cudaStreamIsCapturing(s, &capture)) return ptx::cuda_status(e, "cudaStreamIsCapturing");
+  if (capture != cudaStreamCaptureStatusNone) return PTX_OK;
+  int dev = 0;
+  if (cudaError_t e = cudaGetDevice(&dev)) return ptx::cuda_status(e, "cudaGetDevice");
+  std::lock_guard<std::mutex> lock(ptx::g_status_mutex);
+  ptx::StatusRing& r = ptx::g_status[dev];
+  if (!r.words) {
+    void* p = nullptr;
+    if (cudaError_t e = cudaHostAlloc(&p, ptx::kStatusSlots * sizeof(unsigned), cudaHostAllocPortable)) {
+      return ptx::cuda_status(e, "cudaHostAlloc");
+    }
+    r.words = static_cast<unsigned*>(p);
+  }
+  if (r.pending.size() >= ptx::kStatusSlots - 1) {
+    if (int st = ptx::retire_status(r, true, failed)) return st;
+  }
+  cudaEvent_t ev = nullptr;
+  if (!r.spare.empty()) {
+    ev = r.spare.back();
+    r.spare.pop_back();
+  } else if (cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) {
+    return ptx::cuda_status(e, "cudaEventCreate");
+  }
+  const int slot = r.next;
+  r.words[slot] = 0;
+  cudaError_t e = cudaMemcpyAsync(r.words + slot, workspace, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaEventRecord(ev, s);
+  if (e != cudaSuccess) {
+    r.spare.push_back(ev);
+    return ptx::cuda_status(e, "ptx_status_track");
+  }
+  r.next = (slot + 1) % ptx::kStatusSlots;
+  r.pending.push_back({ev, slot, tag});
+  return PTX_OK;
+}
+
+int ptx_status_poll(int device, int block, int* failed) {
+  if (!failed) return ptx::set_error(PTX_ERR_INVALID_ARGUMENT, "null pointer argument");
+  *failed = -1;
+  std::lock_guard<std::mutex> lock(ptx::g_status_mutex);
+  for (auto& d : ptx::g_status) {
+    if (device >= 0 && d.first != device) continue;
+    if (int st = ptx::retire_status(d.second, block != 0, failed)) return st;
+  }
+  return PTX_OK;
 }
 
 }  // extern "C"

@@ -13,8 +13,8 @@ from __future__ import annotations
 import torch
 
 from . import _abi
-from ._utils import (as_u16, check_complex_scan_inputs, ptr, require_cuda_complex64, scaled_gradients, stream_handle,
-                     upload_small, workspace)
+from ._utils import (as_u16, check_complex_scan_inputs, on_device, ptr, require_cuda_complex64, scaled_gradients,
+                     stream_handle, upload_small, workspace)
 
 __all__ = [
     "ptychoX_fourier",
@@ -71,7 +71,7 @@ class PtychoXFPMFunction(torch.autograd.Function):
         image = torch.empty((batch, lh, lw), dtype=torch.complex64, device=dev)
         amp = torch.empty((batch, lh, lw), dtype=torch.float32, device=dev)
         ws, n = _ws(oh, ow, lh, lw, batch, dev)
-        with torch.cuda.device(dev):
+        with on_device(dev):
             _abi.call("ptx_fpm_forward", ptr(obj), oh, ow, ptr(pupil), lh, lw, ptr(led), batch, ptr(spectrum),
                       ptr(image), ptr(amp), ptr(ws), n, stream_handle(dev))
         ctx.save_for_backward(spectrum, pupil, image, led)
@@ -86,7 +86,7 @@ class PtychoXFPMFunction(torch.autograd.Function):
         grad_object = torch.empty_like(spectrum)
         grad_pupil = torch.empty_like(pupil)
         ws, n = _ws(oh, ow, lh, lw, batch, dev)
-        with torch.cuda.device(dev):
+        with on_device(dev):
             _abi.call("ptx_fpm_backward", ptr(grad_output), ptr(image), ptr(spectrum), oh, ow, ptr(pupil), lh, lw,
                       ptr(led), batch, ptr(grad_object), ptr(grad_pupil), ptr(ws), n, stream_handle(dev))
         return grad_object, grad_pupil, None, None
@@ -101,7 +101,7 @@ def fpm_sweep(obj, pupil, led, measured, scale, ws=None):
     gp = torch.empty_like(pupil)
     if ws is None:
         ws, _ = _ws(oh, ow, lh, lw, batch, dev)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         _abi.call("ptx_fpm_sweep", ptr(obj), oh, ow, ptr(pupil), lh, lw, ptr(led), batch, ptr(measured),
                   float(scale), ptr(loss), ptr(go), ptr(gp), ptr(ws), ws.numel(), stream_handle(dev))
     return loss, go, gp
