@@ -25,7 +25,7 @@
 namespace ptx {
 namespace {
 
-constexpr size_t kHeaderBytes = 256 + kLutBytes;  // error word + padding, count-decode table
+constexpr size_t kHeaderBytes = 256 + kReservedBytes;  // error word + padding
 constexpr size_t kTargetScratch = 4096ull << 20;  // upper bound on workspace frames
 constexpr float kEps = 1.1920928955078125e-07f;  // torch.finfo(float32).eps
 
@@ -361,31 +361,25 @@ __global__ void __launch_bounds__(128, 3) base_rows_forward_reg(
   }
 }
 
-// Column pass (register FFT), same three modes as base_cols_rt.  A CTA owns kColsReg
-// columns of one frame; threads run column-fastest (thread (t, c) owns column c).  In
-// the sweep mode the uint16 counts of the CTA's columns are prefetched into shared
-// memory with cp.async before the forward column DFT, so their latency hides behind it.
+// Column pass (register FFT) of the unfused operator, the forward and backward modes of
+// base_cols_rt (the sweep runs cols_sweep_pair / cols_sweep_pipe).  A CTA owns kColsReg
+// columns of one frame; threads run column-fastest (thread (t, c) owns column c).
 constexpr int kColsReg = 8;
 
 template <int N>
 struct ColCfg {
   static constexpr int LP = col_line_pitch<N>();
-  static constexpr int kMeasOffsetBytes = ((kColsReg * LP * (int)sizeof(float2)) + 15) / 16 * 16;
-  static constexpr int kSmemBytes = kMeasOffsetBytes + N * kColsReg * (int)sizeof(uint16_t);
+  static constexpr int kSmemBytes = kColsReg * LP * (int)sizeof(float2);
 };
 
 template <int MODE, int N>
 __global__ void __launch_bounds__(256, 2) base_cols_reg(
-    float2* __restrict__ scratch, int pw, int frame0, const float2* __restrict__ tw,
-    const uint16_t* __restrict__ measured, const float* __restrict__ lut, float grad_scale, double inv_numel,
-    double* __restrict__ loss, float2* __restrict__ far_field, float* __restrict__ amplitude,
-    const float* __restrict__ grad_output) {
+    float2* __restrict__ scratch, int pw, int frame0, const float2* __restrict__ tw, float2* __restrict__ far_field,
+    float* __restrict__ amplitude, const float* __restrict__ grad_output) {
   pdl_wait();
   using S = RegShape<N>;
   constexpr int LP = ColCfg<N>::LP;
   extern __shared__ float2 sm[];
-  __shared__ double red[32];
-  uint16_t* meas_s = reinterpret_cast<uint16_t*>(reinterpret_cast<char*>(sm) + ColCfg<N>::kMeasOffsetBytes);
   const int tid = threadIdx.x;
   const int c = tid % kColsReg;
   const int t = tid / kColsReg;
@@ -403,28 +397,6 @@ __global__ void __launch_bounds__(256, 2) base_cols_reg(
   if (ic >= pw) ic -= pw;
   float2 v[S::N1];
 
-  if (MODE == kColSweep) {
-    // counts of rows kr (unshifted) -> meas_s[kr][c]
-    int ic0 = c0 + pw / 2;
-    if (ic0 >= pw) ic0 -= pw;
-    const bool fast = (pw % (2 * kColsReg) == 0) && ((reinterpret_cast<uintptr_t>(measured) & 15) == 0);
-    if (fast) {
-      for (int kr = tid; kr < N; kr += blockDim.x) {
-        const int ir = (kr + N / 2) & (N - 1);
-        cp_async16(meas_s + kr * kColsReg, measured + (g * N + ir) * pw + ic0);
-      }
-      cp_async_commit();
-    } else {
-      for (int i = tid; i < N * kColsReg; i += blockDim.x) {
-        const int kr = i / kColsReg, cc = i - kr * kColsReg;
-        const int ir = (kr + N / 2) & (N - 1);
-        int icc = c0 + cc + pw / 2;
-        if (icc >= pw) icc -= pw;
-        meas_s[i] = (c0 + cc < pw) ? measured[(g * N + ir) * pw + icc] : 0;
-      }
-    }
-  }
-
   if (MODE != kColBackward) {
 #pragma unroll
     for (int j = 0; j < S::N1; ++j) {
@@ -433,38 +405,7 @@ __global__ void __launch_bounds__(256, 2) base_cols_reg(
     reg_fft<N, false, true>(v, buf, t, tw);
   }
 
-  if (MODE == kColSweep) {
-    cp_async_wait_all();
-    __syncthreads();
-    float part = 0.f;  // this thread's N1 squared residuals; summed in FP64 across the grid
-#pragma unroll
-    for (int m = 0; m < S::N1; ++m) {
-      const int kr = t + S::T * m;
-      const float2 F = v[m];
-      float2 out = make_float2(0.f, 0.f);
-      if (col_ok) {
-        const float y = __ldg(&lut[meas_s[kr * kColsReg + c]]);
-        float a, inv;
-        abs_and_inv(F, kEps, a, inv);
-        const float rr = a - y;
-        part = fmaf(rr, rr, part);
-        out = cscale(F, grad_scale * rr * inv);
-      }
-      v[m] = out;
-    }
-    double acc = static_cast<double>(part);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((tid & 31) == 0) red[tid >> 5] = acc;
-    __syncthreads();
-    if (tid < 32) {
-      const int nw = (blockDim.x + 31) >> 5;
-      double w = (tid < nw) ? red[tid] : 0.0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-      if (tid == 0) atomicAdd(loss, w * inv_numel);
-    }
-  } else if (MODE == kColForward) {
+  if (MODE == kColForward) {
     if (col_ok) {
 #pragma unroll
       for (int m = 0; m < S::N1; ++m) {
@@ -669,7 +610,7 @@ template <int N, bool STAGE>
 __global__ void __launch_bounds__(256, 1) base_sweep_frame(
     const float2* __restrict__ sample, int H, int W, const float2* __restrict__ probe,
     const int64_t* __restrict__ pos, int nframes, const uint16_t* __restrict__ measured,
-    const float* __restrict__ lut, float grad_scale, double inv_numel, double* __restrict__ loss,
+    float scale, float grad_scale, double inv_numel, double* __restrict__ loss,
     float2* __restrict__ grad_sample, float2* __restrict__ grad_probe, const float2* __restrict__ tw,
     unsigned* __restrict__ err) {
   pdl_wait();
@@ -728,7 +669,7 @@ __global__ void __launch_bounds__(256, 1) base_sweep_frame(
       for (int m = 0; m < S::N1; ++m) {
         const int kr = t + S::T * m;
         const int ir = (kr + N / 2) & (N - 1);
-        const float y = __ldg(&lut[STAGE ? cnt_s[ir * Cfg::CP + ic] : cnt[ir * N + ic]]);
+        const float y = decode_amplitude(STAGE ? cnt_s[ir * Cfg::CP + ic] : cnt[ir * N + ic], scale);
         float a, inv;
         abs_and_inv(v[m], kEps, a, inv);
         const float rr = a - y;
@@ -793,7 +734,6 @@ struct BaseGeom {
   size_t frame_bytes;
   int chunk;
   unsigned* err;
-  float* lut;
   float2* scratch;
 };
 
@@ -829,7 +769,6 @@ int check_common(const void* sample, int H, int W, const void* probe, int ph, in
   // (the column passes put the frame in gridDim.y)
   g->chunk = static_cast<int>(std::min<size_t>({fit, (size_t)std::max(batch, 1), (size_t)65535}));
   g->err = reinterpret_cast<unsigned*>(ws);
-  g->lut = reinterpret_cast<float*>(static_cast<char*>(ws) + 256);
   g->scratch = reinterpret_cast<float2*>(static_cast<char*>(ws) + kHeaderBytes);
   int st = PTX_OK;
   dispatch_len(pw, [&](auto NT) {
@@ -851,6 +790,9 @@ int check_common(const void* sample, int H, int W, const void* probe, int ph, in
       const int sm = RegLaunch<N>::col_smem();
       if (!st) st = ensure_smem((const void*)cols_sweep_pair<N, false, true>, ColPairCfg<N>::kSmemBytes);
       if (!st) st = ensure_smem((const void*)cols_sweep_pair<N, false, true, true, true>, ColPairCfg<N>::kSmemBytes);
+      if constexpr (col_pipe_length<N>()) {
+        if (!st) st = prepare_col_pipe<N, false, true, true>();
+      }
       if (!st) st = ensure_smem((const void*)base_cols_reg<kColForward, N>, sm);
       if (!st) st = ensure_smem((const void*)base_cols_reg<kColBackward, N>, sm);
     } else if (const MixOps* mo = mix_ops(ph)) {
@@ -939,20 +881,27 @@ void launch_cols(const BaseGeom& g, int frame0, int nframes, const uint16_t* mea
       if constexpr (MODE == kColSweep) {
         // column DFT, amplitude-loss epilogue and inverse column DFT; counts fftshifted
         dim3 grid(num_tiles(g.pw), nframes);
+        if constexpr (col_pipe_length<N>()) {
+          if (col_pipe_takes(g.pw, measured)) {
+            launch_col_pipe<N, false, true, true>(g.scratch, g.pw, nframes, frame0, g.col.tw, measured, scale, 1.0f,
+                                                  grad_scale, inv_numel, loss, s);
+            return;
+          }
+        }
         if (g.pw % kTile == 0) {
           launch_pdl(cols_sweep_pair<N, false, true, true, true>, grid, ColPairCfg<N>::kThreads, ColPairCfg<N>::kSmemBytes, s,
-              g.scratch, g.pw, frame0, g.col.tw, measured, g.lut, 1.0f, grad_scale, inv_numel, loss);
+              g.scratch, g.pw, frame0, g.col.tw, measured, scale, 1.0f, grad_scale, inv_numel, loss);
         } else {
           launch_pdl(cols_sweep_pair<N, false, true>, grid, ColPairCfg<N>::kThreads, ColPairCfg<N>::kSmemBytes, s,
-              g.scratch, g.pw, frame0, g.col.tw, measured, g.lut, 1.0f, grad_scale, inv_numel, loss);
+              g.scratch, g.pw, frame0, g.col.tw, measured, scale, 1.0f, grad_scale, inv_numel, loss);
         }
-        return;
+      } else {
+        dim3 grid(num_tiles(g.pw) * (kTile / kColsReg), nframes);
+        launch_pdl(base_cols_reg<MODE, N>, grid, L::col_threads(), L::col_smem(), s, g.scratch, g.pw, frame0, g.col.tw,
+                   far_field, amplitude, grad_output);
       }
-      dim3 grid(num_tiles(g.pw) * (kTile / kColsReg), nframes);
-      launch_pdl(base_cols_reg<MODE, N>, grid, L::col_threads(), L::col_smem(), s, g.scratch, g.pw, frame0,
-                 g.col.tw, measured, g.lut, grad_scale, inv_numel, loss, far_field, amplitude, grad_output);
     } else if (const MixOps* mo = mix_ops(g.ph)) {
-      MixColsArgs a{g.scratch, g.ph, g.pw, frame0, nframes, g.col.mix_twt, g.col.mix_twi, measured, g.lut,
+      MixColsArgs a{g.scratch, g.ph, g.pw, frame0, nframes, g.col.mix_twt, g.col.mix_twi, measured, scale,
                     grad_scale, inv_numel, loss, far_field, amplitude, grad_output};
       mo->cols(MODE == kColSweep ? kMixColSweep : MODE == kColForward ? kMixColForward : kMixColBackward, a, s);
     } else {
@@ -1051,7 +1000,7 @@ int ptx_base_backward(const float* grad_output, const float* far_field, const fl
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   float2* GS = reinterpret_cast<float2*>(grad_sample);
   float2* GP = reinterpret_cast<float2*>(grad_probe);
-  launch_prologue(s, GS, (size_t)sample_h * sample_w, GP, (size_t)probe_h * probe_w, nullptr, g.err, nullptr, 0.f);
+  launch_prologue(s, GS, (size_t)sample_h * sample_w, GP, (size_t)probe_h * probe_w, nullptr, g.err);
   if (batch > 0) {
     prof_begin(kMiscKernel, s);
     launch_pdl(window_check_kernel, (batch + 255) / 256, 256, 0, s, positions_xy, batch, probe_h, probe_w, sample_h,
@@ -1087,7 +1036,7 @@ int ptx_base_sweep(const float* sample, int sample_h, int sample_w, const float*
   float2* GP = reinterpret_cast<float2*>(grad_probe);
   const double numel = (double)batch * probe_h * probe_w;
   const float grad_scale = static_cast<float>(2.0 / std::max(numel, 1.0));
-  launch_prologue(s, GS, (size_t)sample_h * sample_w, GP, (size_t)probe_h * probe_w, loss, g.err, g.lut, scale);
+  launch_prologue(s, GS, (size_t)sample_h * sample_w, GP, (size_t)probe_h * probe_w, loss, g.err);
   const float2* S = reinterpret_cast<const float2*>(sample);
   const float2* P = reinterpret_cast<const float2*>(probe);
   for (int b0 = 0; b0 < batch; b0 += g.chunk) {
@@ -1135,7 +1084,7 @@ int ptx_base_sweep_small(const float* sample, int sample_h, int sample_w, const 
   float2* GP = reinterpret_cast<float2*>(grad_probe);
   const double numel = (double)batch * probe_h * probe_w;
   const float grad_scale = static_cast<float>(2.0 / std::max(numel, 1.0));
-  launch_prologue(s, GS, (size_t)sample_h * sample_w, GP, (size_t)probe_h * probe_w, loss, g.err, g.lut, scale);
+  launch_prologue(s, GS, (size_t)sample_h * sample_w, GP, (size_t)probe_h * probe_w, loss, g.err);
   if (batch == 0) return cuda_status(cudaGetLastError(), "ptx_base_sweep_small launch");
   const float2* S = reinterpret_cast<const float2*>(sample);
   const float2* P = reinterpret_cast<const float2*>(probe);
@@ -1148,7 +1097,7 @@ int ptx_base_sweep_small(const float* sample, int sample_h, int sample_w, const 
         if (st) return;
         const int grid = persistent_grid((const void*)kern, threads, smem, batch);
         prof_begin(kBaseRowsForward, s);
-        launch_pdl(kern, grid, threads, smem, s, S, sample_h, sample_w, P, positions_xy, batch, measured, g.lut,
+        launch_pdl(kern, grid, threads, smem, s, S, sample_h, sample_w, P, positions_xy, batch, measured, scale,
                    grad_scale, 1.0 / std::max(numel, 1.0), loss, GS, GP, g.row.tw, g.err);
         prof_end(kBaseRowsForward, s);
       };

@@ -862,7 +862,7 @@ int coded_backward_impl(const float* grad_output, const float* x_forward, const 
   const float2* M = reinterpret_cast<const float2*>(coded_surface);
   if (zero) {
     const size_t field = g.field_bytes / sizeof(float2);
-    launch_prologue(s, g.gospec, field, reinterpret_cast<float2*>(grad_coded), field, nullptr, nullptr, nullptr, 0.f);
+    launch_prologue(s, g.gospec, field, reinterpret_cast<float2*>(grad_coded), field, nullptr, nullptr);
   }
   for (int b0 = 0; b0 < batch; b0 += g.chunk) {
     const int nf = std::min(g.chunk, batch - b0);
@@ -942,8 +942,8 @@ static int coded_sweep_mse(const float* object, const float* coded_surface, cons
   const float2* T2 = reinterpret_cast<const float2*>(transfer_2);
   const float2* M = reinterpret_cast<const float2*>(coded_surface);
   const size_t field = g.field_bytes / sizeof(float2);
-  launch_prologue(s, g.gospec, field, reinterpret_cast<float2*>(grad_coded), field, loss, nullptr, nullptr, 0.f,
-                  grad_shifts, grad_shifts ? 2 * (size_t)batch : 0);
+  launch_prologue(s, g.gospec, field, reinterpret_cast<float2*>(grad_coded), field, loss, nullptr, grad_shifts,
+                  grad_shifts ? 2 * (size_t)batch : 0);
   const int lw = n / downsample;
   const double numel = (double)batch * lw * lw;
   const float grad_scale = static_cast<float>(2.0 / std::max(numel, 1.0));
@@ -1023,7 +1023,7 @@ static int coded_sweep_fd(const float* object, const float* coded_surface, const
     return st;
   }
   launch_prologue(s, g.gospec, g.field_bytes / sizeof(float2), reinterpret_cast<float2*>(grad_coded),
-                  g.field_bytes / sizeof(float2), loss, nullptr, nullptr, 0.f, grad_shifts,
+                  g.field_bytes / sizeof(float2), loss, nullptr, grad_shifts,
                   grad_shifts ? 2 * (size_t)batch : 0);
   if (int st = ptx_coded_forward(object, coded_surface, transfer_1, transfer_2, n, shifts_xy, batch, downsample, xf,
                                  sensor, amp, p, inner, stream)) {

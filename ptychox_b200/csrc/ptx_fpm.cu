@@ -28,7 +28,7 @@
 namespace ptx {
 namespace {
 
-constexpr size_t kHdr = 256 + kLutBytes;  // padding, count-decode table
+constexpr size_t kHdr = 256 + kReservedBytes;
 enum FpmMode { kFpmSweep = 0, kFpmForward = 1, kFpmBackward = 2 };
 
 __device__ __forceinline__ int wrap2(long long v, int n) { return static_cast<int>(v & (long long)(n - 1)); }
@@ -134,18 +134,15 @@ __global__ void __launch_bounds__(128, 3) fpm_rows_forward(
   }
 }
 
+// Column pass of the unfused operator (the sweep runs cols_sweep_pair / cols_sweep_pipe).
 template <int MODE, int NH>
 __global__ void __launch_bounds__(256, 2) fpm_cols(
-    float2* __restrict__ scratch, int lw, int frame0, const float2* __restrict__ tw,
-    const uint16_t* __restrict__ measured, const float* __restrict__ lut, float norm, float grad_scale,
-    double inv_numel,
-    double* __restrict__ loss, float2* __restrict__ image_out, float* __restrict__ amplitude,
-    const float* __restrict__ grad_output) {
+    float2* __restrict__ scratch, int lw, int frame0, const float2* __restrict__ tw, float norm,
+    float2* __restrict__ image_out, float* __restrict__ amplitude, const float* __restrict__ grad_output) {
   pdl_wait();
   using S = RegShape<NH>;
   using CP = ColPass<NH>;
   extern __shared__ float2 sm[];
-  uint16_t* meas_s = reinterpret_cast<uint16_t*>(reinterpret_cast<char*>(sm) + CP::kMeasOffsetBytes);
   const int tid = threadIdx.x;
   const int c = tid % kColsPerCta;
   const int t = tid / kColsPerCta;
@@ -161,44 +158,12 @@ __global__ void __launch_bounds__(256, 2) fpm_cols(
   float2* buf = sm + c * CP::LP;
   float2 v[S::N1];
 
-  if (MODE == kFpmSweep) {
-    const bool fast = (lw % (2 * kColsPerCta) == 0) && ((reinterpret_cast<uintptr_t>(measured) & 15) == 0);
-    if (fast) {
-      for (int kr = tid; kr < NH; kr += blockDim.x) cp_async16(meas_s + kr * kColsPerCta, measured + (g * NH + kr) * lw + c0);
-      cp_async_commit();
-    } else {
-      for (int q = tid; q < NH * kColsPerCta; q += blockDim.x) {
-        const int kr = q / kColsPerCta, cc = q - kr * kColsPerCta;
-        meas_s[q] = (c0 + cc < lw) ? measured[(g * NH + kr) * lw + c0 + cc] : 0;
-      }
-    }
-  }
   if (MODE != kFpmBackward) {
 #pragma unroll
     for (int j = 0; j < S::N1; ++j) v[j] = col_ok ? tile[(t + S::T * j) * kTile + c] : make_float2(0.f, 0.f);
     reg_fft<NH, true, true>(v, buf, t, tw);
   }
-  if (MODE == kFpmSweep) {
-    cp_async_wait_all();
-    __syncthreads();
-    float part = 0.f;  // this thread's squared residuals; summed in FP64 across the grid
-#pragma unroll
-    for (int m = 0; m < S::N1; ++m) {
-      const int kr = t + S::T * m;
-      const float2 im = cscale(v[m], norm);
-      float2 out = make_float2(0.f, 0.f);
-      if (col_ok) {
-        const float y = __ldg(&lut[meas_s[kr * kColsPerCta + c]]);
-        float a, inv;
-        abs_and_inv(im, kEpsF32, a, inv);
-        const float rr = a - y;
-        part = fmaf(rr, rr, part);
-        out = cscale(im, grad_scale * rr * inv);
-      }
-      v[m] = out;
-    }
-    block_add_double(static_cast<double>(part), inv_numel, loss);
-  } else if (MODE == kFpmForward) {
+  if (MODE == kFpmForward) {
     if (col_ok) {
 #pragma unroll
       for (int m = 0; m < S::N1; ++m) {
@@ -345,7 +310,6 @@ struct FpmGeom {
   float2* gspec;  // gradient w.r.t. the spectrum
   float2* tmp;    // tiled temporary of the 2-D passes
   float2* frames;
-  float* lut;     // count-decode table (sweep)
 };
 
 size_t fpm_fixed_bytes(int oh, int ow) {
@@ -385,7 +349,6 @@ int fpm_check(const void* object, int oh, int ow, const void* pupil, int lh, int
   // passes put the frame in gridDim.y)
   g->chunk = static_cast<int>(
       std::min<size_t>({(ws_bytes - fixed) / g->frame_bytes, (size_t)std::max(batch, 1), (size_t)65535}));
-  g->lut = reinterpret_cast<float*>(static_cast<char*>(ws) + 256);
   char* p = static_cast<char*>(ws) + kHdr;
   g->spec = reinterpret_cast<float2*>(p);
   g->gspec = reinterpret_cast<float2*>(p + g->spec_bytes);
@@ -424,6 +387,9 @@ int fpm_check(const void* object, int oh, int ow, const void* pupil, int lh, int
   });
   dispatch_pow2(lh, [&](auto NT) {
     constexpr int N = decltype(NT)::value;
+    if constexpr (col_pipe_length<N>()) {
+      if (!st) st = prepare_col_pipe<N, true, false, false>();
+    }
     if (!st) st = ensure_smem((const void*)cols_sweep_pair<N, true, false>, ColPairCfg<N>::kSmemBytes);
     if (!st) st = ensure_smem((const void*)cols_sweep_pair<N, true, false, false, true>, ColPairCfg<N>::kSmemBytes);
     if (!st) st = ensure_smem((const void*)fpm_cols<kFpmForward, N>, ColPass<N>::kSmemBytes);
@@ -488,13 +454,13 @@ void launch_rows_forward(const FpmGeom& g, const float2* spec, const float2* pup
 }
 
 template <int MODE>
-void launch_cols(const FpmGeom& g, int frame0, int nf, const uint16_t* measured, float grad_scale,
+void launch_cols(const FpmGeom& g, int frame0, int nf, const uint16_t* measured, float scale, float grad_scale,
                  double inv_numel, double* loss, float2* image, float* amplitude, const float* grad_output,
                  cudaStream_t s) {
   const float norm = 1.0f / static_cast<float>((double)g.lh * g.lw);
   prof_begin(kFpmCols, s);
   if (g.generic) {
-    MixFpmColsArgs a{g.frames, g.lw, frame0, nf, g.p_lh.mix_twt, g.p_lh.mix_twi, measured, g.lut, norm, grad_scale,
+    MixFpmColsArgs a{g.frames, g.lw, frame0, nf, g.p_lh.mix_twt, g.p_lh.mix_twi, measured, scale, norm, grad_scale,
                      inv_numel, loss, image, amplitude, grad_output};
     g.m_lh->cols(MODE == kFpmSweep ? kMixColSweep : MODE == kFpmForward ? kMixColForward : kMixColBackward, a, s);
     prof_end(kFpmCols, s);
@@ -505,18 +471,25 @@ void launch_cols(const FpmGeom& g, int frame0, int nf, const uint16_t* measured,
     if constexpr (MODE == kFpmSweep) {
       // inverse column DFT, 1/(h w), amplitude-loss epilogue, forward column DFT
       dim3 grid(num_tiles(g.lw), nf);
+      if constexpr (col_pipe_length<N>()) {
+        if (col_pipe_takes(g.lw, measured)) {
+          launch_col_pipe<N, true, false, false>(g.frames, g.lw, nf, frame0, g.p_lh.tw, measured, scale, norm,
+                                                 grad_scale, inv_numel, loss, s);
+          return;
+        }
+      }
       if (g.lw % kTile == 0) {
         launch_pdl(cols_sweep_pair<N, true, false, false, true>, grid, ColPairCfg<N>::kThreads, ColPairCfg<N>::kSmemBytes, s,
-            g.frames, g.lw, frame0, g.p_lh.tw, measured, g.lut, norm, grad_scale, inv_numel, loss);
+            g.frames, g.lw, frame0, g.p_lh.tw, measured, scale, norm, grad_scale, inv_numel, loss);
       } else {
         launch_pdl(cols_sweep_pair<N, true, false>, grid, ColPairCfg<N>::kThreads, ColPairCfg<N>::kSmemBytes, s,
-            g.frames, g.lw, frame0, g.p_lh.tw, measured, g.lut, norm, grad_scale, inv_numel, loss);
+            g.frames, g.lw, frame0, g.p_lh.tw, measured, scale, norm, grad_scale, inv_numel, loss);
       }
-      return;
+    } else {
+      dim3 grid(num_tiles(g.lw) * (kTile / kColsPerCta), nf);
+      launch_pdl(fpm_cols<MODE, N>, grid, ColPass<N>::kThreads, ColPass<N>::kSmemBytes, s,
+                 g.frames, g.lw, frame0, g.p_lh.tw, norm, image, amplitude, grad_output);
     }
-    dim3 grid(num_tiles(g.lw) * (kTile / kColsPerCta), nf);
-    launch_pdl(fpm_cols<MODE, N>, grid, ColPass<N>::kThreads, ColPass<N>::kSmemBytes, s, g.frames, g.lw, frame0,
-               g.p_lh.tw, measured, g.lut, norm, grad_scale, inv_numel, loss, image, amplitude, grad_output);
   });
   prof_end(kFpmCols, s);
 }
@@ -575,7 +548,7 @@ int ptx_fpm_forward(const float* object, int object_h, int object_w, const float
   for (int b0 = 0; b0 < batch; b0 += g.chunk) {
     const int nf = std::min(g.chunk, batch - b0);
     launch_rows_forward(g, spec, P, led_indices_xy + 2 * (size_t)b0, nf, s);
-    launch_cols<kFpmForward>(g, b0, nf, nullptr, 0.f, 0.0, nullptr, reinterpret_cast<float2*>(image),
+    launch_cols<kFpmForward>(g, b0, nf, nullptr, 0.f, 0.f, 0.0, nullptr, reinterpret_cast<float2*>(image),
                              amplitude, nullptr, s);
   }
   return cuda_status(cudaGetLastError(), "ptx_fpm_forward launch");
@@ -594,13 +567,13 @@ int ptx_fpm_backward(const float* grad_output, const float* image, const float* 
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   launch_prologue(s, g.gspec, g.spec_bytes / sizeof(float2), reinterpret_cast<float2*>(grad_pupil),
-                  (size_t)low_h * low_w, nullptr, nullptr, nullptr, 0.f);
+                  (size_t)low_h * low_w, nullptr, nullptr);
   const float2* spec = reinterpret_cast<const float2*>(spectrum);
   const float2* P = reinterpret_cast<const float2*>(pupil);
   float2* GP = reinterpret_cast<float2*>(grad_pupil);
   for (int b0 = 0; b0 < batch; b0 += g.chunk) {
     const int nf = std::min(g.chunk, batch - b0);
-    launch_cols<kFpmBackward>(g, b0, nf, nullptr, 0.f, 0.0, nullptr,
+    launch_cols<kFpmBackward>(g, b0, nf, nullptr, 0.f, 0.f, 0.0, nullptr,
                               const_cast<float2*>(reinterpret_cast<const float2*>(image)), nullptr, grad_output, s);
     launch_rows_adjoint(g, spec, P, led_indices_xy + 2 * (size_t)b0, nf, g.gspec, GP, s);
   }
@@ -625,7 +598,7 @@ int ptx_fpm_sweep(const float* object, int object_h, int object_w, const float* 
   const double numel = (double)batch * low_h * low_w;
   const float grad_scale = static_cast<float>(2.0 / std::max(numel, 1.0));
   launch_prologue(s, g.gspec, g.spec_bytes / sizeof(float2), reinterpret_cast<float2*>(grad_pupil),
-                  (size_t)low_h * low_w, loss, nullptr, g.lut, scale);
+                  (size_t)low_h * low_w, loss, nullptr);
   launch_fft2<false>(g, reinterpret_cast<const float2*>(object), object_h, object_w, g.spec, 1.0f, g.tmp, g.p_ow, g.p_oh,
                      s);
   const float2* P = reinterpret_cast<const float2*>(pupil);
@@ -634,7 +607,7 @@ int ptx_fpm_sweep(const float* object, int object_h, int object_w, const float* 
     const int nf = std::min(g.chunk, batch - b0);
     const int64_t* led = led_indices_xy + 2 * (size_t)b0;
     launch_rows_forward(g, g.spec, P, led, nf, s);
-    launch_cols<kFpmSweep>(g, b0, nf, measured, grad_scale, 1.0 / std::max(numel, 1.0), loss, nullptr, nullptr,
+    launch_cols<kFpmSweep>(g, b0, nf, measured, scale, grad_scale, 1.0 / std::max(numel, 1.0), loss, nullptr, nullptr,
                            nullptr, s);
     launch_rows_adjoint(g, g.spec, P, led, nf, g.gspec, GP, s);
   }

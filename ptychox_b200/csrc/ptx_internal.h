@@ -182,7 +182,7 @@ struct MixColsArgs {
   const float2* twt;     // column-length twiddles
   const float2* twi;
   const uint16_t* measured;  // sweep: fftshifted counts
-  const float* lut;          // sweep: count -> observed amplitude
+  float scale;               // sweep: observed amplitude = sqrt(count scale)
   float grad_scale;
   double inv_numel;
   double* loss;
@@ -222,7 +222,7 @@ struct MixFpmColsArgs {
   const float2* twt;  // column-length (lh) twiddles
   const float2* twi;
   const uint16_t* measured;  // sweep: counts (not shifted)
-  const float* lut;
+  float scale;
   float norm;                // 1 / (lh lw)
   float grad_scale;
   double inv_numel;

@@ -69,30 +69,19 @@ struct ColPass {
   static constexpr int T = RegShape<N>::T;
   static constexpr int LP = col_line_pitch<N>();
   static constexpr int kThreads = kColsPerCta * T;
-  static constexpr int kMeasOffsetBytes = ((kColsPerCta * LP * (int)sizeof(float2)) + 15) / 16 * 16;
-  static constexpr int kSmemBytes = kMeasOffsetBytes + N * kColsPerCta * (int)sizeof(uint16_t);
+  static constexpr int kSmemBytes = kColsPerCta * LP * (int)sizeof(float2);
 };
 
-// ---- observed-amplitude decode table -------------------------------------------------
-// lut[c] = sqrtf(float(c) * scale) for every uint16 count c: built once per sweep with the
-// same two IEEE operations the per-element decode would use, then read by the epilogues
-// (a cached load instead of a square root per element).
-constexpr int kLutEntries = 65536;
-constexpr size_t kLutBytes = kLutEntries * sizeof(float);
+// Bytes behind a workspace's error word that the sweeps leave unused: workspaces are sized with
+// them (a count-decode table stood there), and callers hold such sizes.
+constexpr size_t kReservedBytes = 65536 * sizeof(float);
 
-static __global__ void decode_lut_kernel(float* __restrict__ lut, float scale) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < kLutEntries) lut[c] = sqrtf(static_cast<float>(c) * scale);
-}
-
-// One launch for everything a sweep (or an adjoint: no loss, no table) resets before its
-// passes: zero two gradient arrays (n_a and n_b complex elements), the FP64 loss, the error word
-// and n_c doubles, and (lut non-null) build the count-decode table.  Grid-stride; any grid size
-// works.
+// One launch for everything a sweep (or an adjoint: no loss) resets before its passes: two
+// gradient arrays (n_a and n_b complex elements), n_c doubles, the FP64 loss and the error word.
+// Grid-stride; any grid size works.
 static __global__ void sweep_prologue_kernel(float2* __restrict__ zero_a, size_t n_a, float2* __restrict__ zero_b,
                                              size_t n_b, double* __restrict__ loss, unsigned* __restrict__ err,
-                                             float* __restrict__ lut, float scale, double* __restrict__ zero_c,
-                                             size_t n_c) {
+                                             double* __restrict__ zero_c, size_t n_c) {
   pdl_wait();
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -100,9 +89,6 @@ static __global__ void sweep_prologue_kernel(float2* __restrict__ zero_a, size_t
   for (size_t i = i0; i < n_a; i += stride) zero_a[i] = z;
   for (size_t i = i0; i < n_b; i += stride) zero_b[i] = z;
   for (size_t i = i0; i < n_c; i += stride) zero_c[i] = 0.0;
-  if (lut) {
-    for (size_t c = i0; c < (size_t)kLutEntries; c += stride) lut[c] = sqrtf(static_cast<float>(c) * scale);
-  }
   if (i0 == 0) {
     if (loss) *loss = 0.0;
     if (err) *err = 0u;
@@ -116,10 +102,10 @@ inline unsigned prologue_blocks(size_t elements, int sms) {
 }
 
 inline void launch_prologue(cudaStream_t s, float2* zero_a, size_t n_a, float2* zero_b, size_t n_b, double* loss,
-                            unsigned* err, float* lut, float scale, double* zero_c = nullptr, size_t n_c = 0) {
+                            unsigned* err, double* zero_c = nullptr, size_t n_c = 0) {
   prof_begin(kMiscKernel, s);
   launch_pdl(sweep_prologue_kernel, prologue_blocks(std::max(n_a, n_b), sm_count()), 256, 0, s, zero_a, n_a, zero_b, n_b,
-             loss, err, lut, scale, zero_c, n_c);
+             loss, err, zero_c, n_c);
   prof_end(kMiscKernel, s);
 }
 
@@ -128,6 +114,28 @@ inline void launch_prologue(cudaStream_t s, float2* zero_a, size_t n_a, float2* 
 __device__ __forceinline__ float rsqrt_nr(float s) {
   const float y = rsqrtf(s);
   return y * fmaf(-0.5f * s, y * y, 1.5f);
+}
+
+// sqrt(count scale), the amplitude observed at a detector pixel: a reciprocal square root refined
+// by one step of g + (x - g^2) h, h ~ 1 / (2 sqrt x) (P. Markstein, IBM J. Res. Dev. 34, 111
+// (1990)), which rounds to nearest; 0 for no counts.  A table of all 65536 counts read by the
+// epilogues instead cost their warps the loads' latency (Fourier columns of 225 x 256^2: 65.9
+// against 59.3 us) and each sweep its making.
+__device__ __forceinline__ float rsqrt_floor(float x) {  // 1 / sqrt(max(x, the least normal number))
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(fmaxf(x, 1.1754944e-38f)));
+  return y;
+}
+__device__ __forceinline__ float decode_amplitude(uint32_t count, float scale) {
+  const float x = static_cast<float>(count) * scale;
+  const float y = rsqrt_floor(x), g = x * y;
+  return fmaf(fmaf(-g, g, x), 0.5f * y, g);
+}
+// of the two counts of a 32-bit word
+__device__ __forceinline__ float2 decode_amplitudes(uint32_t counts, float2 scale) {
+  const float2 x = mul2(make_float2(static_cast<float>(counts & 0xffffu), static_cast<float>(counts >> 16)), scale);
+  const float2 y = make_float2(rsqrt_floor(x.x), rsqrt_floor(x.y)), g = mul2(x, y);
+  return fma2(fma2(neg2(g), g, x), mul2(f2(0.5f), y), g);
 }
 
 // |z| and 1 / max(|z|, eps) from one reciprocal square root.
@@ -231,7 +239,7 @@ __global__ void __launch_bounds__(256, 2) fft2_cols_kernel(const float2* __restr
 // one packed instruction for two columns.  A column pair is one 16-byte load / store per
 // row (a warp covers four whole 128-byte tile rows).  The sequence per column: DFT in the
 // FIRST_INV direction, scale by `norm`, amplitude-loss epilogue against the counts
-// (decoded through `lut`; SHIFTED: the counts are stored fftshifted in both axes), the
+// (decoded with `scale`; SHIFTED: the counts are stored fftshifted in both axes), the
 // DFT in the other direction, store in place.  The tile's counts arrive by cp.async while
 // the first transform runs; the twiddle table sits in shared memory as broadcast pairs.
 template <int N>
@@ -257,8 +265,8 @@ constexpr int col_pair_min_blocks() {
 template <int N, bool FIRST_INV, bool SHIFTED, bool UNIT_NORM = false, bool FULL = false>
 __global__ void __launch_bounds__(ColPairCfg<N>::kThreads, col_pair_min_blocks<N>()) cols_sweep_pair(
     float2* __restrict__ scratch, int width, int frame0, const float2* __restrict__ tw,
-    const uint16_t* __restrict__ measured, const float* __restrict__ lut, float norm, float grad_scale,
-    double inv_numel, double* __restrict__ loss) {
+    const uint16_t* __restrict__ measured, float scale, float norm, float grad_scale, double inv_numel,
+    double* __restrict__ loss) {
   pdl_wait();
   using S = RegShape<N>;
   using Cfg = ColPairCfg<N>;
@@ -317,8 +325,7 @@ __global__ void __launch_bounds__(ColPairCfg<N>::kThreads, col_pair_min_blocks<N
   cp_async_wait_all();
   __syncthreads();
   float2 part = make_float2(0.f, 0.f);  // squared residuals of the two columns
-  const float2 gs = f2(grad_scale);
-  const float2 nrm = f2(norm);
+  const float2 gs = f2(grad_scale), nrm = f2(norm), sc_y = f2(scale);
 #pragma unroll
   for (int m = 0; m < S::N1; ++m) {
     const int kr = t + S::T * m;
@@ -326,14 +333,12 @@ __global__ void __launch_bounds__(ColPairCfg<N>::kThreads, col_pair_min_blocks<N
     const float2 s2 = fma2(F.re, F.re, mul2(F.im, F.im));
     // rsqrt_nr on both lanes, its Newton-Raphson step in packed form (the same IEEE operations)
     const float2 sc2 = make_float2(fmaxf(s2.x, 1e-37f), fmaxf(s2.y, 1e-37f));
-    const float2 y0 = make_float2(rsqrtf(sc2.x), rsqrtf(sc2.y));
+    const float2 y0 = make_float2(rsqrt_floor(sc2.x), rsqrt_floor(sc2.y));
     const float2 r = mul2(y0, fma2(mul2(f2(-0.5f), sc2), mul2(y0, y0), f2(1.5f)));
     const float2 a = mul2(s2, r);
     const float2 inv =
         make_float2(a.x >= kEpsF32 ? r.x : 1.0f / kEpsF32, a.y >= kEpsF32 ? r.y : 1.0f / kEpsF32);
-    const uint32_t cnt = *reinterpret_cast<const uint32_t*>(meas_s + kr * kTile + 2 * p);
-    const float2 y = make_float2(okA ? __ldg(&lut[cnt & 0xffffu]) : 0.f, okB ? __ldg(&lut[cnt >> 16]) : 0.f);
-    float2 rr = sub2(a, y);
+    float2 rr = sub2(a, decode_amplitudes(*reinterpret_cast<const uint32_t*>(meas_s + kr * kTile + 2 * p), sc_y));
     rr = make_float2(okA ? rr.x : 0.f, okB ? rr.y : 0.f);
     part = fma2(rr, rr, part);
     const float2 sc = mul2(mul2(gs, rr), inv);
@@ -348,6 +353,232 @@ __global__ void __launch_bounds__(ColPairCfg<N>::kThreads, col_pair_min_blocks<N
     }
   }
   block_add_double(static_cast<double>(part.x) + static_cast<double>(part.y), inv_numel, loss);
+}
+
+// ---- the same pass as a pipeline over tiles ------------------------------------------------
+// One wave of CTAs, each walking tiles with two groups of threads (one tile each, alternating)
+// over three tile buffers.  A whole tile is one contiguous block, so it arrives by one bulk copy
+// (cp.async.bulk, no registers, no load instructions) while both groups transform earlier tiles;
+// the exchanges of a tile's two transforms happen in the same buffer: thread (c, t) of column c
+// writes exactly where it has read (rows t + T j), and a half-warp always covers one 128-byte row.  The buffer takes the next tile as soon as the second exchange has been
+// read, before that transform's last step and the stores.
+__device__ __forceinline__ uint32_t smem_addr(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(count) : "memory");
+}
+// Bulk copy of `bytes` (a multiple of 16, both ends 16-byte aligned) that completes on `bar`.
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar, uint64_t pol) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;\n" ::"r"(
+          smem_addr(dst)),
+      "l"(src), "r"(bytes), "r"(smem_addr(bar)), "l"(pol)
+      : "memory");
+}
+// Wait for the phase of `parity`; false if it has not completed after a bounded number of tries
+// (tens of milliseconds at least, where a copy takes microseconds).
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+  for (int i = 0; i < (1 << 20); ++i) {
+    uint32_t done;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(smem_addr(bar)), "r"(parity)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void group_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+}
+
+template <int N>
+struct ColPipeCfg {
+  static constexpr int kPairs = kTile / 2;
+  static constexpr int kGroup = kPairs * RegShape<N>::T;  // threads per tile
+  static constexpr int kBufs = 3;
+  static constexpr int kTileBytes = N * kTile * (int)sizeof(float2);
+  static constexpr int kMeasBytes = N * kTile * (int)sizeof(uint16_t);
+  static constexpr int kTwBytes = N / 2 * (int)sizeof(float2);
+  static constexpr int kSmemBytes = kBufs * kTileBytes + 2 * kMeasBytes + kTwBytes + 64;
+  static constexpr int kBlocks = N <= 256 ? 2 : 1;  // CTAs per SM
+};
+
+// First step of the pair transform for thread t: DFT-N1, twiddles from the half table
+// tw[m] = exp(-2 pi i m / N), m < N / 2 (the other half is its negative), to rows t + T k1.
+template <int N, bool INV>
+__device__ __forceinline__ void pipe_step1(CPair (&v)[RegShape<N>::N1], float4* rows, int t, const float2* tw) {
+  using S = RegShape<N>;
+  constexpr int P = kTile / 2;
+  PRegDft<S::N1, INV>::run(v);
+  rows[t * P] = pack4(v[0]);
+#pragma unroll
+  for (int k1 = 1; k1 < S::N1; ++k1) {
+    const int m = t * k1;
+    float2 w = tw[m & (N / 2 - 1)];
+    const uint32_t flip = static_cast<uint32_t>(m & (N / 2)) << (31 - (S::LOG - 1));
+    w.x = __uint_as_float(__float_as_uint(w.x) ^ flip);
+    w.y = __uint_as_float(__float_as_uint(w.y) ^ (INV ? flip ^ 0x80000000u : flip));
+    const float2 wx = f2(w.x), wy = f2(w.y), wn = f2(-w.y);
+    const CPair z = v[k1];
+    rows[(t + S::T * k1) * P] = pack4({fma2(z.im, wn, mul2(z.re, wx)), fma2(z.im, wx, mul2(z.re, wy))});
+  }
+}
+// Second step: the C rows of T values k1 = q T + t, then their DFT-T.
+template <int N>
+__device__ __forceinline__ void pipe_load2(CPair (&v)[RegShape<N>::N1], const float4* rows, int t) {
+  using S = RegShape<N>;
+  constexpr int P = kTile / 2;
+#pragma unroll
+  for (int q = 0; q < S::C; ++q)
+#pragma unroll
+    for (int j = 0; j < S::T; ++j) v[q * S::T + j] = unpack4(rows[((q * S::T + t) * S::T + j) * P]);
+}
+template <int N, bool INV>
+__device__ __forceinline__ void pipe_step2(CPair (&v)[RegShape<N>::N1]) {
+  using S = RegShape<N>;
+#pragma unroll
+  for (int q = 0; q < S::C; ++q) PRegDft<S::T, INV>::run(v + q * S::T);
+}
+// after pipe_step2: element t + T m of the line (m = q + C k2) is v[pipe_index(m)]
+template <int N>
+__device__ __forceinline__ constexpr int pipe_index(int m) {
+  return (m % RegShape<N>::C) * RegShape<N>::T + m / RegShape<N>::C;
+}
+
+// Whole tiles only (`width` a multiple of 2 kTile) and counts on a 16-byte boundary.
+template <int N, bool FIRST_INV, bool SHIFTED, bool UNIT_NORM>
+__global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlocks) cols_sweep_pipe(
+    float2* __restrict__ scratch, int width, int nframes, int frame0, const float2* __restrict__ tw,
+    const uint16_t* __restrict__ measured, float scale, float norm, float grad_scale, double inv_numel,
+    double* __restrict__ loss) {
+  using S = RegShape<N>;
+  using Cfg = ColPipeCfg<N>;
+  constexpr int P = Cfg::kPairs;
+  extern __shared__ __align__(128) unsigned char pipe_smem[];
+  const int tid = threadIdx.x;
+  const int grp = tid / Cfg::kGroup, gt = tid - grp * Cfg::kGroup;
+  const int p = gt % P, t = gt / P;
+  uint16_t* meas_s = reinterpret_cast<uint16_t*>(pipe_smem + Cfg::kBufs * Cfg::kTileBytes + grp * Cfg::kMeasBytes);
+  float2* tws = reinterpret_cast<float2*>(pipe_smem + Cfg::kBufs * Cfg::kTileBytes + 2 * Cfg::kMeasBytes);
+  uint64_t* full = reinterpret_cast<uint64_t*>(tws + N / 2);
+  for (int i = tid; i < N / 2; i += blockDim.x) tws[i] = __ldg(&tw[i]);
+  if (tid == 0) {
+    for (int b = 0; b < Cfg::kBufs; ++b) mbar_init(full + b, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  __syncthreads();
+  pdl_wait();
+  const int tiles = width / kTile;
+  const long long total = (long long)tiles * nframes;
+  const int n = static_cast<int>((total - blockIdx.x + gridDim.x - 1) / gridDim.x);
+  const uint64_t pol = policy_evict_first();
+  auto tile_at = [&](int i) { return blockIdx.x + (long long)i * gridDim.x; };
+  auto issue = [&](int i) {
+    bulk_load(pipe_smem + (i % Cfg::kBufs) * Cfg::kTileBytes, scratch + tile_at(i) * N * kTile, Cfg::kTileBytes,
+              full + i % Cfg::kBufs, pol);
+  };
+  if (tid == 0) {
+    for (int i = 0; i < Cfg::kBufs && i < n; ++i) issue(i);
+  }
+  constexpr int kRowOff = SHIFTED ? N / 2 : 0;
+  const int col_off = SHIFTED ? width / 2 : 0;
+  const float2 gs = f2(grad_scale), nrm = f2(norm), sc_y = f2(scale);
+  double acc = 0.0;
+  bool late = false;
+  for (int i = grp; i < n; i += 2) {
+    const long long tile = tile_at(i);
+    const int f = static_cast<int>(tile / tiles), c0 = static_cast<int>(tile - (long long)f * tiles) * kTile;
+    // the tile's counts, by rows of the spectrum; the previous tile's were read before a barrier
+    {
+      int ic0 = c0 + col_off;
+      if (ic0 >= width) ic0 -= width;
+      const uint16_t* src = measured + ((size_t)frame0 + f) * N * width + ic0;
+#pragma unroll 4
+      for (int e = gt; e < 2 * N; e += Cfg::kGroup) {
+        const int kr = e >> 1, h = (e & 1) * 8;
+        cp_async16(meas_s + kr * kTile + h, src + (size_t)((kr + kRowOff) & (N - 1)) * width + h);
+      }
+      cp_async_commit();
+    }
+    float4* rows = reinterpret_cast<float4*>(pipe_smem + (i % Cfg::kBufs) * Cfg::kTileBytes) + p;
+    late |= !mbar_wait(full + i % Cfg::kBufs, (i / Cfg::kBufs) & 1);
+    CPair v[S::N1];
+#pragma unroll
+    for (int j = 0; j < S::N1; ++j) {
+      const float4 q = rows[(t + S::T * j) * P];
+      v[j] = {make_float2(q.x, q.z), make_float2(q.y, q.w)};
+    }
+    pipe_step1<N, FIRST_INV>(v, rows, t, tws);
+    group_sync(1 + grp, Cfg::kGroup);
+    pipe_load2<N>(v, rows, t);
+    pipe_step2<N, FIRST_INV>(v);
+    cp_async_wait_all();
+    group_sync(1 + grp, Cfg::kGroup);  // the exchange is read, the counts are complete
+    float2 part = make_float2(0.f, 0.f);  // squared residuals of the two columns
+    CPair g[S::N1];
+#pragma unroll
+    for (int m = 0; m < S::N1; ++m) {
+      const int kr = t + S::T * m;
+      const CPair z = v[pipe_index<N>(m)];
+      const CPair F = UNIT_NORM ? z : CPair{mul2(z.re, nrm), mul2(z.im, nrm)};
+      const float2 s2 = fma2(F.re, F.re, mul2(F.im, F.im));
+      // the reciprocal square root and its Newton-Raphson step as in cols_sweep_pair
+      const float2 sc2 = make_float2(fmaxf(s2.x, 1e-37f), fmaxf(s2.y, 1e-37f));
+      const float2 y0 = make_float2(rsqrt_floor(sc2.x), rsqrt_floor(sc2.y));
+      const float2 r = mul2(y0, fma2(mul2(f2(-0.5f), sc2), mul2(y0, y0), f2(1.5f)));
+      const float2 a = mul2(s2, r);
+      const float2 inv =
+          make_float2(a.x >= kEpsF32 ? r.x : 1.0f / kEpsF32, a.y >= kEpsF32 ? r.y : 1.0f / kEpsF32);
+      const float2 rr = sub2(a, decode_amplitudes(*reinterpret_cast<const uint32_t*>(meas_s + kr * kTile + 2 * p), sc_y));
+      part = fma2(rr, rr, part);
+      const float2 sc = mul2(mul2(gs, rr), inv);
+      g[m] = {mul2(F.re, sc), mul2(F.im, sc)};
+    }
+    acc += static_cast<double>(part.x) + static_cast<double>(part.y);
+    pipe_step1<N, !FIRST_INV>(g, rows, t, tws);
+    group_sync(1 + grp, Cfg::kGroup);
+    pipe_load2<N>(g, rows, t);
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    group_sync(1 + grp, Cfg::kGroup);  // the buffer is free
+    if (gt == 0 && i + Cfg::kBufs < n) issue(i + Cfg::kBufs);
+    pipe_step2<N, !FIRST_INV>(g);
+    float4* out = reinterpret_cast<float4*>(scratch + tile * N * kTile) + p;
+#pragma unroll
+    for (int m = 0; m < S::N1; ++m) {
+      const CPair z = g[pipe_index<N>(m)];
+      out[(t + S::T * m) * P] = make_float4(z.re.x, z.im.x, z.re.y, z.im.y);
+    }
+  }
+  // a copy that never came leaves no valid result: the loss says so
+  block_add_double(late ? __longlong_as_double(0x7ff8000000000000ll) : acc, inv_numel, loss);
+}
+
+// Column lengths the pipeline is used for, and the frames it takes: whole pairs of tiles (the
+// counts' 16-byte pieces stay inside a tile), counts on a 16-byte boundary.
+template <int N>
+constexpr bool col_pipe_length() {
+  return N == 512;
+}
+inline bool col_pipe_takes(int width, const uint16_t* measured) {
+  return width % (2 * kTile) == 0 && (reinterpret_cast<uintptr_t>(measured) & 15) == 0;
+}
+template <int N, bool FIRST_INV, bool SHIFTED, bool UNIT_NORM>
+int prepare_col_pipe() {
+  return ensure_smem((const void*)cols_sweep_pipe<N, FIRST_INV, SHIFTED, UNIT_NORM>, ColPipeCfg<N>::kSmemBytes);
+}
+template <int N, bool FIRST_INV, bool SHIFTED, bool UNIT_NORM>
+void launch_col_pipe(float2* frames, int width, int nframes, int frame0, const float2* tw, const uint16_t* measured,
+                     float scale, float norm, float grad_scale, double inv_numel, double* loss, cudaStream_t s) {
+  using C = ColPipeCfg<N>;
+  auto kern = cols_sweep_pipe<N, FIRST_INV, SHIFTED, UNIT_NORM>;
+  const int grid =
+      persistent_grid((const void*)kern, 2 * C::kGroup, C::kSmemBytes, (long long)num_tiles(width) * nframes);
+  launch_pdl(kern, grid, 2 * C::kGroup, C::kSmemBytes, s, frames, width, nframes, frame0, tw, measured, scale, norm,
+             grad_scale, inv_numel, loss);
 }
 
 }  // namespace ptx

@@ -32,7 +32,7 @@
 namespace ptx {
 namespace {
 
-constexpr size_t kSpHeader = 256 + kLutBytes;       // error word + padding, count-decode table
+constexpr size_t kSpHeader = 256 + kReservedBytes;  // error word + padding
 constexpr size_t kSpTargetScratch = 4096ull << 20;  // upper bound on workspace frames
 constexpr int kSpCols = 8;                          // columns per column-pass CTA
 constexpr int kSpRowThreads = 128;
@@ -247,7 +247,6 @@ struct SpGeom {
   const MixSubpixOps* mcol;  // mixed-radix column passes (ph not a power of two), else null
   const MixSubpixOps* mrow;  // mixed-radix row passes (pw not a power of two), else null
   unsigned* err;
-  float* lut;
   float2* rx;
   float2* ry;
   float2* scratch;
@@ -296,7 +295,6 @@ int sp_check(const void* sample, int H, int W, const void* probe, int ph, int pw
   }
   char* base = static_cast<char*>(ws);
   g->err = reinterpret_cast<unsigned*>(base);
-  g->lut = reinterpret_cast<float*>(base + 256);
   g->rx = reinterpret_cast<float2*>(base + kSpHeader);
   g->ry = g->rx + (size_t)std::max(batch, 1) * pw;
   g->scratch = reinterpret_cast<float2*>(base + fixed);
@@ -402,10 +400,10 @@ int sp_launch_rows(const SpGeom& g, const float2* probe, float2* grad_probe, int
   return st;
 }
 
-int sp_launch_cols_sweep(const SpGeom& g, int frame0, int nf, const uint16_t* measured, float grad_scale,
+int sp_launch_cols_sweep(const SpGeom& g, int frame0, int nf, const uint16_t* measured, float scale, float grad_scale,
                          double inv_numel, double* loss, cudaStream_t s) {
   if (const MixOps* mo = (g.ph & (g.ph - 1)) ? mix_ops(g.ph) : nullptr) {
-    MixColsArgs a{g.scratch, g.ph, g.pw, frame0, nf, g.col.mix_twt, g.col.mix_twi, measured, g.lut,
+    MixColsArgs a{g.scratch, g.ph, g.pw, frame0, nf, g.col.mix_twt, g.col.mix_twi, measured, scale,
                   grad_scale, inv_numel, loss, nullptr, nullptr, nullptr};
     prof_begin(kBaseCols, s);
     mo->cols(kMixColSweep, a, s);
@@ -416,6 +414,17 @@ int sp_launch_cols_sweep(const SpGeom& g, int frame0, int nf, const uint16_t* me
   dispatch_pow2(g.ph, [&](auto NT) {
     constexpr int N = decltype(NT)::value;
     if constexpr (N >= 16) {
+      if constexpr (col_pipe_length<N>()) {
+        if (col_pipe_takes(g.pw, measured)) {
+          st = prepare_col_pipe<N, false, true, true>();
+          if (st) return;
+          prof_begin(kBaseCols, s);
+          launch_col_pipe<N, false, true, true>(g.scratch, g.pw, nf, frame0, g.col.tw, measured, scale, 1.0f, grad_scale,
+                                                inv_numel, loss, s);
+          prof_end(kBaseCols, s);
+          return;
+        }
+      }
       // the full-tile variant needs whole 16-column tiles
       auto kern = (g.pw % kTile == 0) ? cols_sweep_pair<N, false, true, true, true> : cols_sweep_pair<N, false, true, true>;
       st = ensure_smem((const void*)kern, ColPairCfg<N>::kSmemBytes);
@@ -423,7 +432,7 @@ int sp_launch_cols_sweep(const SpGeom& g, int frame0, int nf, const uint16_t* me
       dim3 grid(num_tiles(g.pw), nf);
       prof_begin(kBaseCols, s);
       launch_pdl(kern, grid, ColPairCfg<N>::kThreads, ColPairCfg<N>::kSmemBytes, s, g.scratch, g.pw, frame0,
-                 g.col.tw, measured, g.lut, 1.0f, grad_scale, inv_numel, loss);
+                 g.col.tw, measured, scale, 1.0f, grad_scale, inv_numel, loss);
       prof_end(kBaseCols, s);
     }
   });
@@ -465,13 +474,13 @@ int ptx_base_subpix_sweep(const float* sample, int sample_h, int sample_w, const
   const float2* P = reinterpret_cast<const float2*>(probe);
   const double numel = (double)batch * probe_h * probe_w;
   const float grad_scale = static_cast<float>(2.0 / std::max(numel, 1.0));
-  launch_prologue(s, GS, (size_t)sample_h * sample_w, GP, (size_t)probe_h * probe_w, loss, g.err, g.lut, scale);
+  launch_prologue(s, GS, (size_t)sample_h * sample_w, GP, (size_t)probe_h * probe_w, loss, g.err);
   sp_launch_ramps(g, positions_xy, s);
   for (int b0 = 0; b0 < batch; b0 += g.chunk) {
     const int nf = std::min(g.chunk, batch - b0);
     int st = sp_launch_cols<true>(g, S, nullptr, positions_xy, b0, nf, s);
     if (!st) st = sp_launch_rows<true, true, true>(g, P, nullptr, b0, nf, s, positions_xy);
-    if (!st) st = sp_launch_cols_sweep(g, b0, nf, measured, grad_scale, 1.0 / std::max(numel, 1.0), loss, s);
+    if (!st) st = sp_launch_cols_sweep(g, b0, nf, measured, scale, grad_scale, 1.0 / std::max(numel, 1.0), loss, s);
     if (!st) st = sp_launch_rows<false, false, false>(g, P, GP, b0, nf, s, positions_xy);
     if (!st) st = sp_launch_cols<false>(g, nullptr, GS, positions_xy, b0, nf, s);
     if (st) return st;
@@ -521,7 +530,7 @@ int ptx_base_subpix_backward(const float* grad_output, const float* far_field, c
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   float2* GS = reinterpret_cast<float2*>(grad_sample);
   float2* GP = reinterpret_cast<float2*>(grad_probe);
-  launch_prologue(s, GS, (size_t)sample_h * sample_w, GP, (size_t)probe_h * probe_w, nullptr, g.err, nullptr, 0.f);
+  launch_prologue(s, GS, (size_t)sample_h * sample_w, GP, (size_t)probe_h * probe_w, nullptr, g.err);
   sp_launch_ramps(g, positions_xy, s);
   const float2* S = reinterpret_cast<const float2*>(sample);
   const float2* P = reinterpret_cast<const float2*>(probe);
