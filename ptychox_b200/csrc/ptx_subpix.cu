@@ -141,94 +141,149 @@ __global__ void __launch_bounds__(kSpCols * RegShape<N>::T) subpix_cols_kernel(
   }
 }
 
-// Row passes (frame side M along the rows).  A CTA owns `lines` rows (T threads each, one
-// line per T lanes of a warp) of the frames [f0, f1); its probe rows, and in the adjoint the
-// grad_P partials of its rows, sit in shared memory (each thread touches only its own
-// elements, so no barrier guards them).
+// Row passes (frame side M along the rows), three transforms per row.  Work units are (row
+// group, frame) pairs in row-group-major order over one wave of resident CTAs (CTA b takes the
+// contiguous units [u0, u1)); T lanes of a warp own a line, so no block barrier is needed.  The
+// probe rows of the current row group and the twiddles (by thread) sit in shared memory, and
+// the next unit's frame row is requested by cp.async as soon as the last transform has released
+// the line buffer, so it lands while this unit stores.
 // FORWARD: row DFT, x ramp_x, inverse DFT (= S, stored into `sbuf` when STORE_S), x P, row
-// DFT (stored in place when STORE_OUT).  Adjoint: inverse row DFT (= G),
-// grad_P += G conj(S) (one float2 atomic per element per CTA at the end), G conj(P), row DFT,
-// x conj(ramp_x), inverse DFT, stored in place.
+// DFT (stored in place when STORE_OUT).  Adjoint: inverse row DFT (= G), grad_P += G conj(S) in
+// registers (one float2 atomic per element when a CTA leaves a row group), G conj(P), row
+// DFT, x conj(ramp_x), inverse DFT, stored in place; the S row lands beside the frame row.
+// Bound by the shared-memory path (30 wavefronts per 32 elements forward, about 0.8 ms for 900
+// frames of 512^2) and the 5.7 GB of frames (0.88 ms): 1764 us forward and 1867 us adjoint with
+// plain loads and 8 warps' exchanges through odd pitches, 1257 and 1292 us in this form.
+template <int M>
+struct SpRowCfg {
+  static constexpr int BP = row_line_pitch<M>() > M ? row_line_pitch<M>() : M;
+  static_assert(BP % 2 == 0, "16-byte landing lines");
+  static int smem(int lines, bool forward) { return (lines * (BP + (forward ? 1 : 2) * M) + M) * (int)sizeof(float2); }
+};
+
 template <int M, bool FORWARD, bool STORE_S, bool STORE_OUT>
-__global__ void __launch_bounds__(kSpRowThreads) subpix_rows_kernel(
+__global__ void __launch_bounds__(kSpRowThreads, FORWARD ? 3 : 2) subpix_rows_kernel(
     float2* __restrict__ scratch, float2* __restrict__ sbuf, int ph, const float2* __restrict__ probe, int nframes,
-    int frame0, int frames_per_cta, const float2* __restrict__ rx_all, float2* __restrict__ grad_probe,
+    int frame0, int rowgroups, const float2* __restrict__ rx_all, float2* __restrict__ grad_probe,
     const float2* __restrict__ tw, int lines) {
   pdl_wait();
   using S = RegShape<M>;
-  constexpr int LP = row_line_pitch<M>();
+  using Cfg = SpRowCfg<M>;
   constexpr int kTiles = M / kTile;
   extern __shared__ float2 sm[];
   const int tid = threadIdx.x;
   const int l = tid / S::T;  // blockDim.x = lines * T (whole warps: T and lines are powers of two)
   const int t = tid - l * S::T;
-  const int r = blockIdx.x * lines + l;
-  const bool row_ok = r < ph;
-  float2* buf = sm + l * LP;
-  float2* pbuf = sm + lines * LP + l * M;
-  float2* acc = sm + lines * (LP + M) + l * M;  // adjoint only
-  const int f0 = blockIdx.y * frames_per_cta;
-  const int f1 = min(nframes, f0 + frames_per_cta);
+  const long long units = (long long)rowgroups * nframes;
+  const long long u0 = units * blockIdx.x / gridDim.x;
+  const long long u1 = units * (blockIdx.x + 1) / gridDim.x;
+  if (u0 >= u1) return;
+  int g = static_cast<int>(u0 / nframes);
+  int f = static_cast<int>(u0 - (long long)g * nframes);
+  float2* buf = sm + l * Cfg::BP;
+  float2* pbuf = sm + lines * Cfg::BP + l * M;
+  float2* land = sm + lines * (Cfg::BP + M) + l * M;  // adjoint only: the S row
+  float2* tws = sm + lines * (Cfg::BP + (FORWARD ? 1 : 2) * M);
+  load_twiddles_by_thread<M>(tws, tw);
+  __syncthreads();
+  const uint64_t pol_first = policy_evict_first();
+  auto row_at = [&](int row, int frame) { return ((size_t)frame * kTiles * ph + row) * kTile; };
+  // element c of a tiled row
+  auto slot = [&](int c) { return (size_t)(c / kTile) * ph * kTile + (c % kTile); };
+  auto request = [&](const float2* src, float2* dst) {
 #pragma unroll
-  for (int m = 0; m < S::N1; ++m) {
-    const int k = t + S::T * m;
-    pbuf[k] = row_ok ? __ldg(&probe[(size_t)r * M + k]) : make_float2(0.f, 0.f);
-    if (!FORWARD) acc[k] = make_float2(0.f, 0.f);
+    for (int i = 0; i < S::N1 / 2; ++i) {
+      const int c = 2 * (t + S::T * i);
+      cp_async16_hint(dst + c, src + slot(c), pol_first);
+    }
+    cp_async_commit();
+  };
+  float2 acc[FORWARD ? 1 : S::N1];
+  if constexpr (!FORWARD) {
+#pragma unroll
+    for (int m = 0; m < S::N1; ++m) acc[m] = make_float2(0.f, 0.f);
   }
-  for (int f = f0; f < f1; ++f) {
+  int r = g * lines + l;
+  if (r < ph) request(scratch + row_at(r, f), buf);
+  bool new_group = true;
+  for (long long u = u0; u < u1; ++u) {
+    const bool row_ok = r < ph;
+    const size_t row0 = row_at(r, f);
     const float2* rx = rx_all + (size_t)(frame0 + f) * M;
-    const size_t row0 = (size_t)f * kTiles * ph * kTile + (size_t)r * kTile;
+    if (!FORWARD && row_ok) request(sbuf + row0, land);
+    if (new_group) {
+      // each thread copies and later reads its own elements
+#pragma unroll
+      for (int m = 0; m < S::N1; ++m) {
+        pbuf[t + S::T * m] = row_ok ? __ldg(&probe[(size_t)r * M + t + S::T * m]) : make_float2(0.f, 0.f);
+      }
+      new_group = false;
+    }
+    if (FORWARD || !row_ok) {
+      cp_async_wait_all();
+    } else {
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // the frame row
+    }
+    __syncwarp();
     float2 v[S::N1];
 #pragma unroll
-    for (int j = 0; j < S::N1; ++j) {
-      const int k = t + S::T * j;
-      v[j] = row_ok ? scratch[row0 + (size_t)(k / kTile) * ph * kTile + (k % kTile)] : make_float2(0.f, 0.f);
-    }
-    if (FORWARD) {
-      reg_fft<M, false, false>(v, buf, t, tw);
+    for (int j = 0; j < S::N1; ++j) v[j] = row_ok ? buf[t + S::T * j] : make_float2(0.f, 0.f);
+    __syncwarp();
+    if constexpr (FORWARD) {
+      reg_fft<M, false, false, true>(v, buf, t, tws);
 #pragma unroll
       for (int m = 0; m < S::N1; ++m) v[m] = cmul(v[m], __ldg(&rx[t + S::T * m]));
-      reg_fft<M, true, false>(v, buf, t, tw);
+      reg_fft<M, true, false, true>(v, buf, t, tws);
       if (STORE_S && row_ok) {
 #pragma unroll
-        for (int j = 0; j < S::N1; ++j) {
-          const int k = t + S::T * j;
-          sbuf[row0 + (size_t)(k / kTile) * ph * kTile + (k % kTile)] = v[j];
-        }
+        for (int j = 0; j < S::N1; ++j) sbuf[row0 + slot(t + S::T * j)] = v[j];
       }
       if constexpr (STORE_OUT) {
 #pragma unroll
         for (int m = 0; m < S::N1; ++m) v[m] = cmul(v[m], pbuf[t + S::T * m]);
-        reg_fft<M, false, false>(v, buf, t, tw);
+        reg_fft<M, false, false, true>(v, buf, t, tws);
       }
     } else {
-      reg_fft<M, true, false>(v, buf, t, tw);
+      reg_fft<M, true, false, true>(v, buf, t, tws);
+      cp_async_wait_all();  // the S row
+      __syncwarp();
 #pragma unroll
       for (int m = 0; m < S::N1; ++m) {
         const int k = t + S::T * m;
-        const float2 s = row_ok ? sbuf[row0 + (size_t)(k / kTile) * ph * kTile + (k % kTile)] : make_float2(0.f, 0.f);
-        acc[k] = cadd(acc[k], cmulc(v[m], s));
+        if (row_ok) acc[m] = cadd(acc[m], cmulc(v[m], land[k]));
         v[m] = cmulc(v[m], pbuf[k]);
       }
-      reg_fft<M, false, false>(v, buf, t, tw);
+      reg_fft<M, false, false, true>(v, buf, t, tws);
 #pragma unroll
       for (int m = 0; m < S::N1; ++m) v[m] = cmulc(v[m], __ldg(&rx[t + S::T * m]));
-      reg_fft<M, true, false>(v, buf, t, tw);
+      reg_fft<M, true, false, true>(v, buf, t, tws);
     }
+    int gn = g, fn = f + 1;
+    if (fn == nframes) {
+      gn = g + 1;
+      fn = 0;
+    }
+    const int rn = gn * lines + l;
+    if (u + 1 < u1 && rn < ph) request(scratch + row_at(rn, fn), buf);
     if (row_ok && (STORE_OUT || !FORWARD)) {
 #pragma unroll
-      for (int j = 0; j < S::N1; ++j) {
-        const int k = t + S::T * j;
-        scratch[row0 + (size_t)(k / kTile) * ph * kTile + (k % kTile)] = v[j];
+      for (int j = 0; j < S::N1; ++j) scratch[row0 + slot(t + S::T * j)] = v[j];
+    }
+    if (u + 1 == u1 || gn != g) {
+      new_group = true;
+      if constexpr (!FORWARD) {
+        if (row_ok) {
+#pragma unroll
+          for (int m = 0; m < S::N1; ++m) {
+            atomicAdd(&grad_probe[(size_t)r * M + t + S::T * m], acc[m]);
+            acc[m] = make_float2(0.f, 0.f);
+          }
+        }
       }
     }
-  }
-  if (!FORWARD && row_ok) {
-#pragma unroll
-    for (int m = 0; m < S::N1; ++m) {
-      const int k = t + S::T * m;
-      atomicAdd(&grad_probe[(size_t)r * M + k], acc[k]);
-    }
+    g = gn;
+    f = fn;
+    r = rn;
   }
 }
 
@@ -380,20 +435,16 @@ int sp_launch_rows(const SpGeom& g, const float2* probe, float2* grad_probe, int
   dispatch_pow2(g.pw, [&](auto NT) {
     constexpr int M = decltype(NT)::value;
     if constexpr (M >= 16) {
-      const int lines = std::min(kSpRowThreads / RegShape<M>::T, g.ph);
+      const int lines = RowPass<M>::lines(kSpRowThreads, g.ph);
       const int rowgroups = (g.ph + lines - 1) / lines;
-      const int smem = lines * (row_line_pitch<M>() + (FORWARD ? 1 : 2) * M) * (int)sizeof(float2);
+      const int threads = lines * RegShape<M>::T, smem = SpRowCfg<M>::smem(lines, FORWARD);
       auto kern = subpix_rows_kernel<M, FORWARD, STORE_S, STORE_OUT>;
       st = ensure_smem((const void*)kern, smem);
       if (st) return;
-      // about 8 CTAs per SM in all; each CTA keeps its probe rows (and grad_P partials) over its frames
-      const long long target = (long long)sm_count() * 8;
-      int fpc = static_cast<int>(std::max<long long>(1, ((long long)rowgroups * nf) / target));
-      fpc = std::min(fpc, std::max(nf, 1));
-      dim3 grid(rowgroups, (nf + fpc - 1) / fpc);
+      const int grid = persistent_grid((const void*)kern, threads, smem, (long long)rowgroups * nf);
       prof_begin(kSubpixRows, s);
-      launch_pdl(kern, grid, lines * RegShape<M>::T, smem, s, g.scratch, g.sbuf, g.ph, probe, nf, frame0, fpc, g.rx,
-                 grad_probe, g.row.tw, lines);
+      launch_pdl(kern, grid, threads, smem, s, g.scratch, g.sbuf, g.ph, probe, nf, frame0, rowgroups, g.rx, grad_probe,
+                 g.row.tw, lines);
       prof_end(kSubpixRows, s);
     }
   });
