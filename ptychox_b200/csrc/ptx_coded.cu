@@ -55,79 +55,133 @@ __device__ __forceinline__ int signed_freq(int k, int n) { return k < n / 2 ? k 
 
 // ---- column passes ---------------------------------------------------------------------
 // STAGE 1: load O^ T1 R, inverse DFT.  STAGE 3: forward DFT, x T2 (or conj(T2)/n when
-// CONJ), inverse DFT.  STAGE 7: forward DFT, /n, grad_O^ += . conj(T1 R).
-template <int STAGE, bool CONJ, int N>
+// CONJ), inverse DFT.  STAGE 7: forward DFT, /n, grad += . conj(R) (T1's conjugate follows in
+// the spectrum gradient's own transform, as O^ comes with T1 applied).
+// Work units are (8-column strip, frame) pairs in strip-major order over one wave of resident
+// CTAs (CTA b takes the contiguous units [u0, u1)).  A unit's strip of the frame (of O^ T1 in
+// stage 1) lands by cp.async in the exchange buffer as soon as the previous unit's last exchange
+// has been read, with the frame's y ramp beside it, so both arrive while that unit finishes.
+// Bound by issue and the shared-memory path (16 warps per SM): stage 1 335 -> 195 us and stage 7
+// 346 -> 204 us for 64 frames of 1024^2 against the same transforms with plain loads, twiddles
+// from global memory and the ramp evaluated per element; the frames alone would take 83 us each.
+template <int N>
+struct CodedColCfg {
+  using S = RegShape<N>;
+  static constexpr int kThreads = kColsPerCta * S::T;
+  // exchange pitch per column: even rows (reg_fft's 16-byte reads), = 2 (mod 16) float2, so that
+  // 8 columns x 2 rows of a half-warp fall in different bank pairs
+  static constexpr int LP = S::BUFV + ((2 - S::BUFV % 16) + 16) % 16;
+  static constexpr int kBuf = kColsPerCta * (LP > N ? LP : N);
+  static int smem(bool table) { return (kBuf + N + (table ? 2 * N : 0)) * (int)sizeof(float2); }
+};
+
+template <int STAGE, bool CONJ, bool TABLE, int N>
 __global__ void __launch_bounds__(256, 2) coded_cols(
-    float2* __restrict__ scratch, const float2* __restrict__ ospec, const float2* __restrict__ t1,
-    const float2* __restrict__ t2, const float* __restrict__ shifts, float inv_n, float2* __restrict__ grad_ospec,
-    const float2* __restrict__ tw, double* __restrict__ grad_shifts) {
+    float2* __restrict__ scratch, const float2* __restrict__ ospec, const float2* __restrict__ t2,
+    const float* __restrict__ shifts, const float2* __restrict__ ramps, float inv_n, int nframes,
+    float2* __restrict__ grad_ospec, const float2* __restrict__ tw, double* __restrict__ grad_shifts) {
   pdl_wait();
   using S = RegShape<N>;
-  using CP = ColPass<N>;
-  extern __shared__ float2 sm[];
+  using Cfg = CodedColCfg<N>;
+  constexpr bool kRamp = STAGE != 3;
+  extern __shared__ __align__(16) float2 sm[];
+  float2* tws = sm + Cfg::kBuf;
+  float2* rys = tws + N;  // [2][N], TABLE only
   const int tid = threadIdx.x;
   const int c = tid % kColsPerCta;
   const int t = tid / kColsPerCta;
+  constexpr int kStrips = N / kColsPerCta;
   constexpr int kSubs = kTile / kColsPerCta;
-  constexpr int kTiles = (N + kTile - 1) / kTile;
-  const int ct = blockIdx.x / kSubs;
-  const int c0 = ct * kTile + (blockIdx.x - ct * kSubs) * kColsPerCta;
-  const int f = blockIdx.y;
-  const int kc = c0 + c;
-  const bool col_ok = kc < N;
-  float2* tile = scratch + ((size_t)f * kTiles + ct) * N * kTile + (c0 - ct * kTile);
-  float2* buf = sm + c * CP::LP;
-  float2 v[S::N1];
-  const float dx = (STAGE == 1 || STAGE == 7) ? shifts[2 * f] : 0.f;
-  const float dy = (STAGE == 1 || STAGE == 7) ? shifts[2 * f + 1] : 0.f;
-  const int fx = signed_freq(kc, N);
-
-  if (STAGE == 1) {
+  const long long units = (long long)kStrips * nframes;
+  const long long u0 = units * blockIdx.x / gridDim.x;
+  const long long u1 = units * (blockIdx.x + 1) / gridDim.x;
+  if (u0 >= u1) return;
+  load_twiddles_by_thread<N>(tws, tw);
+  float2* buf = sm + c * Cfg::LP;
+  const uint64_t pol = STAGE == 1 ? policy_evict_last() : policy_evict_first();
+  auto strip_at = [&](int strip, int f) {  // a frame's strip: rows of kTile elements
+    return scratch + ((size_t)f * (N / kTile) + strip / kSubs) * N * kTile + (strip % kSubs) * kColsPerCta;
+  };
+  auto request = [&](int strip, int f, int slot) {
+    const float2* src = STAGE == 1 ? ospec + strip * kColsPerCta : strip_at(strip, f);
+    constexpr int pitch = STAGE == 1 ? N : kTile;
+#pragma unroll 4
+    for (int i = tid; i < N * kColsPerCta / 2; i += Cfg::kThreads) {
+      const int r = i / (kColsPerCta / 2), q = i % (kColsPerCta / 2);
+      cp_async16_hint(sm + 2 * i, src + (size_t)r * pitch + 2 * q, pol);
+    }
+    if constexpr (kRamp && TABLE) {
+      const float2* ry = ramps + ((size_t)2 * f + 1) * N;
+      for (int i = tid; i < N / 2; i += Cfg::kThreads) cp_async16(rys + slot * N + 2 * i, ry + 2 * i);
+    }
+    cp_async_commit();
+  };
+  int strip = static_cast<int>(u0 / nframes);
+  int f = static_cast<int>(u0 - (long long)strip * nframes);
+  request(strip, f, 0);
+  for (long long u = u0; u < u1; ++u) {
+    const int slot = static_cast<int>(u - u0) & 1;
+    const int kc = strip * kColsPerCta + c;
+    const int fx = signed_freq(kc, N);
+    // the ramp at row kr: exp(2 pi i dx fx) times exp(2 pi i dy fy) from the frame's tables, or evaluated
+    float2 ex = make_float2(1.f, 0.f);
+    float dx = 0.f, dy = 0.f;
+    if constexpr (kRamp) {
+      if constexpr (TABLE) {
+        ex = __ldg(&ramps[(size_t)2 * f * N + kc]);
+      } else {
+        dx = shifts[2 * f];
+        dy = shifts[2 * f + 1];
+      }
+    }
+    auto ramp = [&](int kr) {
+      if constexpr (TABLE) {
+        return cmul(ex, rys[slot * N + kr]);
+      } else {
+        return shift_ramp(dx, dy, fx, signed_freq(kr, N));
+      }
+    };
+    cp_async_wait_all();
+    __syncthreads();
+    float2 v[S::N1];
 #pragma unroll
     for (int j = 0; j < S::N1; ++j) {
       const int kr = t + S::T * j;
-      float2 w = make_float2(0.f, 0.f);
-      if (col_ok) {
-        const size_t idx = (size_t)kr * N + kc;
-        w = cmul(ospec[idx], shift_ramp(dx, dy, fx, signed_freq(kr, N)));
-        if (t1) w = cmul(w, t1[idx]);
-      }
-      v[j] = w;
+      v[j] = sm[kr * kColsPerCta + c];
+      if constexpr (STAGE == 1) v[j] = cmul(v[j], ramp(kr));
     }
-    reg_fft<N, true, true>(v, buf, t, tw);
-  } else {
-#pragma unroll
-    for (int j = 0; j < S::N1; ++j) v[j] = col_ok ? tile[(t + S::T * j) * kTile + c] : make_float2(0.f, 0.f);
-    reg_fft<N, false, true>(v, buf, t, tw);
-    if (STAGE == 3) {
+    __syncthreads();  // the strip is read
+    reg_fft<N, STAGE == 1, true, true>(v, buf, t, tws);
+    if constexpr (STAGE == 3) {
 #pragma unroll
       for (int m = 0; m < S::N1; ++m) {
-        const int kr = t + S::T * m;
-        if (col_ok) {
-          const float2 h = t2[(size_t)kr * N + kc];
-          v[m] = CONJ ? cscale(cmulc(v[m], h), inv_n) : cmul(v[m], h);
-        }
+        const float2 h = __ldg(&t2[(size_t)(t + S::T * m) * N + kc]);
+        v[m] = CONJ ? cscale(cmulc(v[m], h), inv_n) : cmul(v[m], h);
       }
-      reg_fft<N, true, true>(v, buf, t, tw);
-    } else {  // STAGE 7
+      reg_fft<N, true, true, true>(v, buf, t, tws);
+    }
+    int sn = strip, fn = f + 1;
+    if (fn == nframes) {
+      sn = strip + 1;
+      fn = 0;
+    }
+    if (u + 1 < u1) request(sn, fn, slot ^ 1);
+    if constexpr (STAGE == 7) {
       // with grad_shifts: dL/d(dx, dy) += -2 pi sum (fx, fy) Im(conj(G) u), G = v / n the
       // gradient of u = O^ T1 R (the ramp is the only place the shifts enter)
       float sx = 0.f, sy = 0.f;
-      if (col_ok) {
 #pragma unroll
-        for (int m = 0; m < S::N1; ++m) {
-          const int kr = t + S::T * m;
-          const size_t idx = (size_t)kr * N + kc;
-          float2 w = shift_ramp(dx, dy, fx, signed_freq(kr, N));
-          if (t1) w = cmul(w, t1[idx]);
-          const float2 G = cscale(v[m], inv_n);
-          atomicAdd(&grad_ospec[idx], cmulc(G, w));
-          if (grad_shifts) {
-            const float2 u = cmul(ospec[idx], w);
-            const float im = fmaf(G.x, u.y, -G.y * u.x);  // Im(conj(G) u)
-            sx = fmaf(static_cast<float>(fx), im, sx);
-            sy = fmaf(static_cast<float>(signed_freq(kr, N)), im, sy);
-          }
+      for (int m = 0; m < S::N1; ++m) {
+        const int kr = t + S::T * m;
+        const size_t idx = (size_t)kr * N + kc;
+        const float2 w = ramp(kr);
+        const float2 G = cscale(v[m], inv_n);
+        atomicAdd(&grad_ospec[idx], cmulc(G, w));
+        if (grad_shifts) {
+          const float2 z = cmul(ospec[idx], w);
+          const float im = fmaf(G.x, z.y, -G.y * z.x);  // Im(conj(G) u)
+          sx = fmaf(static_cast<float>(fx), im, sx);
+          sy = fmaf(static_cast<float>(signed_freq(kr, N)), im, sy);
         }
       }
       if (grad_shifts) {
@@ -135,12 +189,91 @@ __global__ void __launch_bounds__(256, 2) coded_cols(
         block_add_double(static_cast<double>(sx), -kTwoPi, &grad_shifts[2 * f]);
         block_add_double(static_cast<double>(sy), -kTwoPi, &grad_shifts[2 * f + 1]);
       }
-      return;
-    }
-  }
-  if (col_ok) {
+    } else {
+      float2* out = strip_at(strip, f);
 #pragma unroll
-    for (int m = 0; m < S::N1; ++m) tile[(t + S::T * m) * kTile + c] = v[m];
+      for (int m = 0; m < S::N1; ++m) out[(t + S::T * m) * kTile + c] = v[m];
+    }
+    strip = sn;
+    f = fn;
+  }
+}
+
+// Stage 3 with the strip of T2 in shared memory: a CTA's two groups of threads take the strip's
+// frames in turn, each with its own exchange buffer and prefetched strips (as coded_cols), and
+// share T2 and the twiddles.
+template <int N>
+struct CodedFilterCfg {
+  using C = CodedColCfg<N>;
+  static constexpr int kSmemBytes = (2 * C::kBuf + N + N * kColsPerCta) * (int)sizeof(float2);
+};
+
+template <bool CONJ, int N>
+__global__ void __launch_bounds__(2 * CodedColCfg<N>::kThreads, 1) coded_cols_filter(
+    float2* __restrict__ scratch, const float2* __restrict__ t2, float inv_n, int nframes,
+    const float2* __restrict__ tw) {
+  pdl_wait();
+  using S = RegShape<N>;
+  using Cfg = CodedColCfg<N>;
+  extern __shared__ __align__(16) float2 sm[];
+  float2* tws = sm + 2 * Cfg::kBuf;
+  float2* t2s = tws + N;  // [N][8]
+  const int tid = threadIdx.x;
+  const int grp = tid / Cfg::kThreads, gt = tid - grp * Cfg::kThreads;
+  const int c = gt % kColsPerCta;
+  const int t = gt / kColsPerCta;
+  constexpr int kStrips = N / kColsPerCta;
+  constexpr int kSubs = kTile / kColsPerCta;
+  const long long units = (long long)kStrips * nframes;
+  const long long u0 = units * blockIdx.x / gridDim.x;
+  const long long u1 = units * (blockIdx.x + 1) / gridDim.x;
+  load_twiddles_by_thread<N>(tws, tw);
+  float2* land = sm + grp * Cfg::kBuf;
+  float2* buf = land + c * Cfg::LP;
+  const uint64_t pol_first = policy_evict_first(), pol_last = policy_evict_last();
+  auto sync = [&] { group_sync(1 + grp, Cfg::kThreads); };
+  auto strip_at = [&](int strip, int f) {
+    return scratch + ((size_t)f * (N / kTile) + strip / kSubs) * N * kTile + (strip % kSubs) * kColsPerCta;
+  };
+  // a strip of `pitch` elements per row to rows of 8, by `count` threads
+  auto copy = [&](float2* dst, const float2* src, int pitch, int i0, int count, uint64_t pol) {
+#pragma unroll 4
+    for (int i = i0; i < N * kColsPerCta / 2; i += count) {
+      const int r = i / (kColsPerCta / 2), q = i % (kColsPerCta / 2);
+      cp_async16_hint(dst + 2 * i, src + (size_t)r * pitch + 2 * q, pol);
+    }
+    cp_async_commit();
+  };
+  for (long long u = u0; u < u1;) {
+    // the frames [f0, f1) of one strip
+    const int strip = static_cast<int>(u / nframes);
+    const int f0 = static_cast<int>(u - (long long)strip * nframes);
+    const int f1 = static_cast<int>(min((long long)nframes, f0 + (u1 - u)));
+    u += f1 - f0;
+    __syncthreads();  // the previous strip's T2 is read
+    copy(t2s, t2 + strip * kColsPerCta, N, tid, 2 * Cfg::kThreads, pol_last);
+    if (f0 + grp < f1) copy(land, strip_at(strip, f0 + grp), kTile, gt, Cfg::kThreads, pol_first);
+    cp_async_wait_all();
+    __syncthreads();
+    for (int f = f0 + grp; f < f1; f += 2) {
+      float2 v[S::N1];
+#pragma unroll
+      for (int j = 0; j < S::N1; ++j) v[j] = land[(t + S::T * j) * kColsPerCta + c];
+      sync();  // the strip is read
+      reg_fft_with<N, false, true>(v, buf, t, tws, sync);
+#pragma unroll
+      for (int m = 0; m < S::N1; ++m) {
+        const float2 h = t2s[(t + S::T * m) * kColsPerCta + c];
+        v[m] = CONJ ? cscale(cmulc(v[m], h), inv_n) : cmul(v[m], h);
+      }
+      reg_fft_with<N, true, true>(v, buf, t, tws, sync);
+      if (f + 2 < f1) copy(land, strip_at(strip, f + 2), kTile, gt, Cfg::kThreads, pol_first);
+      float2* out = strip_at(strip, f);
+#pragma unroll
+      for (int m = 0; m < S::N1; ++m) out[(t + S::T * m) * kTile + c] = v[m];
+      cp_async_wait_all();
+      sync();
+    }
   }
 }
 
@@ -199,34 +332,6 @@ __global__ void __launch_bounds__(ColPairCfg<N>::kThreads, ColPairCfg<N>::kThrea
 
 // ---- row passes ------------------------------------------------------------------------
 
-template <int N>
-__device__ __forceinline__ void load_frame_row(const float2* __restrict__ scratch, int f, int r,
-                                               float2 (&v)[RegShape<N>::N1], int t) {
-  using S = RegShape<N>;
-  constexpr int kTiles = (N + kTile - 1) / kTile;
-  const float2* base = scratch + (size_t)f * kTiles * N * kTile + (size_t)r * kTile;
-#pragma unroll
-  for (int j = 0; j < S::N1; ++j) {
-    const int c = t + S::T * j;
-    v[j] = base[(size_t)(c / kTile) * N * kTile + (c % kTile)];
-  }
-}
-
-// Frame row r of frame f loaded straight into registers with loads that do not allocate in
-// L1 (the frames stream through once per pass; L1 is left to the twiddles and masks).
-template <int N>
-__device__ __forceinline__ void load_frame_row_stream(const float2* __restrict__ scratch, int f, int r,
-                                                      float2 (&v)[RegShape<N>::N1], int t, uint64_t pol) {
-  using S = RegShape<N>;
-  constexpr int kTiles = (N + kTile - 1) / kTile;
-  const float2* base = scratch + (size_t)f * kTiles * N * kTile + (size_t)r * kTile;
-#pragma unroll
-  for (int j = 0; j < S::N1; ++j) {
-    const int c = t + S::T * j;
-    const float4 q = ld_stream4(base + (size_t)(c / kTile) * N * kTile + (c % kTile) - (c & 1), pol);
-    v[j] = (c & 1) ? make_float2(q.z, q.w) : make_float2(q.x, q.y);
-  }
-}
 // Frame row r of frame f into the line buffer `dst` (element c at dst[c]) by 16-byte
 // cp.async that bypasses L1; thread t of the line's T threads copies chunks t + T i, so the
 // line meets at a warp barrier after the wait before reading.
@@ -341,83 +446,125 @@ __global__ void __launch_bounds__(128, 3) coded_rows_mask(float2* __restrict__ s
 // Pass 4.  kCodedSweep: inverse row DFT, s = ./n, RMS pool over ds x ds, FP64 loss,
 // g_s = gA / (A ds^2) s, forward row DFT.  kCodedForward: inverse row DFT, write s and
 // the pooled amplitude.  kCodedBackward: g_s from saved s, amplitude and grad_output,
-// forward row DFT.  A CTA owns `lines` consecutive rows, a multiple of ds.
+// forward row DFT.  A CTA owns `lines` consecutive rows, a multiple of ds, per unit; units are
+// (row group, frame) pairs over one wave of resident CTAs, and the next unit's rows land by
+// cp.async once this unit's transforms have released the line buffers.  64 frames of 1024^2: 431
+// us with a CTA per unit, loads on demand and the pool's rows read a word at a time, 299 in this form.
 template <int MODE, int N>
 __global__ void __launch_bounds__(256, 2) coded_rows_pool(
-    float2* __restrict__ scratch, int ds, int frame0, float inv_n, const uint16_t* __restrict__ measured,
-    float scale, float grad_scale, double inv_numel, double* __restrict__ loss, float2* __restrict__ sensor,
-    float* __restrict__ amplitude, const float* __restrict__ grad_output, const float2* __restrict__ tw,
-    int lines) {
+    float2* __restrict__ scratch, int ds, int frame0, int nframes, int rowgroups, float inv_n,
+    const uint16_t* __restrict__ measured, float scale, float grad_scale, double inv_numel, double* __restrict__ loss,
+    float2* __restrict__ sensor, float* __restrict__ amplitude, const float* __restrict__ grad_output,
+    const float2* __restrict__ tw, int lines) {
   pdl_wait();
   using S = RegShape<N>;
+  constexpr int BP = CodedRowCfg<N>::BP;
   extern __shared__ float2 sm[];
-  float* pool = reinterpret_cast<float*>(sm + lines * RowPass<N>::LP);  // [lines][N] |s|^2, then factors
-  float2* tws = reinterpret_cast<float2*>(pool + lines * N);             // twiddles by thread
+  float* pool = reinterpret_cast<float*>(sm + lines * BP);    // [lines][N] |s|^2
+  float2* tws = reinterpret_cast<float2*>(pool + lines * N);  // twiddles by thread
+  float* factor = reinterpret_cast<float*>(tws + N);          // per pooled pixel
   load_twiddles_by_thread<N>(tws, tw);
   __syncthreads();
   const int tid = threadIdx.x;
   const int l = tid / S::T;
   const int t = tid - l * S::T;
-  const int r0 = blockIdx.x * lines;
-  const int r = r0 + l;
-  const int f = blockIdx.y;
-  const size_t g = (size_t)frame0 + f;
-  const int lw = N / ds;  // pooled width
-  float2 v[S::N1];
-  if (MODE == kCodedBackward) {
-    const float2* srow = sensor + (g * N + r) * N;
-    const float* arow = amplitude + (g * lw + r / ds) * lw;
-    const float* grow = grad_output + (g * lw + r / ds) * lw;
+  const int sh = __ffs(ds) - 1;  // ds divides the power of two N
+  const int lw = N >> sh;        // pooled width
+  const long long units = (long long)rowgroups * nframes;
+  const long long u0 = units * blockIdx.x / gridDim.x;
+  const long long u1 = units * (blockIdx.x + 1) / gridDim.x;
+  float2* buf = sm + l * BP;
+  const uint64_t pol_first = policy_evict_first();
+  int rg = static_cast<int>(u0 / nframes);
+  int f = static_cast<int>(u0 - (long long)rg * nframes);
+  double acc = 0.0;
+  if (MODE != kCodedBackward && u0 < u1) prefetch_frame_row<N>(buf, scratch, f, rg * lines + l, t, pol_first);
+  for (long long u = u0; u < u1; ++u) {
+    const int r0 = rg * lines, r = r0 + l;
+    const size_t g = (size_t)frame0 + f;
+    float2 v[S::N1];
+    if (MODE == kCodedBackward) {
+      const float2* srow = sensor + (g * N + r) * N;
+      const float* arow = amplitude + (g * lw + (r >> sh)) * lw;
+      const float* grow = grad_output + (g * lw + (r >> sh)) * lw;
 #pragma unroll
-    for (int m = 0; m < S::N1; ++m) {
-      const int c = t + S::T * m;
-      const float a = fmaxf(arow[c / ds], kAmpFloor);
-      v[m] = cscale(srow[c], grow[c / ds] / (a * static_cast<float>(ds * ds)));
-    }
-  } else {
-    load_frame_row_stream<N>(scratch, f, r, v, t, policy_evict_first());
-    reg_fft<N, true, false, true>(v, sm + l * RowPass<N>::LP, t, tws);
-#pragma unroll
-    for (int m = 0; m < S::N1; ++m) {
-      v[m] = cscale(v[m], inv_n);
-      pool[l * N + t + S::T * m] = cabs2(v[m]);
-    }
-    __syncthreads();
-    // pooled values of this CTA: (lines/ds) x lw, one per thread-iteration
-    const int nb = (lines / ds) * lw;
-    double acc = 0.0;
-    for (int q = tid; q < nb; q += blockDim.x) {
-      const int py = q / lw, px = q - py * lw;
-      float sum = 0.f;
-      for (int yy = 0; yy < ds; ++yy)
-        for (int xx = 0; xx < ds; ++xx) sum += pool[(py * ds + yy) * N + px * ds + xx];
-      const float a = sqrtf(fmaxf(sum / static_cast<float>(ds * ds), 0.f));
-      const size_t oidx = (g * lw + r0 / ds + py) * lw + px;
-      if (MODE == kCodedForward) {
-        amplitude[oidx] = a;
-      } else {
-        const float y = sqrtf(static_cast<float>(measured[oidx]) * scale);
-        const float d = a - y;
-        acc += static_cast<double>(d) * static_cast<double>(d);
-        // store the factor gA / (A ds^2) at the block's first pixel
-        pool[(py * ds) * N + px * ds] = grad_scale * d / (fmaxf(a, kAmpFloor) * static_cast<float>(ds * ds));
+      for (int m = 0; m < S::N1; ++m) {
+        const int c = t + S::T * m;
+        const float a = fmaxf(arow[c >> sh], kAmpFloor);
+        v[m] = cscale(srow[c], grow[c >> sh] / (a * static_cast<float>(ds * ds)));
       }
+    } else {
+      cp_async_wait_all();
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < S::N1; ++j) v[j] = buf[t + S::T * j];
+      __syncwarp();
+      reg_fft<N, true, false, true>(v, buf, t, tws);
+#pragma unroll
+      for (int m = 0; m < S::N1; ++m) {
+        v[m] = cscale(v[m], inv_n);
+        pool[l * N + t + S::T * m] = cabs2(v[m]);
+      }
+      __syncthreads();
+      // pooled values of this unit: (lines/ds) x lw, one per thread-iteration
+      const int nb = (lines >> sh) * lw;
+      for (int q = tid; q < nb; q += blockDim.x) {
+        const int py = q >> (S::LOG - sh), px = q & (lw - 1);
+        const float* p = pool + (py * ds) * N + px * ds;
+        float sum = 0.f;
+        if (ds == 4) {
+#pragma unroll
+          for (int yy = 0; yy < 4; ++yy) {  // 16-byte reads, the same order of summation
+            const float4 x = *reinterpret_cast<const float4*>(p + yy * N);
+            sum = (((sum + x.x) + x.y) + x.z) + x.w;
+          }
+        } else if (ds == 2) {
+#pragma unroll
+          for (int yy = 0; yy < 2; ++yy) {
+            const float2 x = *reinterpret_cast<const float2*>(p + yy * N);
+            sum = (sum + x.x) + x.y;
+          }
+        } else {
+          for (int yy = 0; yy < ds; ++yy)
+            for (int xx = 0; xx < ds; ++xx) sum += p[yy * N + xx];
+        }
+        const float a = sqrtf(fmaxf(sum / static_cast<float>(ds * ds), 0.f));
+        const size_t oidx = (g * lw + (r0 >> sh) + py) * lw + px;
+        if (MODE == kCodedForward) {
+          amplitude[oidx] = a;
+        } else {
+          const float d = a - sqrtf(static_cast<float>(measured[oidx]) * scale);
+          acc += static_cast<double>(d) * static_cast<double>(d);
+          // the factor gA / (A ds^2) of the block
+          factor[q] = grad_scale * d / (fmaxf(a, kAmpFloor) * static_cast<float>(ds * ds));
+        }
+      }
+      __syncthreads();
     }
+    int gn = rg, fn = f + 1;
+    if (fn == nframes) {
+      gn = rg + 1;
+      fn = 0;
+    }
+    const bool more = MODE != kCodedBackward && u + 1 < u1;
     if (MODE == kCodedForward) {
+      if (more) prefetch_frame_row<N>(buf, scratch, fn, gn * lines + l, t, pol_first);
       float2* srow = sensor + (g * N + r) * N;
 #pragma unroll
       for (int m = 0; m < S::N1; ++m) srow[t + S::T * m] = v[m];
-      return;
-    }
-    block_add_double(acc, inv_numel, loss);  // synchronises the block
+    } else {
+      if (MODE == kCodedSweep) {
 #pragma unroll
-    for (int m = 0; m < S::N1; ++m) {
-      const int c = t + S::T * m;
-      v[m] = cscale(v[m], pool[((l / ds) * ds) * N + (c / ds) * ds]);
+        for (int m = 0; m < S::N1; ++m) v[m] = cscale(v[m], factor[(l >> sh) * lw + ((t + S::T * m) >> sh)]);
+      }
+      reg_fft<N, false, false, true>(v, buf, t, tws);
+      if (more) prefetch_frame_row<N>(buf, scratch, fn, gn * lines + l, t, pol_first);
+      store_frame_row<N>(scratch, f, r, v, t);
     }
+    rg = gn;
+    f = fn;
   }
-  reg_fft<N, false, false, true>(v, sm + l * RowPass<N>::LP, t, tws);
-  store_frame_row<N>(scratch, f, r, v, t);
+  if (MODE == kCodedSweep) block_add_double(acc, inv_numel, loss);
 }
 
 // Pass 6: inverse row DFT (g_a), grad_M += g_a conj(x) in registers over the CTA's frames,
@@ -597,6 +744,11 @@ int coded_lines(int n) {
   return lines;
 }
 
+// Pass 4 beyond its exchange lines: |s|^2, the twiddles, the factor of each pooled pixel
+int pool_bytes(int lines, int n, int ds) {
+  return (lines * n + (lines / ds) * (n / ds)) * (int)sizeof(float) + n * (int)sizeof(float2);
+}
+
 int coded_check(int n, int ds, const void* a, const void* b, const void* t2, const float* shifts, int batch, void* ws,
                 size_t ws_bytes, bool need_xstore, CodedGeom* g) {
   if (!a || !b || !t2 || (!shifts && batch > 0) || !ws) return set_error(PTX_ERR_INVALID_ARGUMENT, "null pointer argument");
@@ -649,18 +801,28 @@ int coded_check(int n, int ds, const void* a, const void* b, const void* t2, con
     constexpr int N = decltype(NT)::value;
     const int rs = RowPass<N>::smem(lines);
     const int lines128 = RowPass<N>::lines(128, N);
-    const int pool = rs + lines * N * (int)sizeof(float) + N * (int)sizeof(float2);
+    const int pool = lines * CodedRowCfg<N>::BP * (int)sizeof(float2) + pool_bytes(lines, N, ds);
     const int cs = kColsPerCta * ColPass<N>::LP * (int)sizeof(float2);
     if (!st) st = ensure_smem((const void*)fft2_rows_kernel<N, false>, rs);
     if (!st) st = ensure_smem((const void*)fft2_rows_kernel<N, true>, rs);
     if (!st) st = ensure_smem((const void*)fft2_cols_kernel<N, false>, cs);
     if (!st) st = ensure_smem((const void*)fft2_cols_kernel<N, true>, cs);
-    if (!st) st = ensure_smem((const void*)coded_cols<1, false, N>, cs);
-    if (!st) st = ensure_smem((const void*)coded_cols<3, false, N>, cs);
-    if (!st) st = ensure_smem((const void*)coded_cols<3, true, N>, cs);
-    if (!st) st = ensure_smem((const void*)coded_cols_filter_pair<false, N>, ColPairCfg<N>::kExchBytes + ColPairCfg<N>::kTwBytes);
-    if (!st) st = ensure_smem((const void*)coded_cols_filter_pair<true, N>, ColPairCfg<N>::kExchBytes + ColPairCfg<N>::kTwBytes);
-    if (!st) st = ensure_smem((const void*)coded_cols<7, false, N>, cs);
+    if constexpr (N >= 16) {
+      using C = CodedColCfg<N>;
+      if (!st) st = ensure_smem((const void*)coded_cols<1, false, false, N>, C::smem(false));
+      if (!st) st = ensure_smem((const void*)coded_cols<1, false, true, N>, C::smem(true));
+      if constexpr (N == 1024) {
+        if (!st) st = ensure_smem((const void*)coded_cols_filter<false, N>, CodedFilterCfg<N>::kSmemBytes);
+        if (!st) st = ensure_smem((const void*)coded_cols_filter<true, N>, CodedFilterCfg<N>::kSmemBytes);
+      } else {
+        if (!st) st = ensure_smem((const void*)coded_cols_filter_pair<false, N>, ColPairCfg<N>::kExchBytes + ColPairCfg<N>::kTwBytes);
+        if (!st) st = ensure_smem((const void*)coded_cols_filter_pair<true, N>, ColPairCfg<N>::kExchBytes + ColPairCfg<N>::kTwBytes);
+      }
+      if (!st) st = ensure_smem((const void*)coded_cols<3, false, false, N>, C::smem(false));
+      if (!st) st = ensure_smem((const void*)coded_cols<3, true, false, N>, C::smem(false));
+      if (!st) st = ensure_smem((const void*)coded_cols<7, false, false, N>, C::smem(false));
+      if (!st) st = ensure_smem((const void*)coded_cols<7, false, true, N>, C::smem(true));
+    }
     if (!st) st = ensure_smem((const void*)coded_rows_mask<N>, CodedRowCfg<N>::smem(lines128, 1));
     if (!st) st = ensure_smem((const void*)coded_rows_pool<kCodedSweep, N>, pool);
     if (!st) st = ensure_smem((const void*)coded_rows_pool<kCodedForward, N>, pool);
@@ -669,6 +831,61 @@ int coded_check(int n, int ds, const void* a, const void* b, const void* t2, con
   });
   return st;
 }
+
+// Shift ramps of every frame, tabulated in FP64 and rounded once: ramps[f][0][k] =
+// exp(2 pi i dx_f fk), ramps[f][1][k] = exp(2 pi i dy_f fk), fk the signed frequency of bin k
+// (numpy fftfreq * n).  Part of the sweeps' first launch, which also zeroes what they accumulate
+// into.  Evaluating the two-dimensional ramp per element cost the column passes that apply it a
+// third of their instructions; the product of the two tables is also the more accurate (6e-8
+// against up to 2e-7 rad from the FP32 reduction of the summed argument).
+__global__ void __launch_bounds__(256) coded_prologue_kernel(float2* __restrict__ gospec, float2* __restrict__ grad_mask,
+                                                             size_t field, double* __restrict__ loss,
+                                                             double* __restrict__ grad_shifts,
+                                                             const float* __restrict__ shifts, int batch, int n,
+                                                             float2* __restrict__ ramps) {
+  pdl_wait();
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const float2 z = make_float2(0.f, 0.f);
+  for (size_t i = i0; i < field; i += stride) {
+    gospec[i] = z;
+    grad_mask[i] = z;
+  }
+  if (grad_shifts) {
+    for (size_t i = i0; i < 2 * (size_t)batch; i += stride) grad_shifts[i] = 0.0;
+  }
+  if (loss && i0 == 0) *loss = 0.0;
+  if (ramps) {
+    for (size_t i = i0; i < 2 * (size_t)batch * n; i += stride) {
+      const int k = static_cast<int>(i % n);
+      const double d = shifts[i / n];
+      double s, c;
+      sincospi(2.0 * d * (k <= (n - 1) / 2 ? k : k - n), &s, &c);
+      ramps[i] = make_float2(static_cast<float>(c), static_cast<float>(s));
+    }
+  }
+}
+
+// The ramp tables' place: grad_object, which nothing else writes before the last transform; null
+// where they do not fit (more frames than n / 2) or where the caller computes in place, and the
+// passes then evaluate the ramp themselves, as the mixed-radix ones do.
+float2* ramp_tables(int n, int batch, float* grad_object, const float* object, const float* coded_surface) {
+  const bool fits = is_pow2_len(n) && 2 * (long long)batch <= n && grad_object != object && grad_object != coded_surface &&
+                    (reinterpret_cast<uintptr_t>(grad_object) & 15) == 0;
+  return fits ? reinterpret_cast<float2*>(grad_object) : nullptr;
+}
+
+// The first launch of a sweep or adjoint.
+void launch_coded_prologue(const CodedGeom& g, float* grad_coded, double* loss, double* grad_shifts,
+                           const float* shifts, float2* ramps, cudaStream_t s) {
+  const size_t field = g.field_bytes / sizeof(float2);
+  prof_begin(kMiscKernel, s);
+  launch_pdl(coded_prologue_kernel, prologue_blocks(field, sm_count()), 256, 0, s, g.gospec,
+             reinterpret_cast<float2*>(grad_coded), field, loss, grad_shifts, shifts, g.batch, g.n, ramps);
+  prof_end(kMiscKernel, s);
+}
+
+const float2* ramps_at(const float2* ramps, int frame, int n) { return ramps ? ramps + 2 * (size_t)frame * n : nullptr; }
 
 // Arguments of the mixed-radix passes common to all of them; callers fill in the rest.
 MixCodedArgs mix_args(const CodedGeom& g, int nf, float inv_n) {
@@ -686,7 +903,7 @@ MixCodedArgs mix_args(const CodedGeom& g, int nf, float inv_n) {
 
 template <bool INV>
 void launch_fft2(const CodedGeom& g, const float2* in, int n, float2* out, float2* tmp, const LinePlan& p,
-                 cudaStream_t s) {
+                 const float2* t1, cudaStream_t s) {
   if (g.mix) {
     prof_begin(kFft2Rows, s);
     g.mfft->fft2_rows(INV, in, n, tmp, p.mix_twt, s);
@@ -701,18 +918,19 @@ void launch_fft2(const CodedGeom& g, const float2* in, int n, float2* out, float
     const int lines = RowPass<N>::lines(256, N);
     prof_begin(kFft2Rows, s);
     launch_pdl(fft2_rows_kernel<N, INV>, (N + lines - 1) / lines, lines * RowPass<N>::T, RowPass<N>::smem(lines), s,
-                in, N, tmp, p.tw, lines);
+                in, N, tmp, p.tw, lines, INV ? t1 : nullptr);
     prof_end(kFft2Rows, s);
     prof_begin(kFft2Cols, s);
     launch_pdl(fft2_cols_kernel<N, INV>, num_tiles(N) * (kTile / kColsPerCta), ColPass<N>::kThreads,
-               kColsPerCta * ColPass<N>::LP * (int)sizeof(float2), s, tmp, N, out, 1.0f, p.tw);
+               kColsPerCta * ColPass<N>::LP * (int)sizeof(float2), s, tmp, N, out, 1.0f, p.tw,
+               INV ? nullptr : t1);
     prof_end(kFft2Cols, s);
   });
 }
 
 template <int STAGE, bool CONJ>
 void launch_cols(const CodedGeom& g, int nf, const float2* t1, const float2* t2, const float* shifts,
-                 cudaStream_t s, double* grad_shifts = nullptr) {
+                 const float2* ramps, cudaStream_t s, double* grad_shifts = nullptr) {
   const float inv_n = 1.0f / static_cast<float>((double)g.n * g.n);
   prof_begin(kCodedCols, s);
   if (g.mix) {
@@ -727,20 +945,42 @@ void launch_cols(const CodedGeom& g, int nf, const float2* t1, const float2* t2,
   }
   dispatch_pow2(g.n, [&](auto NT) {
     constexpr int N = decltype(NT)::value;
-    if constexpr (STAGE == 3) {
-      // the paired kernel reads T2 two columns at a time (16-byte loads)
-      if ((reinterpret_cast<uintptr_t>(t2) & 15) == 0) {
-        using C = ColPairCfg<N>;
-        dim3 grid(num_tiles(N), nf);
-        launch_pdl(coded_cols_filter_pair<CONJ, N>, grid, C::kThreads, C::kExchBytes + C::kTwBytes, s, g.frames, t2,
-                   inv_n, g.plan.tw);
-        return;
+    if constexpr (N >= 16) {
+      if constexpr (STAGE == 3) {
+        // both take T2 by 16 bytes.  At 1024 points the paired kernel leaves one CTA of 8 warps per
+        // SM, so that its loads and stores stand alone (64 frames, both directions: 775 us, the
+        // strips with T2 in shared memory 675); shorter columns keep two to four CTAs and it is
+        // the faster one (16 frames of 512^2: 41.6 against 44.8 us, of 256^2: 13.2 against 15.9).
+        if ((reinterpret_cast<uintptr_t>(t2) & 15) == 0) {
+          if constexpr (N == 1024) {
+            constexpr int smem = CodedFilterCfg<N>::kSmemBytes, threads = 2 * CodedColCfg<N>::kThreads;
+            const int grid = persistent_grid((const void*)coded_cols_filter<CONJ, N>, threads, smem,
+                                             (long long)(N / kColsPerCta) * nf);
+            launch_pdl(coded_cols_filter<CONJ, N>, grid, threads, smem, s, g.frames, t2, inv_n, nf, g.plan.tw);
+          } else {
+            using C = ColPairCfg<N>;
+            dim3 grid(num_tiles(N), nf);
+            launch_pdl(coded_cols_filter_pair<CONJ, N>, grid, C::kThreads, C::kExchBytes + C::kTwBytes, s, g.frames, t2,
+                       inv_n, g.plan.tw);
+          }
+          return;
+        }
+      }
+      using C = CodedColCfg<N>;
+      auto run = [&](auto kern, bool table) {
+        const int smem = C::smem(table);
+        const int grid = persistent_grid((const void*)kern, C::kThreads, smem, (long long)(N / kColsPerCta) * nf);
+        launch_pdl(kern, grid, C::kThreads, smem, s, g.frames, g.ospec, t2, shifts, ramps, inv_n, nf, g.gospec,
+                   g.plan.tw, grad_shifts);
+      };
+      if constexpr (STAGE == 3) {
+        run(coded_cols<STAGE, CONJ, false, N>, false);
+      } else if (ramps) {
+        run(coded_cols<STAGE, CONJ, true, N>, true);
+      } else {
+        run(coded_cols<STAGE, CONJ, false, N>, false);
       }
     }
-    dim3 grid(num_tiles(N) * (kTile / kColsPerCta), nf);
-    launch_pdl(coded_cols<STAGE, CONJ, N>, grid, ColPass<N>::kThreads,
-               kColsPerCta * ColPass<N>::LP * (int)sizeof(float2), s, g.frames, g.ospec, t1, t2, shifts, inv_n,
-               g.gospec, g.plan.tw, STAGE == 7 ? grad_shifts : nullptr);
   });
   prof_end(kCodedCols, s);
 }
@@ -793,10 +1033,11 @@ void launch_rows_pool(const CodedGeom& g, int frame0, int nf, const uint16_t* me
   dispatch_pow2(g.n, [&](auto NT) {
     constexpr int N = decltype(NT)::value;
     const int lines = RowPass<N>::lines(256, N);
-    dim3 grid((N + lines - 1) / lines, nf);
-    const int smem = RowPass<N>::smem(lines) + lines * N * (int)sizeof(float) + N * (int)sizeof(float2);
-    launch_pdl(coded_rows_pool<MODE, N>, grid, lines * RowPass<N>::T, smem, s, g.frames, g.ds, frame0, inv_n,
-               measured, scale, grad_scale, inv_numel, loss, sensor, amplitude, grad_output, g.plan.tw, lines);
+    const int rowgroups = N / lines, threads = lines * RowPass<N>::T;
+    const int smem = lines * CodedRowCfg<N>::BP * (int)sizeof(float2) + pool_bytes(lines, N, g.ds);
+    const int grid = persistent_grid((const void*)coded_rows_pool<MODE, N>, threads, smem, (long long)rowgroups * nf);
+    launch_pdl(coded_rows_pool<MODE, N>, grid, threads, smem, s, g.frames, g.ds, frame0, nf, rowgroups, inv_n, measured,
+               scale, grad_scale, inv_numel, loss, sensor, amplitude, grad_output, g.plan.tw, lines);
   });
   prof_end(kCodedRows, s);
 }
@@ -827,11 +1068,11 @@ void launch_rows_grad_mask(const CodedGeom& g, int nf, const float2* mask, const
 
 // The adjoint passes 4 (backward part) to 7 for one chunk, given g_s already in the frames.
 void adjoint_tail(const CodedGeom& g, int nf, const float2* mask, const float2* t1, const float2* t2,
-                  const float* shifts, const float2* xstore, float2* grad_mask, cudaStream_t s,
+                  const float* shifts, const float2* ramps, const float2* xstore, float2* grad_mask, cudaStream_t s,
                   double* grad_shifts = nullptr) {
-  launch_cols<3, true>(g, nf, t1, t2, shifts, s);
+  launch_cols<3, true>(g, nf, t1, t2, shifts, ramps, s);
   launch_rows_grad_mask(g, nf, mask, xstore, grad_mask, s);
-  launch_cols<7, false>(g, nf, t1, t2, shifts, s, grad_shifts);
+  launch_cols<7, false>(g, nf, t1, t2, shifts, ramps, s, grad_shifts);
 }
 
 }  // namespace
@@ -844,7 +1085,8 @@ namespace {
 int coded_backward_impl(const float* grad_output, const float* x_forward, const float* sensor, const float* amplitude,
                         const float* coded_surface, const float* transfer_1, const float* transfer_2, int n,
                         const float* shifts_xy, int batch, int downsample, float* grad_object, float* grad_coded,
-                        void* workspace, size_t workspace_bytes, void* stream, double* grad_shifts, bool zero) {
+                        void* workspace, size_t workspace_bytes, void* stream, double* grad_shifts,
+                        const float2* ramps, bool prepared) {
   CodedGeom g;
   if (int st = coded_check(n, downsample, coded_surface, coded_surface, transfer_2, shifts_xy, batch, workspace,
                            workspace_bytes, false, &g)) {
@@ -860,20 +1102,21 @@ int coded_backward_impl(const float* grad_output, const float* x_forward, const 
   const float2* T1 = reinterpret_cast<const float2*>(transfer_1);
   const float2* T2 = reinterpret_cast<const float2*>(transfer_2);
   const float2* M = reinterpret_cast<const float2*>(coded_surface);
-  if (zero) {
-    const size_t field = g.field_bytes / sizeof(float2);
-    launch_prologue(s, g.gospec, field, reinterpret_cast<float2*>(grad_coded), field, nullptr, nullptr);
+  if (!prepared) {  // else the caller has launched the prologue
+    float2* tables = ramp_tables(n, batch, grad_object, nullptr, coded_surface);
+    launch_coded_prologue(g, grad_coded, nullptr, nullptr, shifts_xy, tables, s);
+    ramps = tables;
   }
   for (int b0 = 0; b0 < batch; b0 += g.chunk) {
     const int nf = std::min(g.chunk, batch - b0);
     launch_rows_pool<kCodedBackward>(g, b0, nf, nullptr, 0.f, 0.f, 0.0, nullptr,
                                      const_cast<float2*>(reinterpret_cast<const float2*>(sensor)),
                                      const_cast<float*>(amplitude), grad_output, s);
-    adjoint_tail(g, nf, M, T1, T2, shifts_xy + 2 * (size_t)b0,
+    adjoint_tail(g, nf, M, T1, T2, shifts_xy + 2 * (size_t)b0, ramps_at(ramps, b0, n),
                  reinterpret_cast<const float2*>(x_forward) + (size_t)b0 * n * n,
                  reinterpret_cast<float2*>(grad_coded), s, grad_shifts ? grad_shifts + 2 * (size_t)b0 : nullptr);
   }
-  launch_fft2<true>(g, g.gospec, n, reinterpret_cast<float2*>(grad_object), g.tmp, g.plan, s);
+  launch_fft2<true>(g, g.gospec, n, reinterpret_cast<float2*>(grad_object), g.tmp, g.plan, T1, s);
   return cuda_status(cudaGetLastError(), "ptx_coded_backward launch");
 }
 
@@ -889,9 +1132,10 @@ size_t ptx_coded_workspace_bytes(int n, int batch) {
   return coded_fixed_bytes(n) + frames * per;
 }
 
-int ptx_coded_forward(const float* object, const float* coded_surface, const float* transfer_1, const float* transfer_2,
-                      int n, const float* shifts_xy, int batch, int downsample, float* x_forward, float* sensor,
-                      float* amplitude, void* workspace, size_t workspace_bytes, void* stream) {
+static int coded_forward_impl(const float* object, const float* coded_surface, const float* transfer_1,
+                              const float* transfer_2, int n, const float* shifts_xy, int batch, int downsample,
+                              float* x_forward, float* sensor, float* amplitude, void* workspace,
+                              size_t workspace_bytes, const float2* ramps, void* stream) {
   CodedGeom g;
   if (int st = coded_check(n, downsample, object, coded_surface, transfer_2, shifts_xy, batch, workspace,
                            workspace_bytes, false, &g)) {
@@ -902,17 +1146,24 @@ int ptx_coded_forward(const float* object, const float* coded_surface, const flo
   const float2* T1 = reinterpret_cast<const float2*>(transfer_1);
   const float2* T2 = reinterpret_cast<const float2*>(transfer_2);
   const float2* M = reinterpret_cast<const float2*>(coded_surface);
-  launch_fft2<false>(g, reinterpret_cast<const float2*>(object), n, g.ospec, g.tmp, g.plan, s);
+  launch_fft2<false>(g, reinterpret_cast<const float2*>(object), n, g.ospec, g.tmp, g.plan, T1, s);
   for (int b0 = 0; b0 < batch; b0 += g.chunk) {
     const int nf = std::min(g.chunk, batch - b0);
     const float* sh = shifts_xy + 2 * (size_t)b0;
-    launch_cols<1, false>(g, nf, T1, T2, sh, s);
+    launch_cols<1, false>(g, nf, T1, T2, sh, ramps_at(ramps, b0, n), s);
     launch_rows_mask(g, nf, M, reinterpret_cast<float2*>(x_forward) + (size_t)b0 * n * n, s);
-    launch_cols<3, false>(g, nf, T1, T2, sh, s);
+    launch_cols<3, false>(g, nf, T1, T2, sh, nullptr, s);
     launch_rows_pool<kCodedForward>(g, b0, nf, nullptr, 0.f, 0.f, 0.0, nullptr, reinterpret_cast<float2*>(sensor),
                                     amplitude, nullptr, s);
   }
   return cuda_status(cudaGetLastError(), "ptx_coded_forward launch");
+}
+
+int ptx_coded_forward(const float* object, const float* coded_surface, const float* transfer_1, const float* transfer_2,
+                      int n, const float* shifts_xy, int batch, int downsample, float* x_forward, float* sensor,
+                      float* amplitude, void* workspace, size_t workspace_bytes, void* stream) {
+  return coded_forward_impl(object, coded_surface, transfer_1, transfer_2, n, shifts_xy, batch, downsample, x_forward,
+                            sensor, amplitude, workspace, workspace_bytes, nullptr, stream);
 }
 
 int ptx_coded_backward(const float* grad_output, const float* x_forward, const float* sensor, const float* amplitude,
@@ -921,7 +1172,7 @@ int ptx_coded_backward(const float* grad_output, const float* x_forward, const f
                        void* workspace, size_t workspace_bytes, void* stream) {
   return coded_backward_impl(grad_output, x_forward, sensor, amplitude, coded_surface, transfer_1, transfer_2, n,
                              shifts_xy, batch, downsample, grad_object, grad_coded, workspace, workspace_bytes, stream,
-                             nullptr, true);
+                             nullptr, nullptr, false);
 }
 
 static int coded_sweep_mse(const float* object, const float* coded_surface, const float* transfer_1,
@@ -941,25 +1192,25 @@ static int coded_sweep_mse(const float* object, const float* coded_surface, cons
   const float2* T1 = reinterpret_cast<const float2*>(transfer_1);
   const float2* T2 = reinterpret_cast<const float2*>(transfer_2);
   const float2* M = reinterpret_cast<const float2*>(coded_surface);
-  const size_t field = g.field_bytes / sizeof(float2);
-  launch_prologue(s, g.gospec, field, reinterpret_cast<float2*>(grad_coded), field, loss, nullptr, grad_shifts,
-                  grad_shifts ? 2 * (size_t)batch : 0);
+  float2* ramps = ramp_tables(n, batch, grad_object, object, coded_surface);
+  launch_coded_prologue(g, grad_coded, loss, grad_shifts, shifts_xy, ramps, s);
   const int lw = n / downsample;
   const double numel = (double)batch * lw * lw;
   const float grad_scale = static_cast<float>(2.0 / std::max(numel, 1.0));
-  launch_fft2<false>(g, reinterpret_cast<const float2*>(object), n, g.ospec, g.tmp, g.plan, s);
+  launch_fft2<false>(g, reinterpret_cast<const float2*>(object), n, g.ospec, g.tmp, g.plan, T1, s);
   for (int b0 = 0; b0 < batch; b0 += g.chunk) {
     const int nf = std::min(g.chunk, batch - b0);
     const float* sh = shifts_xy + 2 * (size_t)b0;
-    launch_cols<1, false>(g, nf, T1, T2, sh, s);
+    const float2* rp = ramps_at(ramps, b0, n);
+    launch_cols<1, false>(g, nf, T1, T2, sh, rp, s);
     launch_rows_mask(g, nf, M, g.xstore, s);
-    launch_cols<3, false>(g, nf, T1, T2, sh, s);
+    launch_cols<3, false>(g, nf, T1, T2, sh, nullptr, s);
     launch_rows_pool<kCodedSweep>(g, b0, nf, measured, scale, grad_scale, 1.0 / std::max(numel, 1.0), loss, nullptr,
                                   nullptr, nullptr, s);
-    adjoint_tail(g, nf, M, T1, T2, sh, g.xstore, reinterpret_cast<float2*>(grad_coded), s,
+    adjoint_tail(g, nf, M, T1, T2, sh, rp, g.xstore, reinterpret_cast<float2*>(grad_coded), s,
                  grad_shifts ? grad_shifts + 2 * (size_t)b0 : nullptr);
   }
-  launch_fft2<true>(g, g.gospec, n, reinterpret_cast<float2*>(grad_object), g.tmp, g.plan, s);
+  launch_fft2<true>(g, g.gospec, n, reinterpret_cast<float2*>(grad_object), g.tmp, g.plan, T1, s);
   return cuda_status(cudaGetLastError(), "ptx_coded_sweep launch");
 }
 
@@ -1022,11 +1273,10 @@ static int coded_sweep_fd(const float* object, const float* coded_surface, const
   if (int st = coded_check(n, downsample, object, coded_surface, transfer_2, shifts_xy, batch, p, inner, false, &g)) {
     return st;
   }
-  launch_prologue(s, g.gospec, g.field_bytes / sizeof(float2), reinterpret_cast<float2*>(grad_coded),
-                  g.field_bytes / sizeof(float2), loss, nullptr, grad_shifts,
-                  grad_shifts ? 2 * (size_t)batch : 0);
-  if (int st = ptx_coded_forward(object, coded_surface, transfer_1, transfer_2, n, shifts_xy, batch, downsample, xf,
-                                 sensor, amp, p, inner, stream)) {
+  float2* ramps = ramp_tables(n, batch, grad_object, object, coded_surface);
+  launch_coded_prologue(g, grad_coded, loss, grad_shifts, shifts_xy, ramps, s);
+  if (int st = coded_forward_impl(object, coded_surface, transfer_1, transfer_2, n, shifts_xy, batch, downsample, xf,
+                                  sensor, amp, p, inner, ramps, stream)) {
     return st;
   }
   const long long total = (long long)batch * h * h;
@@ -1037,7 +1287,7 @@ static int coded_sweep_fd(const float* object, const float* coded_surface, const
     prof_end(kMiscKernel, s);
   }
   return coded_backward_impl(gamp, xf, sensor, amp, coded_surface, transfer_1, transfer_2, n, shifts_xy, batch,
-                             downsample, grad_object, grad_coded, p, inner, stream, grad_shifts, false);
+                             downsample, grad_object, grad_coded, p, inner, stream, grad_shifts, ramps, true);
 }
 
 int ptx_coded_sweep_fd(const float* object, const float* coded_surface, const float* transfer_1,

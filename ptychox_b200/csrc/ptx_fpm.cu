@@ -418,7 +418,7 @@ void launch_fft2(const FpmGeom& g, const float2* in, int H, int W, float2* out, 
     // the single wave (10.8 against 11.4 us per pass with 256-thread CTAs on 128 SMs)
     const int lines = RowPass<N>::lines(128, H);
     launch_pdl(fft2_rows_kernel<N, INV>, (H + lines - 1) / lines, lines * RowPass<N>::T, RowPass<N>::smem(lines), s,
-        in, H, tmp, prow.tw, lines);
+        in, H, tmp, prow.tw, lines, nullptr);
   });
   prof_end(kFft2Rows, s);
   prof_begin(kFft2Cols, s);
@@ -426,7 +426,7 @@ void launch_fft2(const FpmGeom& g, const float2* in, int H, int W, float2* out, 
     constexpr int N = decltype(NT)::value;
     const int sm = kColsPerCta * ColPass<N>::LP * (int)sizeof(float2);
     launch_pdl(fft2_cols_kernel<N, INV>, num_tiles(W) * (kTile / kColsPerCta), ColPass<N>::kThreads, sm, s,
-        tmp, W, out, scale, pcol.tw);
+        tmp, W, out, scale, pcol.tw, nullptr);
   });
   prof_end(kFft2Cols, s);
 }

@@ -179,11 +179,12 @@ __device__ __forceinline__ void block_add_double(double v, double scale, double*
 // Generic 2-D transform passes (unnormalised; INV selects the sign)
 // ---------------------------------------------------------------------------------------
 
-// Row pass: in [H][N] natural -> row DFT -> tiled [N/16][H][16].
+// Row pass: in [H][N] natural (times conj(factor), when given) -> row DFT -> tiled [N/16][H][16].
 template <int N, bool INV>
 __global__ void __launch_bounds__(256, 2) fft2_rows_kernel(const float2* __restrict__ in, int H,
                                                             float2* __restrict__ tiled,
-                                                            const float2* __restrict__ tw, int lines) {
+                                                            const float2* __restrict__ tw, int lines,
+                                                            const float2* __restrict__ factor) {
   pdl_wait();
   using S = RegShape<N>;
   extern __shared__ float2 sm[];
@@ -195,6 +196,10 @@ __global__ void __launch_bounds__(256, 2) fft2_rows_kernel(const float2* __restr
   float2 v[S::N1];
 #pragma unroll
   for (int j = 0; j < S::N1; ++j) v[j] = row_ok ? in[(size_t)r * N + t + S::T * j] : make_float2(0.f, 0.f);
+  if (factor && row_ok) {
+#pragma unroll
+    for (int j = 0; j < S::N1; ++j) v[j] = cmulc(v[j], __ldg(&factor[(size_t)r * N + t + S::T * j]));
+  }
   reg_fft<N, INV, false>(v, sm + l * RowPass<N>::LP, t, tw);
   if (row_ok) {
 #pragma unroll
@@ -205,11 +210,13 @@ __global__ void __launch_bounds__(256, 2) fft2_rows_kernel(const float2* __restr
   }
 }
 
-// Column pass: tiled [tiles][N][16] -> column DFT -> out [N][W] natural, times `scale`.
+// Column pass: tiled [tiles][N][16] -> column DFT -> out [N][W] natural, times `scale` (and
+// `factor`, when given).
 template <int N, bool INV>
 __global__ void __launch_bounds__(256, 2) fft2_cols_kernel(const float2* __restrict__ tiled, int W,
                                                             float2* __restrict__ out, float scale,
-                                                            const float2* __restrict__ tw) {
+                                                            const float2* __restrict__ tw,
+                                                            const float2* __restrict__ factor) {
   pdl_wait();
   using S = RegShape<N>;
   extern __shared__ float2 sm[];
@@ -228,7 +235,11 @@ __global__ void __launch_bounds__(256, 2) fft2_cols_kernel(const float2* __restr
   reg_fft<N, INV, true>(v, sm + c * ColPass<N>::LP, t, tw);
   if (col_ok) {
 #pragma unroll
-    for (int m = 0; m < S::N1; ++m) out[(size_t)(t + S::T * m) * W + kc] = cscale(v[m], scale);
+    for (int m = 0; m < S::N1; ++m) {
+      const size_t at = (size_t)(t + S::T * m) * W + kc;
+      const float2 z = cscale(v[m], scale);
+      out[at] = factor ? cmul(z, __ldg(&factor[at])) : z;
+    }
   }
 }
 

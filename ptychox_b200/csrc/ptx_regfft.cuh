@@ -210,9 +210,11 @@ __device__ __forceinline__ void line_sync() {
 // exchange out with the even pitch RPV, so step 3 reads its contiguous row two elements per
 // 16-byte load (half the shared-memory load instructions); with T lanes per line the loads
 // of a warp still take the minimum number of shared-memory wavefronts.
-template <int N, bool INV, bool BLOCK, bool TW_SHARED = false>
-__device__ __forceinline__ void reg_fft(float2 (&v)[RegShape<N>::N1], float2* buf, int t,
-                                        const float2* __restrict__ tw) {
+//
+// reg_fft_with takes the barrier as a function (lines spread over a group of a block's warps).
+template <int N, bool INV, bool TW_SHARED, typename Sync>
+__device__ __forceinline__ void reg_fft_with(float2 (&v)[RegShape<N>::N1], float2* buf, int t,
+                                             const float2* __restrict__ tw, Sync&& sync) {
   using S = RegShape<N>;
   constexpr int RP = TW_SHARED ? S::RPV : S::RP;
   RegDft<S::N1, INV>::run(v);
@@ -224,7 +226,7 @@ __device__ __forceinline__ void reg_fft(float2 (&v)[RegShape<N>::N1], float2* bu
   }
 #pragma unroll
   for (int k1 = 0; k1 < S::N1; ++k1) buf[k1 * RP + t] = v[k1];
-  line_sync<BLOCK>();
+  sync();
 #pragma unroll
   for (int q = 0; q < S::C; ++q) {
     float2 u[S::T];
@@ -244,7 +246,13 @@ __device__ __forceinline__ void reg_fft(float2 (&v)[RegShape<N>::N1], float2* bu
 #pragma unroll
     for (int k2 = 0; k2 < S::T; ++k2) v[q + S::C * k2] = u[k2];
   }
-  line_sync<BLOCK>();
+  sync();
+}
+
+template <int N, bool INV, bool BLOCK, bool TW_SHARED = false>
+__device__ __forceinline__ void reg_fft(float2 (&v)[RegShape<N>::N1], float2* buf, int t,
+                                        const float2* __restrict__ tw) {
+  reg_fft_with<N, INV, TW_SHARED>(v, buf, t, tw, [] { line_sync<BLOCK>(); });
 }
 
 }  // namespace ptx
