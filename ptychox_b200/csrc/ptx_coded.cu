@@ -834,8 +834,8 @@ int coded_check(int n, int ds, const void* a, const void* b, const void* t2, con
 
 // Shift ramps of every frame, tabulated in FP64 and rounded once: ramps[f][0][k] =
 // exp(2 pi i dx_f fk), ramps[f][1][k] = exp(2 pi i dy_f fk), fk the signed frequency of bin k
-// (numpy fftfreq * n).  Part of the sweeps' first launch, which also zeroes what they accumulate
-// into.  Evaluating the two-dimensional ramp per element cost the column passes that apply it a
+// (numpy fftfreq * n, odd n too).  Part of the sweeps' first launch, which also zeroes what they
+// accumulate into.  Evaluating the two-dimensional ramp per element cost the column passes that apply it a
 // third of their instructions; the product of the two tables is also the more accurate (6e-8
 // against up to 2e-7 rad from the FP32 reduction of the summed argument).
 __global__ void __launch_bounds__(256) coded_prologue_kernel(float2* __restrict__ gospec, float2* __restrict__ grad_mask,
@@ -868,9 +868,9 @@ __global__ void __launch_bounds__(256) coded_prologue_kernel(float2* __restrict_
 
 // The ramp tables' place: grad_object, which nothing else writes before the last transform; null
 // where they do not fit (more frames than n / 2) or where the caller computes in place, and the
-// passes then evaluate the ramp themselves, as the mixed-radix ones do.
+// passes then evaluate the ramp themselves.
 float2* ramp_tables(int n, int batch, float* grad_object, const float* object, const float* coded_surface) {
-  const bool fits = is_pow2_len(n) && 2 * (long long)batch <= n && grad_object != object && grad_object != coded_surface &&
+  const bool fits = 2 * (long long)batch <= n && grad_object != object && grad_object != coded_surface &&
                     (reinterpret_cast<uintptr_t>(grad_object) & 15) == 0;
   return fits ? reinterpret_cast<float2*>(grad_object) : nullptr;
 }
@@ -906,10 +906,10 @@ void launch_fft2(const CodedGeom& g, const float2* in, int n, float2* out, float
                  const float2* t1, cudaStream_t s) {
   if (g.mix) {
     prof_begin(kFft2Rows, s);
-    g.mfft->fft2_rows(INV, in, n, tmp, p.mix_twt, s);
+    g.mfft->fft2_rows(INV, in, n, tmp, p.mix_twt, INV ? t1 : nullptr, s);
     prof_end(kFft2Rows, s);
     prof_begin(kFft2Cols, s);
-    g.mfft->fft2_cols(INV, tmp, n, out, 1.0f, p.mix_twt, s);
+    g.mfft->fft2_cols(INV, tmp, n, out, 1.0f, p.mix_twt, INV ? nullptr : t1, s);
     prof_end(kFft2Cols, s);
     return;
   }
@@ -929,15 +929,15 @@ void launch_fft2(const CodedGeom& g, const float2* in, int n, float2* out, float
 }
 
 template <int STAGE, bool CONJ>
-void launch_cols(const CodedGeom& g, int nf, const float2* t1, const float2* t2, const float* shifts,
+void launch_cols(const CodedGeom& g, int nf, const float2* t2, const float* shifts,
                  const float2* ramps, cudaStream_t s, double* grad_shifts = nullptr) {
   const float inv_n = 1.0f / static_cast<float>((double)g.n * g.n);
   prof_begin(kCodedCols, s);
   if (g.mix) {
     MixCodedArgs a = mix_args(g, nf, inv_n);
-    a.t1 = t1;
     a.t2 = t2;
     a.shifts = shifts;
+    a.ramps = ramps;
     a.grad_shifts = STAGE == 7 ? grad_shifts : nullptr;
     g.mix->cols(STAGE, CONJ, a, s);
     prof_end(kCodedCols, s);
@@ -1067,12 +1067,12 @@ void launch_rows_grad_mask(const CodedGeom& g, int nf, const float2* mask, const
 }
 
 // The adjoint passes 4 (backward part) to 7 for one chunk, given g_s already in the frames.
-void adjoint_tail(const CodedGeom& g, int nf, const float2* mask, const float2* t1, const float2* t2,
+void adjoint_tail(const CodedGeom& g, int nf, const float2* mask, const float2* t2,
                   const float* shifts, const float2* ramps, const float2* xstore, float2* grad_mask, cudaStream_t s,
                   double* grad_shifts = nullptr) {
-  launch_cols<3, true>(g, nf, t1, t2, shifts, ramps, s);
+  launch_cols<3, true>(g, nf, t2, shifts, ramps, s);
   launch_rows_grad_mask(g, nf, mask, xstore, grad_mask, s);
-  launch_cols<7, false>(g, nf, t1, t2, shifts, ramps, s, grad_shifts);
+  launch_cols<7, false>(g, nf, t2, shifts, ramps, s, grad_shifts);
 }
 
 }  // namespace
@@ -1112,7 +1112,7 @@ int coded_backward_impl(const float* grad_output, const float* x_forward, const 
     launch_rows_pool<kCodedBackward>(g, b0, nf, nullptr, 0.f, 0.f, 0.0, nullptr,
                                      const_cast<float2*>(reinterpret_cast<const float2*>(sensor)),
                                      const_cast<float*>(amplitude), grad_output, s);
-    adjoint_tail(g, nf, M, T1, T2, shifts_xy + 2 * (size_t)b0, ramps_at(ramps, b0, n),
+    adjoint_tail(g, nf, M, T2, shifts_xy + 2 * (size_t)b0, ramps_at(ramps, b0, n),
                  reinterpret_cast<const float2*>(x_forward) + (size_t)b0 * n * n,
                  reinterpret_cast<float2*>(grad_coded), s, grad_shifts ? grad_shifts + 2 * (size_t)b0 : nullptr);
   }
@@ -1150,9 +1150,9 @@ static int coded_forward_impl(const float* object, const float* coded_surface, c
   for (int b0 = 0; b0 < batch; b0 += g.chunk) {
     const int nf = std::min(g.chunk, batch - b0);
     const float* sh = shifts_xy + 2 * (size_t)b0;
-    launch_cols<1, false>(g, nf, T1, T2, sh, ramps_at(ramps, b0, n), s);
+    launch_cols<1, false>(g, nf, T2, sh, ramps_at(ramps, b0, n), s);
     launch_rows_mask(g, nf, M, reinterpret_cast<float2*>(x_forward) + (size_t)b0 * n * n, s);
-    launch_cols<3, false>(g, nf, T1, T2, sh, nullptr, s);
+    launch_cols<3, false>(g, nf, T2, sh, nullptr, s);
     launch_rows_pool<kCodedForward>(g, b0, nf, nullptr, 0.f, 0.f, 0.0, nullptr, reinterpret_cast<float2*>(sensor),
                                     amplitude, nullptr, s);
   }
@@ -1202,12 +1202,12 @@ static int coded_sweep_mse(const float* object, const float* coded_surface, cons
     const int nf = std::min(g.chunk, batch - b0);
     const float* sh = shifts_xy + 2 * (size_t)b0;
     const float2* rp = ramps_at(ramps, b0, n);
-    launch_cols<1, false>(g, nf, T1, T2, sh, rp, s);
+    launch_cols<1, false>(g, nf, T2, sh, rp, s);
     launch_rows_mask(g, nf, M, g.xstore, s);
-    launch_cols<3, false>(g, nf, T1, T2, sh, nullptr, s);
+    launch_cols<3, false>(g, nf, T2, sh, nullptr, s);
     launch_rows_pool<kCodedSweep>(g, b0, nf, measured, scale, grad_scale, 1.0 / std::max(numel, 1.0), loss, nullptr,
                                   nullptr, nullptr, s);
-    adjoint_tail(g, nf, M, T1, T2, sh, rp, g.xstore, reinterpret_cast<float2*>(grad_coded), s,
+    adjoint_tail(g, nf, M, T2, sh, rp, g.xstore, reinterpret_cast<float2*>(grad_coded), s,
                  grad_shifts ? grad_shifts + 2 * (size_t)b0 : nullptr);
   }
   launch_fft2<true>(g, g.gospec, n, reinterpret_cast<float2*>(grad_object), g.tmp, g.plan, T1, s);

@@ -404,10 +404,10 @@ void launch_fft2(const FpmGeom& g, const float2* in, int H, int W, float2* out, 
                  const LinePlan& prow, const LinePlan& pcol, cudaStream_t s) {
   if (g.generic) {
     prof_begin(kFft2Rows, s);
-    g.m_ow->fft2_rows(INV, in, H, tmp, prow.mix_twt, s);
+    g.m_ow->fft2_rows(INV, in, H, tmp, prow.mix_twt, nullptr, s);
     prof_end(kFft2Rows, s);
     prof_begin(kFft2Cols, s);
-    g.m_oh->fft2_cols(INV, tmp, W, out, scale, pcol.mix_twt, s);
+    g.m_oh->fft2_cols(INV, tmp, W, out, scale, pcol.mix_twt, nullptr, s);
     prof_end(kFft2Cols, s);
     return;
   }

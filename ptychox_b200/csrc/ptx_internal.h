@@ -234,10 +234,12 @@ struct MixFpmColsArgs {
 struct MixFpmOps {
   int (*prepare)();
   // one image: rows (natural [H][n] -> tiled [tiles(n)][H][16]) and columns (tiled
-  // [tiles(W)][n][16] -> natural [n][W] times `scale`); plus: exp(+i) (unnormalised inverse)
-  void (*fft2_rows)(bool plus, const float2* in, int H, float2* tiled, const float2* twt, cudaStream_t);
-  void (*fft2_cols)(bool plus, const float2* tiled, int W, float2* out, float scale, const float2* twt,
+  // [tiles(W)][n][16] -> natural [n][W] times `scale`); plus: exp(+i) (unnormalised inverse).
+  // factor, when given: rows take in conj(factor), columns write out factor
+  void (*fft2_rows)(bool plus, const float2* in, int H, float2* tiled, const float2* twt, const float2* factor,
                     cudaStream_t);
+  void (*fft2_cols)(bool plus, const float2* tiled, int W, float2* out, float scale, const float2* twt,
+                    const float2* factor, cudaStream_t);
   void (*rows_forward)(const MixFpmRowsArgs&, cudaStream_t);
   void (*rows_adjoint)(const MixFpmRowsArgs&, cudaStream_t);
   void (*cols)(int mode, const MixFpmColsArgs&, cudaStream_t);
@@ -249,10 +251,10 @@ const MixFpmOps* mix_fpm_ops(int n);
 // null for every other side).
 struct MixCodedArgs {
   float2* scratch;          // tiled frames [frame][tile][row][16], n x n
-  const float2* ospec;      // O^ = fft2(O)
-  const float2* t1;         // first transfer function (null: near-field)
+  const float2* ospec;      // O^ T1 = fft2(O) T1 (near-field: fft2(O))
   const float2* t2;
   const float* shifts;      // (dx, dy) per frame of this chunk
+  const float2* ramps;      // their ramps [frame][x, y][n], or null (evaluated)
   float inv_n;              // 1 / n^2
   float2* grad_ospec;
   const float2* twt;        // line twiddles of n (LinePlan::mix_twt / mix_twi)

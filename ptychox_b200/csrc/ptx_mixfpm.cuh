@@ -43,11 +43,13 @@ __device__ __forceinline__ int pymod(long long v, int n) {
   return static_cast<int>(r < 0 ? r + n : r);
 }
 
-// ---- 2-D transform of one image: rows (natural [H][N] -> tiled [tiles(N)][H][16]) --------
+// ---- 2-D transform of one image: rows (natural [H][N], times conj(factor) when given -> tiled
+// [tiles(N)][H][16]) ------------------------------------------------------------------------
 template <int N, bool PLUS>
 __global__ void __launch_bounds__(RowCfg<N>::THREADS) mix_fft2_rows(const float2* __restrict__ in, int H,
                                                                      float2* __restrict__ tiled,
-                                                                     const float2* __restrict__ twt, int lines) {
+                                                                     const float2* __restrict__ twt, int lines,
+                                                                     const float2* __restrict__ factor) {
   pdl_wait();
   using Cfg = RowCfg<N>;
   constexpr int A = Cfg::A, B = Cfg::B;
@@ -60,6 +62,10 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS) mix_fft2_rows(const float2
   float2 y[A];
 #pragma unroll
   for (int j = 0; j < A; ++j) y[j] = row_ok ? in[(size_t)r * N + t + B * j] : make_float2(0.f, 0.f);
+  if (factor && row_ok) {
+#pragma unroll
+    for (int j = 0; j < A; ++j) y[j] = cmulc(y[j], __ldg(&factor[(size_t)r * N + t + B * j]));
+  }
   float2* buf = sm + l * Cfg::BUF;
   mix::fwd_step1<N, Cfg::P, 1, PLUS>(y, buf, t, twt);
   __syncthreads();
@@ -74,11 +80,12 @@ __global__ void __launch_bounds__(RowCfg<N>::THREADS) mix_fft2_rows(const float2
   }
 }
 
-// ---- columns (tiled [tiles(W)][N][16] -> natural out [N][W], times `scale`) ---------------
+// ---- columns (tiled [tiles(W)][N][16] -> natural out [N][W], times `scale` and `factor`) -----
 template <int N, bool PLUS>
 __global__ void __launch_bounds__(ColCfg<N>::THREADS) mix_fft2_cols(const float2* __restrict__ tiled, int W,
                                                                      float2* __restrict__ out, float scale,
-                                                                     const float2* __restrict__ twt) {
+                                                                     const float2* __restrict__ twt,
+                                                                     const float2* __restrict__ factor) {
   pdl_wait();
   using Cfg = ColCfg<N>;
   constexpr int A = Cfg::A, B = Cfg::B, C = Cfg::C;
@@ -101,7 +108,11 @@ __global__ void __launch_bounds__(ColCfg<N>::THREADS) mix_fft2_cols(const float2
     float2 z[B];
     mix::fwd_step2<N, Cfg::RS, C, PLUS>(z, sm + c, t);
 #pragma unroll
-    for (int k = 0; k < B; ++k) out[(size_t)(t + A * k) * W + kc] = cscale(z[k], scale);
+    for (int k = 0; k < B; ++k) {
+      const size_t at = (size_t)(t + A * k) * W + kc;
+      const float2 v = cscale(z[k], scale);
+      out[at] = factor ? cmul(v, __ldg(&factor[at])) : v;
+    }
   }
 }
 
@@ -368,24 +379,27 @@ struct Ops {
     if (!st) st = ensure_smem((const void*)mix_fpm_cols<kMixColBackward, N>, CC::SMEM);
     return st;
   }
-  static void fft2_rows(bool plus, const float2* in, int H, float2* tiled, const float2* twt, cudaStream_t s) {
+  static void fft2_rows(bool plus, const float2* in, int H, float2* tiled, const float2* twt, const float2* factor,
+                        cudaStream_t s) {
     if (H <= 0) return;
     const int lines = std::min(RC::LINES, H);
     const int grid = (H + lines - 1) / lines;
     if (plus) {
-      launch_pdl(mix_fft2_rows<N, true>, grid, lines * RC::B, RC::smem_forward(lines), s, in, H, tiled, twt, lines);
+      launch_pdl(mix_fft2_rows<N, true>, grid, lines * RC::B, RC::smem_forward(lines), s, in, H, tiled, twt, lines,
+                 factor);
     } else {
-      launch_pdl(mix_fft2_rows<N, false>, grid, lines * RC::B, RC::smem_forward(lines), s, in, H, tiled, twt, lines);
+      launch_pdl(mix_fft2_rows<N, false>, grid, lines * RC::B, RC::smem_forward(lines), s, in, H, tiled, twt, lines,
+                 factor);
     }
   }
   static void fft2_cols(bool plus, const float2* tiled, int W, float2* out, float scale, const float2* twt,
-                        cudaStream_t s) {
+                        const float2* factor, cudaStream_t s) {
     if (W <= 0) return;
     const int grid = num_tiles(W) * (kTile / CC::C);
     if (plus) {
-      launch_pdl(mix_fft2_cols<N, true>, grid, CC::THREADS, CC::SMEM, s, tiled, W, out, scale, twt);
+      launch_pdl(mix_fft2_cols<N, true>, grid, CC::THREADS, CC::SMEM, s, tiled, W, out, scale, twt, factor);
     } else {
-      launch_pdl(mix_fft2_cols<N, false>, grid, CC::THREADS, CC::SMEM, s, tiled, W, out, scale, twt);
+      launch_pdl(mix_fft2_cols<N, false>, grid, CC::THREADS, CC::SMEM, s, tiled, W, out, scale, twt, factor);
     }
   }
   static void rows_forward(const MixFpmRowsArgs& a, cudaStream_t s) {

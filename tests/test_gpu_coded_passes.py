@@ -86,3 +86,55 @@ def test_gradient_in_place_of_the_object():
     call_on(dev, "ptx_coded_sweep", ptr(obj), ptr(m), ptr(a), ptr(b), 64, ptr(sh), 4, 2, ptr(y), scale, ptr(loss),
             ptr(obj), ptr(gm), ptr(ws), ws.numel())
     check((loss, obj, gm), args, 2)
+
+
+@pytest.mark.parametrize("n, ds, count", [
+    (18, 3, 9),     # fewer columns than three strips, the last one partial
+    (25, 5, 12),    # odd: rows off 16 bytes, as many frames as the ramp tables hold
+    (25, 1, 13),    # and one more
+    (27, 27, 3),    # one pooled row
+    (45, 3, 2),
+    (75, 15, 4),    # row groups that end past the last row
+    (100, 2, 5),
+    (243, 9, 2),
+    (625, 1, 1),    # 25 x 25
+    (972, 6, 1),
+    (1000, 8, 2),
+])
+@pytest.mark.parametrize("nearfield", [False, True])
+def test_mixed_radix_edges(n, ds, count, nearfield):
+    from ptychox_b200.coded import coded_sweep
+
+    args = problem(n, count, ds, nearfield)
+    guess, mask, t1, t2, shifts, meas, scale = args
+    got = coded_sweep(cuda(guess), cuda(mask), cuda(t1, 1), cuda(t2, 1), cuda(shifts), ds, cuda(meas), scale,
+                      with_shifts=True)
+    check(got, args, ds)
+
+
+@pytest.mark.parametrize("n, ds", [(60, 4), (45, 3)])
+def test_mixed_radix_backward_of_unaligned_buffers(n, ds):
+    """The adjoint on a sensor field that starts 8 bytes off a 16-byte boundary; x there is refused."""
+    from ptychox_b200 import _abi
+    from ptychox_b200._utils import call_on, ptr, workspace
+
+    count = 3
+    guess, mask, t1, t2, shifts, _, _ = problem(n, count, ds, False)
+    _, xf, sensor, amp = O.coded_forward(guess, mask, t1, t2, shifts, ds)
+    gout = np.random.default_rng(n).standard_normal(amp.shape).astype(np.float32)
+    want = O.coded_backward(gout, xf, sensor, amp, mask, t1, t2, shifts, ds)
+    dev = torch.device("cuda", torch.cuda.current_device())
+    g, a, m, x1, x2, sh = (cuda(v) for v in (gout, amp.astype(np.float32), mask, t1, t2, shifts))
+    off, xc, sc = (cuda(v.astype(np.complex64), o) for v, o in ((xf, 1), (xf, 0), (sensor, 1)))
+    go, gm = torch.empty_like(m), torch.empty_like(m)
+    ws = workspace(_abi.query("ptx_coded_workspace_bytes", n, count), dev)
+
+    def backward(x):
+        call_on(dev, "ptx_coded_backward", ptr(g), ptr(x), ptr(sc), ptr(a), ptr(m), ptr(x1), ptr(x2), n, ptr(sh), count,
+                ds, ptr(go), ptr(gm), ptr(ws), ws.numel())
+
+    with pytest.raises(ValueError):
+        backward(off)
+    backward(xc)
+    for got, ref in zip((go, gm), want):
+        assert rel_l2(got.cpu().numpy(), ref) < 1e-5
