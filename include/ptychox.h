@@ -486,6 +486,19 @@ size_t ptx_reg_estimate_workspace_bytes(int batch, int rows, int cols);
 int ptx_reg_estimate(const float* correlation, int batch, int rows, int cols, int usfac, int* half_rc,
                      int* row_center, int* col_center, double* peak_cc, void* workspace, size_t workspace_bytes,
                      void* stream);
+/* Transforms of image sides R p, p a prime of 37 to 127 and R in {2..6, 8, 9, 10, 12} (both sides;
+ * 472 = 8 * 59 is a 512-pixel crop less its border).
+ *   ptx_reg_prime_fft_workspace_bytes  of either call, 0 for other sides
+ *   ptx_reg_prime_fft2          real images (element (b, r, c) at b * image_stride + r * row_stride
+ *                               + c) -> their spectra `out` [batch][rows][cols] complex; `half` is
+ *                               scratch of the same size
+ *   ptx_reg_prime_correlation   `cross_power` -> `correlation` of ptx_reg_estimate (padding
+ *                               included); `half` is scratch of [batch][2 cols][rows] complex */
+size_t ptx_reg_prime_fft_workspace_bytes(int rows, int cols);
+int ptx_reg_prime_fft2(const float* images, long long image_stride, long long row_stride, int batch, int rows,
+                       int cols, float* half, float* out, void* workspace, size_t workspace_bytes, void* stream);
+int ptx_reg_prime_correlation(const float* cross_power, int batch, int rows, int cols, float* half,
+                              float* correlation, void* workspace, size_t workspace_bytes, void* stream);
 int ptx_reg_energy(const float* spec, int batch, int rows, int cols, double* energy, void* stream);
 
 #ifdef __cplusplus

@@ -86,6 +86,9 @@ SIGNATURES: dict[str, tuple] = {
     "ptx_reg_pad_transpose": (_i, [_p, _i, _i, _i, _p, _p]),
     "ptx_reg_estimate_workspace_bytes": (_sz, [_i, _i, _i]),
     "ptx_reg_estimate": (_i, [_p, _i, _i, _i, _i, _p, _p, _p, _p, _p, _sz, _p]),
+    "ptx_reg_prime_fft_workspace_bytes": (_sz, [_i, _i]),
+    "ptx_reg_prime_fft2": (_i, [_p, C.c_longlong, C.c_longlong, _i, _i, _i, _p, _p, _p, _sz, _p]),
+    "ptx_reg_prime_correlation": (_i, [_p, _i, _i, _i, _p, _p, _p, _sz, _p]),
     "ptx_reg_energy": (_i, [_p, _i, _i, _i, _p, _p]),
     "ptx_server_create": (_i, [_i, _sz, _i, _p]),
     "ptx_server_submit": (_i, [_p, _p, _p]),

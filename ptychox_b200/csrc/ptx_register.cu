@@ -405,7 +405,7 @@ __device__ __forceinline__ int unpadded_bin(int c, int n) {
 }
 
 // One pass from the two spectra to the product spec1 conj(spec2), rows zero-padded to 2 cols
-// (what the row transform reads), and the cross-power conj(spec1) spec2 the refinement reads.
+// (what a library's row transform reads; null where the padding is the transform's own), and the cross-power conj(spec1) spec2 the refinement reads.
 // HBM-bound: 8 B read (spec1 of a tracked stack is one image, resident in L2), 24 B written.
 __global__ void __launch_bounds__(256) reg_cross_power_kernel(const float2* __restrict__ s1, bool one,
                                                               const float2* __restrict__ s2, int rows, int cols,
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(256) reg_cross_power_kernel(const float2* __re
       q[row * cols + k] = z;
       v = cconj(z);
     }
-    padded[row * 2 * cols + c] = v;
+    if (padded) padded[row * 2 * cols + c] = v;
   }
 }
 
@@ -658,7 +658,7 @@ int ptx_reg_cross_power(const float* spec1, int batch1, const float* spec2, int 
   if (int st = reg_check_stack(batch, rows, cols)) return st;
   if (batch1 != 1 && batch1 != batch) return set_error(PTX_ERR_INVALID_ARGUMENT, "spec1 holds 1 or %d images", batch);
   if (batch == 0) return PTX_OK;
-  if (!spec1 || !spec2 || !padded || !cross_power) return set_error(PTX_ERR_INVALID_ARGUMENT, "null pointer argument");
+  if (!spec1 || !spec2 || !cross_power) return set_error(PTX_ERR_INVALID_ARGUMENT, "null pointer argument");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   prof_begin(kMiscKernel, s);
   const size_t image = (size_t)rows * cols;
@@ -666,7 +666,8 @@ int ptx_reg_cross_power(const float* spec1, int batch1, const float* spec2, int 
     reg_cross_power_kernel<<<dim3(rows, nb), 256, 0, s>>>(
         reinterpret_cast<const float2*>(spec1) + (batch1 == 1 ? 0 : b0 * image), batch1 == 1,
         reinterpret_cast<const float2*>(spec2) + b0 * image, rows, cols,
-        reinterpret_cast<float2*>(padded) + 2 * b0 * image, reinterpret_cast<float2*>(cross_power) + b0 * image);
+        padded ? reinterpret_cast<float2*>(padded) + 2 * b0 * image : nullptr,
+        reinterpret_cast<float2*>(cross_power) + b0 * image);
   });
   prof_end(kMiscKernel, s);
   return cuda_status(cudaGetLastError(), "ptx_reg_cross_power launch");
