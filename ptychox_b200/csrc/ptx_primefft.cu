@@ -16,10 +16,11 @@
 // 128 bytes) at a time, so that the second dimension is again contiguous and nothing is
 // transposed in a pass of its own.
 //
-// Bound: FP32 issue and shared memory about equally in the product (57 FMA a point), and the loads of
-// step 1, which nothing hides but the other CTA of the SM; HBM alone would take a third of the time.
-// 200 images of 472^2 (us; cuFFT with its padding and transposing passes before): their spectra
-// 1420 -> 390 (first pass 158, second 230), the correlation on 944^2 2900 -> 1720 (551 and 1165).
+// Bound: FP32 issue and shared memory about equally in the product (57 FMA a point), and step 1, whose
+// loads only the other CTA of the SM hides where they are not staged; HBM alone would take a third
+// of the time.  200 images of 472^2 (us; cuFFT with its padding and transposing passes before): their
+// spectra 1420 -> 570 (first pass 230, second 340), the correlation on 944^2 2900 -> 1410 (494 and
+// 918; 551 and 1165 with loads on demand).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -36,6 +37,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kColumns = 128;  // columns (line, k1) of a CTA
 constexpr int kOut = 8;        // outputs k2 of a warp's step
+constexpr int kStagedSmem = 113 << 10;  // lines are staged where two CTAs still fit an SM
 
 int padded_outputs(int p) { return ((p - 1) / 2 + 1 + kOut - 1) / kOut * kOut; }
 
@@ -91,10 +93,11 @@ struct PrimeArgs {
   float2* out;
 };
 
-// R-point stride of the input: PAD = false: element n of the line; PAD = true: the line holds
+// STAGE: a unit's lines (one contiguous block) land in shared memory by cp.async while the previous
+// unit's product runs.  PAD = false: element n of the line; PAD = true: the line holds
 // R p / 2 bins, zero-padded to twice as many around the highest frequency (FTpad,
 // dftregistration.m:189-224).
-template <int R, bool PLUS, bool PAD, bool REAL, bool TRANSPOSE>
+template <int R, bool PLUS, bool PAD, bool REAL, bool TRANSPOSE, bool STAGE>
 __global__ void __launch_bounds__(kThreads, R <= 16 ? 2 : 1) prime_lines_kernel(PrimeArgs a) {
   constexpr int LINES = kColumns / R, COLS = LINES * R;
   constexpr int PITCH = kColumns + 1;  // float4 of a row j: consecutive j fall in consecutive banks
@@ -104,12 +107,25 @@ __global__ void __launch_bounds__(kThreads, R <= 16 ? 2 : 1) prime_lines_kernel(
   float2* coef = reinterpret_cast<float2*>(sd + (size_t)h * PITCH);
   float2* y0 = coef + (size_t)h * kpad;
   const float2* tw = a.tables;
+  float2* raw = coef + (size_t)h * kpad + kColumns;  // STAGE: [LINES][valid]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int i = tid; i < h * kpad; i += kThreads) coef[i] = __ldg(a.tables + n + i);
   const int per_image = (a.lines + LINES - 1) / LINES;
   const long long units = (long long)per_image * a.images;
   const int valid = PAD ? n / 2 : n, low = valid - valid / 2;
+  auto request = [&](long long u) {
+    const long long image = u / per_image, line0 = (u - image * per_image) * LINES;
+    const float2* src = a.in + (image * a.lines + line0) * valid;
+    const int count = static_cast<int>(min((long long)LINES, a.lines - line0)) * valid;
+    for (int i = tid; i < count; i += kThreads) cp_async8(raw + i, src + i);
+    cp_async_commit();
+  };
+  if (STAGE && blockIdx.x < units) request(blockIdx.x);
   for (long long u = blockIdx.x; u < units; u += gridDim.x) {
+    if (STAGE) {
+      cp_async_wait_all();
+      __syncthreads();
+    }
     const int image = static_cast<int>(u / per_image);
     const int line0 = static_cast<int>(u - (long long)image * per_image) * LINES;
     // step 1: item (line, j) takes the elements j and p - j of every stretch of p
@@ -123,7 +139,7 @@ __global__ void __launch_bounds__(kThreads, R <= 16 ? 2 : 1) prime_lines_kernel(
         if constexpr (REAL) {
           return make_float2(__ldg(a.real + image * a.real_image + line * a.real_line + at), 0.f);
         } else {
-          const float2 v = __ldg(a.in + ((size_t)image * a.lines + line) * valid + at);
+          const float2 v = STAGE ? raw[l * valid + at] : __ldg(a.in + ((size_t)image * a.lines + line) * valid + at);
           return make_float2(v.x, a.sign * v.y);
         }
       };
@@ -150,6 +166,7 @@ __global__ void __launch_bounds__(kThreads, R <= 16 ? 2 : 1) prime_lines_kernel(
       }
     }
     __syncthreads();
+    if (STAGE && u + gridDim.x < units) request(u + gridDim.x);
     // step 2: kOut outputs of 64 columns per warp
     const int tiles = kpad / kOut;
     for (int task = warp; task < 2 * tiles; task += kThreads / 32) {
@@ -207,12 +224,15 @@ __global__ void __launch_bounds__(kThreads, R <= 16 ? 2 : 1) prime_lines_kernel(
   }
 }
 
-template <int R, bool PLUS, bool PAD, bool REAL, bool TRANSPOSE>
+template <int R, bool PLUS, bool PAD, bool REAL, bool TRANSPOSE, bool STAGE = PAD>
 int launch_lines(const PrimeArgs& a, cudaStream_t s) {
   constexpr int LINES = kColumns / R;
-  auto kern = prime_lines_kernel<R, PLUS, PAD, REAL, TRANSPOSE>;
+  auto kern = prime_lines_kernel<R, PLUS, PAD, REAL, TRANSPOSE, STAGE>;
   const int h = (a.p - 1) / 2, kpad = padded_outputs(a.p);
-  const int smem = h * (kColumns + 1) * (int)sizeof(float4) + (h * kpad + kColumns) * (int)sizeof(float2);
+  const int smem = h * (kColumns + 1) * (int)sizeof(float4) + (h * kpad + kColumns + (STAGE ? LINES * R * a.p / 2 : 0)) * (int)sizeof(float2);
+  if constexpr (STAGE) {
+    if (smem > kStagedSmem) return launch_lines<R, PLUS, PAD, REAL, TRANSPOSE, false>(a, s);
+  }
   if (int st = ensure_smem((const void*)kern, smem)) return st;
   const long long units = (long long)((a.lines + LINES - 1) / LINES) * a.images;
   const int grid = persistent_grid((const void*)kern, kThreads, smem, units);
