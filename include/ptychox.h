@@ -162,7 +162,7 @@ int ptx_base_sweep(const float* sample, int sample_h, int sample_w,
  * otherwise), same arguments and results: one CTA runs the whole sweep of a frame in shared
  * memory (gather, row and column DFTs with the loss epilogue, inverse DFTs, gradient
  * scatter), so a sweep is the prologue and one launch, with no scratch frames in HBM (the
- * workspace still holds the count-decode table and the error word).  The Python operators
+ * workspace still holds the error word).  The Python operators
  * use it for such probes. */
 int ptx_base_sweep_small(const float* sample, int sample_h, int sample_w,
                          const float* probe, int probe_h, int probe_w,
@@ -373,7 +373,7 @@ int ptx_adam_step(float* param, const float* grad, float* exp_avg, float* exp_av
  * Same arguments and results as ptx_base_sweep minus the workspace: the scratch frames
  * live in a fixed PTX_NOALLOC_SCRATCH_BYTES device array that every GPU loading the
  * library holds until exit.  ptx_base_workspace_bytes(probe_h, probe_w, 1) (one frame of
- * ph x pw rounded up to 16 columns, 8 bytes each, plus a 256 KiB table and 256 bytes)
+ * ph x pw rounded up to 16 columns, 8 bytes each, plus 256 KiB reserved and 256 bytes)
  * must fit in it, else PTX_ERR_WORKSPACE.  The first call on a device looks up the
  * array's device address (make it before any CUDA graph capture).  All calls share the
  * array: calls that overlap on the GPU race and must be serialised by the caller. */
@@ -470,7 +470,7 @@ int ptx_reg_upsampled_peak(const float* cross_power, int batch, int rows, int co
  * the cross-correlation upsampled twice.  Images are [batch][rows][cols] complex64 spectra.
  *   ptx_reg_cross_power    spec1 (batch1 = 1 or batch images) and spec2 -> `padded`
  *                          [batch][rows][2 cols], spec1 .* conj(spec2) with each row zero-padded
- *                          (FTpad, :189-224), and `cross_power` [batch][rows][cols], its conjugate
+ *                          (FTpad, :189-224; may be null), and `cross_power` [batch][rows][cols], its conjugate
  *   ptx_reg_pad_transpose  [batch][rows][2 cols] -> [batch][2 cols][2 rows], transposed and
  *                          zero-padded along the rows
  *   ptx_reg_estimate       `correlation` [batch][2 cols][2 rows] (unnormalised inverse transform
