@@ -19,8 +19,9 @@
 // Bound: FP32 issue and shared memory about equally in the product (57 FMA a point), and step 1, whose
 // loads only the other CTA of the SM hides where they are not staged; HBM alone would take a third
 // of the time.  200 images of 472^2 (us; cuFFT with its padding and transposing passes before): their
-// spectra 1420 -> 570 (first pass 230, second 340), the correlation on 944^2 2900 -> 1410 (494 and
-// 918; 551 and 1165 with loads on demand).
+// spectra 1420 -> 470 (first pass 232, second 240), the correlation on 944^2 2900 -> 1260 (431 and
+// 828; 551 and 1165 with loads on demand and the padding tested element by element).  At 60 images
+// 70 to 73% of the issue slots and half of the FMA pipe are busy.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -131,24 +132,30 @@ __global__ void __launch_bounds__(kThreads, R <= 16 ? 2 : 1) prime_lines_kernel(
     // step 1: item (line, j) takes the elements j and p - j of every stretch of p
     for (int item = tid; item < LINES * (h + 1); item += kThreads) {
       const int l = item / (h + 1), j = item - l * (h + 1);
-      const int line = line0 + l;
-      auto element = [&](int i) {
-        int at = i;
-        if (PAD) at = i < low ? i : (i >= low + valid ? i - valid : -1);
-        if (line >= a.lines || at < 0) return make_float2(0.f, 0.f);
-        if constexpr (REAL) {
-          return make_float2(__ldg(a.real + image * a.real_image + line * a.real_line + at), 0.f);
+      const int line = min(line0 + l, a.lines - 1);  // columns past the last line are not stored
+      const float* real = REAL ? a.real + image * a.real_image + line * a.real_line : nullptr;
+      const float2* src = STAGE ? raw + (line - line0) * valid : a.in + ((size_t)image * a.lines + line) * valid;
+      auto load = [&](int at) {
+        if constexpr (REAL) return make_float2(__ldg(real + at), 0.f);
+        const float2 v = STAGE ? src[at] : __ldg(src + at);
+        return make_float2(v.x, a.sign * v.y);
+      };
+      auto element = [&](int i, int j) {  // element p i + j of the (padded) line
+        const int at = p * i + j;
+        if constexpr (!PAD) {
+          return load(at);
+        } else if constexpr (R % 4 == 0) {  // the padding is whole stretches of p
+          return i < R / 4 ? load(at) : i >= 3 * R / 4 ? load(at - valid) : make_float2(0.f, 0.f);
         } else {
-          const float2 v = STAGE ? raw[l * valid + at] : __ldg(a.in + ((size_t)image * a.lines + line) * valid + at);
-          return make_float2(v.x, a.sign * v.y);
+          return at < low ? load(at) : at >= low + valid ? load(at - valid) : make_float2(0.f, 0.f);
         }
       };
       float2 ya[R], yb[R];
       const int jb = j ? p - j : 0;
 #pragma unroll
       for (int i = 0; i < R; ++i) {
-        ya[i] = element(p * i + j);
-        yb[i] = element(p * i + jb);
+        ya[i] = element(i, j);
+        yb[i] = element(i, jb);
       }
       mix::Dft<R, PLUS>::run(ya);
       mix::Dft<R, PLUS>::run(yb);
