@@ -460,7 +460,9 @@ __device__ __forceinline__ constexpr int pipe_index(int m) {
   return (m % RegShape<N>::C) * RegShape<N>::T + m / RegShape<N>::C;
 }
 
-// Whole tiles only (`width` a multiple of 2 kTile) and counts on a 16-byte boundary.
+// Whole tiles only (`width` a multiple of 2 kTile) and counts on a 16-byte boundary.  Bound: the
+// latency of the exchanges and the epilogue at 8 to 16 warps per SM (900 frames of 512^2: 1023 us,
+// of cols_sweep_pair 1135; 825 without the DFT arithmetic, 780 with the frames in L2 as well).
 template <int N, bool FIRST_INV, bool SHIFTED, bool UNIT_NORM>
 __global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlocks) cols_sweep_pipe(
     float2* __restrict__ scratch, int width, int nframes, int frame0, const float2* __restrict__ tw,
@@ -569,7 +571,9 @@ __global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlo
 }
 
 // Column lengths the pipeline is used for, and the frames it takes: whole pairs of tiles (the
-// counts' 16-byte pieces stay inside a tile), counts on a 16-byte boundary.
+// counts' 16-byte pieces stay inside a tile), counts on a 16-byte boundary.  At 512 points a CTA of
+// cols_sweep_pair leaves no room for the next tile's loads beside it (1135 us against 1023 here);
+// at 256 several of its CTAs share an SM and it is the faster one (225 frames: 60.5 us against 69.8).
 template <int N>
 constexpr bool col_pipe_length() {
   return N == 512;
