@@ -98,6 +98,11 @@ def _half_pixel_estimate(b1: torch.Tensor, b2: torch.Tensor, usfac: int):
     return half, centre, value, q
 
 
+def _in_memory(t: torch.Tensor) -> torch.Tensor:
+    """``t`` contiguous with a lazy conjugation or negation carried out: a pointer sees neither."""
+    return t.contiguous().resolve_conj().resolve_neg()
+
+
 def _plain(t: torch.Tensor) -> bool:
     """Whether the library may read ``t`` directly: it has storage of its own (not a batched
     tensor of vmap) and carries no derivative."""
@@ -158,7 +163,7 @@ def dftregistration(buf1ft: torch.Tensor, buf2ft: torch.Tensor, usfac: int = 1, 
     b1 = buf1ft.to(torch.complex64).reshape(-1, *buf1ft.shape[-2:])
     b2 = buf2ft.to(torch.complex64).reshape(-1, *buf2ft.shape[-2:])
     bsz = max(b1.shape[0], b2.shape[0])
-    b1, b2 = b1.expand(min(bsz, b1.shape[0]), -1, -1).contiguous(), b2.expand(bsz, -1, -1).contiguous()
+    b1, b2 = _in_memory(b1.expand(min(bsz, b1.shape[0]), -1, -1)), _in_memory(b2.expand(bsz, -1, -1))
     if b1.shape[0] not in (1, bsz):
         b1 = b1.expand(bsz, -1, -1)  # raises: the two batches differ
     nr, nc = b2.shape[-2:]

@@ -1,0 +1,30 @@
+"""Registration of spectra and images in the forms torch hands them out."""
+
+import pytest
+import torch
+
+
+def spectra(count, h, w, seed=0):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    base = torch.randn(h, w, generator=gen, device="cuda")
+    shifted = [torch.roll(base, (3 * i, -2 * i), dims=(0, 1)) for i in range(count)]
+    noise = 0.1 * torch.randn(count, h, w, generator=gen, device="cuda")
+    return torch.fft.fft2(torch.stack(shifted) + noise)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("usfac", [0, 1, 2, 3, 100])
+@pytest.mark.parametrize("sides", [(48, 40), (33, 51)])
+@pytest.mark.parametrize("first, second", [(True, False), (False, True), (True, True)])
+def test_conjugate_views(usfac, sides, first, second):
+    """A lazily conjugated spectrum is the conjugate in memory: the same numbers, to the bit."""
+    from ptychox_b200.registration import dftregistration
+
+    s = spectra(5, *sides)
+    a, b = s[0], s
+    lazy = a.conj() if first else a, b.conj() if second else b
+    assert lazy[0].is_conj() == first and lazy[1].is_conj() == second
+    got = dftregistration(*lazy, usfac, return_registered=True)
+    want = dftregistration(lazy[0].resolve_conj(), lazy[1].resolve_conj(), usfac, return_registered=True)
+    for g, w in zip(got, want):
+        assert torch.equal(g, w)
