@@ -220,7 +220,7 @@ def _spectra(images: torch.Tensor) -> torch.Tensor:
     own = _prime_fft_bytes(images.numel() // max(1, h * w), h, w)
     if not own or images.dtype != torch.float32 or not _plain(images):
         return torch.fft.fft2(images.to(torch.complex64))
-    x = images.reshape(-1, h, w)
+    x = images.reshape(-1, h, w).resolve_neg()
     if x.stride(2) != 1:
         x = x.contiguous()
     half = torch.empty(x.shape[0], w, h, dtype=torch.complex64, device=x.device)

@@ -28,3 +28,24 @@ def test_conjugate_views(usfac, sides, first, second):
     want = dftregistration(lazy[0].resolve_conj(), lazy[1].resolve_conj(), usfac, return_registered=True)
     for g, w in zip(got, want):
         assert torch.equal(g, w)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("view", ["negated", "imaginary"])
+def test_negated_images(view):
+    """A stack with the negative bit set, at a side of the library's own transforms and enough pixels
+    for them: the positions of the same images in memory."""
+    from ptychox_b200.registration import _prime_fft_bytes, track_position
+
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    base = torch.rand(158, 158, generator=gen, device="cuda")
+    images = torch.stack([torch.roll(base, (i % 7, -(i % 5)), dims=(0, 1)) for i in range(48)])
+    assert _prime_fft_bytes(48, 118, 118) > 0
+    if view == "negated":
+        stack = torch._neg_view((-images).contiguous())
+    else:
+        stack = torch.imag(torch.complex(torch.zeros_like(images), -images).conj())
+    assert stack.is_neg()
+    for g, w in zip(track_position(stack, usfac=10, return_registered=True),
+                    track_position(images, usfac=10, return_registered=True)):
+        assert torch.equal(g, w)
