@@ -156,6 +156,8 @@ def dftregistration(buf1ft: torch.Tensor, buf2ft: torch.Tensor, usfac: int = 1, 
         raise ValueError("buf1ft and buf2ft must be CUDA tensors (ptychox_b200 has no CPU path).")
     if buf1ft.shape[-2:] != buf2ft.shape[-2:]:
         raise ValueError("buf1ft and buf2ft must have the same image size.")
+    if buf1ft.device != buf2ft.device:
+        raise ValueError("buf1ft and buf2ft must live on the same device.")
     usfac = int(usfac)
     if usfac < 0:
         raise ValueError("usfac must be non-negative.")

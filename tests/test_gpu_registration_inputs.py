@@ -1,4 +1,6 @@
-"""Registration of spectra and images in the forms torch hands them out."""
+"""Registration of spectra and images in the forms torch hands them out, and on two devices."""
+
+from types import SimpleNamespace
 
 import pytest
 import torch
@@ -49,3 +51,14 @@ def test_negated_images(view):
     for g, w in zip(track_position(stack, usfac=10, return_registered=True),
                     track_position(images, usfac=10, return_registered=True)):
         assert torch.equal(g, w)
+
+
+def test_spectra_on_two_devices_are_refused():
+    """Before anything is launched: the stand-ins hold nothing that a later step could use."""
+    from ptychox_b200.registration import dftregistration
+
+    a, b = (SimpleNamespace(ndim=2, is_cuda=True, shape=torch.Size((8, 8)), device=torch.device("cuda", i))
+            for i in range(2))
+    for usfac in (0, 1, 2, 100):
+        with pytest.raises(ValueError, match="same device"):
+            dftregistration(a, b, usfac)
