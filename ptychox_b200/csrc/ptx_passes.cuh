@@ -10,6 +10,7 @@
 
 #include "ptx_internal.h"
 #include "ptx_pairfft.cuh"
+#include "ptx_pipering.h"
 #include "ptx_regfft.cuh"
 
 namespace ptx {
@@ -410,11 +411,11 @@ template <int N>
 struct ColPipeCfg {
   static constexpr int kPairs = kTile / 2;
   static constexpr int kGroup = kPairs * RegShape<N>::T;  // threads per tile
-  static constexpr int kBufs = 3;
+  static constexpr int kBufs = PipeRing::kBufs;
   static constexpr int kTileBytes = N * kTile * (int)sizeof(float2);
   static constexpr int kMeasBytes = N * kTile * (int)sizeof(uint16_t);
   static constexpr int kTwBytes = N / 2 * (int)sizeof(float2);
-  static constexpr int kSmemBytes = kBufs * kTileBytes + 2 * kMeasBytes + kTwBytes + 64;
+  static constexpr int kSmemBytes = kBufs * kTileBytes + 2 * kMeasBytes + kTwBytes + PipeRing::kBars * (int)sizeof(uint64_t);
   static constexpr int kBlocks = N <= 256 ? 2 : 1;  // CTAs per SM
 };
 
@@ -480,7 +481,7 @@ __global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlo
   uint64_t* full = reinterpret_cast<uint64_t*>(tws + N / 2);
   for (int i = tid; i < N / 2; i += blockDim.x) tws[i] = __ldg(&tw[i]);
   if (tid == 0) {
-    for (int b = 0; b < Cfg::kBufs; ++b) mbar_init(full + b, 1);
+    for (int b = 0; b < PipeRing::kBars; ++b) mbar_init(full + b, 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncthreads();
@@ -491,8 +492,8 @@ __global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlo
   const uint64_t pol = policy_evict_first();
   auto tile_at = [&](int i) { return blockIdx.x + (long long)i * gridDim.x; };
   auto issue = [&](int i) {
-    bulk_load(pipe_smem + (i % Cfg::kBufs) * Cfg::kTileBytes, scratch + tile_at(i) * N * kTile, Cfg::kTileBytes,
-              full + i % Cfg::kBufs, pol);
+    bulk_load(pipe_smem + PipeRing::buffer(i) * Cfg::kTileBytes, scratch + tile_at(i) * N * kTile, Cfg::kTileBytes,
+              full + PipeRing::barrier(i), pol);
   };
   if (tid == 0) {
     for (int i = 0; i < Cfg::kBufs && i < n; ++i) issue(i);
@@ -502,7 +503,7 @@ __global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlo
   const float2 gs = f2(grad_scale), nrm = f2(norm), sc_y = f2(scale);
   double acc = 0.0;
   bool late = false;
-  for (int i = grp; i < n; i += 2) {
+  for (int i = grp; i < n; i += PipeRing::kGroups) {
     const long long tile = tile_at(i);
     const int f = static_cast<int>(tile / tiles), c0 = static_cast<int>(tile - (long long)f * tiles) * kTile;
     // the tile's counts, by rows of the spectrum; the previous tile's were read before a barrier
@@ -517,8 +518,8 @@ __global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlo
       }
       cp_async_commit();
     }
-    float4* rows = reinterpret_cast<float4*>(pipe_smem + (i % Cfg::kBufs) * Cfg::kTileBytes) + p;
-    late |= !mbar_wait(full + i % Cfg::kBufs, (i / Cfg::kBufs) & 1);
+    float4* rows = reinterpret_cast<float4*>(pipe_smem + PipeRing::buffer(i) * Cfg::kTileBytes) + p;
+    late |= !mbar_wait(full + PipeRing::barrier(i), PipeRing::parity(i));
     CPair v[S::N1];
 #pragma unroll
     for (int j = 0; j < S::N1; ++j) {
