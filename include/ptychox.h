@@ -190,7 +190,8 @@ int ptx_workspace_status(const void* workspace, unsigned* status, void* stream);
  * are pending).  Calls on a capturing stream are not tracked. */
 int ptx_status_track(const void* workspace, int tag, int* failed, void* stream);
 int ptx_status_poll(int device, int block, int* failed);
-/* PTX_ERR_OUT_OF_BOUNDS when bit 0 of a status word is set, else PTX_OK. */
+/* PTX_ERR_OUT_OF_BOUNDS when bit 0 of a status word is set, else PTX_ERR_TIMEOUT when bit 1 is (a
+ * bounded device wait of the sweep gave up; its loss and gradients are NaN), else PTX_OK. */
 int ptx_status_code(unsigned status);
 
 /* ---- conventional ptychography at sub-pixel scan positions -------------------------

@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(256) base_rows_forward_rt(
   for (int f = f0; f < f1; ++f) {
     const long long x0 = pos[2 * f], y0 = pos[2 * f + 1];
     const bool ok = window_ok(x0, y0, ph, pw, H, W);
-    if (!ok && tid == 0) atomicOr(err, 1u);
+    if (!ok && tid == 0) atomicOr(err, kStatusWindow);
     for (int i = tid; i < nrows * pw; i += blockDim.x) {
       const int li = i / pw, c = i - li * pw;
       const int r = r0 + li;
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(128, 3) base_rows_forward_reg(
   bool new_group = true;
   for (long long u = u0; u < u1; ++u) {
     const bool row_ok = r < ph;
-    if (tid == 0 && !window_ok(pos[2 * f], pos[2 * f + 1], ph, N, H, W)) atomicOr(err, 1u);
+    if (tid == 0 && !window_ok(pos[2 * f], pos[2 * f + 1], ph, N, H, W)) atomicOr(err, kStatusWindow);
     if (new_group && row_ok) {
       // probe row of the new row group (each thread copies and later reads its own elements)
 #pragma unroll
@@ -626,7 +626,7 @@ __global__ void __launch_bounds__(256, 1) base_sweep_frame(
   for (int f = blockIdx.x; f < nframes; f += gridDim.x) {
     const long long x0 = pos[2 * f], y0 = pos[2 * f + 1];
     if (!window_ok(x0, y0, N, N, H, W)) {
-      if (tid == 0) atomicOr(err, 1u);
+      if (tid == 0) atomicOr(err, kStatusWindow);
       continue;  // uniform across the CTA
     }
     if constexpr (STAGE) {
@@ -723,7 +723,7 @@ static __global__ void window_check_kernel(const int64_t* __restrict__ pos, int 
                                            unsigned* __restrict__ err) {
   pdl_wait();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b < n && !window_ok(pos[2 * b], pos[2 * b + 1], ph, pw, H, W)) atomicOr(err, 1u);
+  if (b < n && !window_ok(pos[2 * b], pos[2 * b + 1], ph, pw, H, W)) atomicOr(err, kStatusWindow);
 }
 
 struct BaseGeom {
@@ -884,7 +884,7 @@ void launch_cols(const BaseGeom& g, int frame0, int nframes, const uint16_t* mea
         if constexpr (col_pipe_length<N>()) {
           if (col_pipe_takes(g.pw, measured)) {
             launch_col_pipe<N, false, true, true>(g.scratch, g.pw, nframes, frame0, g.col.tw, measured, scale, 1.0f,
-                                                  grad_scale, inv_numel, loss, s);
+                                                  grad_scale, inv_numel, loss, g.err, s);
             return;
           }
         }
@@ -1060,7 +1060,9 @@ int ptx_workspace_status(const void* workspace, unsigned* status, void* stream) 
                      "ptx_workspace_status copy");
 }
 
-int ptx_status_code(unsigned status) { return (status & 1u) ? PTX_ERR_OUT_OF_BOUNDS : PTX_OK; }
+int ptx_status_code(unsigned status) {
+  return (status & kStatusWindow) ? PTX_ERR_OUT_OF_BOUNDS : (status & kStatusTimeout) ? PTX_ERR_TIMEOUT : PTX_OK;
+}
 
 int ptx_base_sweep_small(const float* sample, int sample_h, int sample_w, const float* probe, int probe_h,
                          int probe_w, const int64_t* positions_xy, int batch, const uint16_t* measured, float scale,

@@ -353,7 +353,9 @@ std::mutex g_status_mutex;
 std::map<int, StatusRing> g_status;
 
 // Retire the ring's completed calls (all of them, waiting, with `block`); the tag of the first
-// one whose window check failed goes to *failed if that is still negative.
+// one whose window check failed goes to *failed if that is still negative.  A call whose device
+// wait gave up ends the retiring with its error, after a failed window of an earlier one has been
+// reported.
 int retire_status(StatusRing& r, bool block, int* failed) {
   while (!r.pending.empty()) {
     const StatusRing::Call c = r.pending.front();
@@ -363,9 +365,14 @@ int retire_status(StatusRing& r, bool block, int* failed) {
       return PTX_OK;
     }
     if (e != cudaSuccess) return cuda_status(e, "status event");
-    if (*failed < 0 && (r.words[c.slot] & 1u)) *failed = c.tag;
+    const unsigned word = r.words[c.slot];
+    if ((word & kStatusTimeout) && *failed >= 0) return PTX_OK;
+    if (*failed < 0 && (word & kStatusWindow)) *failed = c.tag;
     r.spare.push_back(c.done);
     r.pending.pop_front();
+    if (word & kStatusTimeout) {
+      return set_error(PTX_ERR_TIMEOUT, "a device wait of an earlier sweep gave up: its loss and gradients are NaN");
+    }
   }
   return PTX_OK;
 }

@@ -28,7 +28,7 @@
 namespace ptx {
 namespace {
 
-constexpr size_t kHdr = 256 + kReservedBytes;
+constexpr size_t kHdr = 256 + kReservedBytes;  // error word + padding
 enum FpmMode { kFpmSweep = 0, kFpmForward = 1, kFpmBackward = 2 };
 
 __device__ __forceinline__ int wrap2(long long v, int n) { return static_cast<int>(v & (long long)(n - 1)); }
@@ -308,6 +308,7 @@ struct FpmGeom {
   int chunk;
   float2* spec;   // workspace spectrum (sweep)
   float2* gspec;  // gradient w.r.t. the spectrum
+  unsigned* err;
   float2* tmp;    // tiled temporary of the 2-D passes
   float2* frames;
 };
@@ -349,6 +350,7 @@ int fpm_check(const void* object, int oh, int ow, const void* pupil, int lh, int
   // passes put the frame in gridDim.y)
   g->chunk = static_cast<int>(
       std::min<size_t>({(ws_bytes - fixed) / g->frame_bytes, (size_t)std::max(batch, 1), (size_t)65535}));
+  g->err = static_cast<unsigned*>(ws);
   char* p = static_cast<char*>(ws) + kHdr;
   g->spec = reinterpret_cast<float2*>(p);
   g->gspec = reinterpret_cast<float2*>(p + g->spec_bytes);
@@ -474,7 +476,7 @@ void launch_cols(const FpmGeom& g, int frame0, int nf, const uint16_t* measured,
       if constexpr (col_pipe_length<N>()) {
         if (col_pipe_takes(g.lw, measured)) {
           launch_col_pipe<N, true, false, false>(g.frames, g.lw, nf, frame0, g.p_lh.tw, measured, scale, norm,
-                                                 grad_scale, inv_numel, loss, s);
+                                                 grad_scale, inv_numel, loss, g.err, s);
           return;
         }
       }
@@ -598,7 +600,7 @@ int ptx_fpm_sweep(const float* object, int object_h, int object_w, const float* 
   const double numel = (double)batch * low_h * low_w;
   const float grad_scale = static_cast<float>(2.0 / std::max(numel, 1.0));
   launch_prologue(s, g.gspec, g.spec_bytes / sizeof(float2), reinterpret_cast<float2*>(grad_pupil),
-                  (size_t)low_h * low_w, loss, nullptr);
+                  (size_t)low_h * low_w, loss, g.err);
   launch_fft2<false>(g, reinterpret_cast<const float2*>(object), object_h, object_w, g.spec, 1.0f, g.tmp, g.p_ow, g.p_oh,
                      s);
   const float2* P = reinterpret_cast<const float2*>(pupil);

@@ -18,6 +18,10 @@ int set_error(int code, const char* fmt, ...);
 // Map a CUDA error to PTX_ERR_CUDA with a message; returns PTX_OK for cudaSuccess.
 int cuda_status(cudaError_t e, const char* what);
 
+// Bits of a workspace's status word (ptx_workspace_status).
+constexpr unsigned kStatusWindow = 1u;   // a scan window left the object
+constexpr unsigned kStatusTimeout = 2u;  // a bounded device wait gave up; loss and gradients are NaN
+
 // Build (or fetch from the per-device cache) the line plan for length n on the current
 // device.  Returns PTX_OK or PTX_ERR_UNSUPPORTED_SIZE / PTX_ERR_CUDA.
 int get_line_plan(int n, LinePlan* out);

@@ -390,7 +390,8 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
       : "memory");
 }
 // Wait for the phase of `parity`; false if it has not completed after a bounded number of tries
-// (tens of milliseconds at least, where a copy takes microseconds).
+// (tens of milliseconds at least, where a copy takes microseconds): the caller then stops, waits
+// once more for the copies it still has under way, and reports kStatusTimeout and NaN results.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   for (int i = 0; i < (1 << 20); ++i) {
     uint32_t done;
@@ -405,6 +406,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
 }
 __device__ __forceinline__ void group_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+}
+// group_sync that tells every thread whether `flag` holds for any of them.
+__device__ __forceinline__ bool group_sync_any(int id, int threads, bool flag) {
+  uint32_t any;
+  asm volatile(
+      "{\n.reg .pred p, q;\nsetp.ne.u32 q, %3, 0;\nbar.red.or.pred p, %1, %2, q;\nselp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(any)
+      : "r"(id), "r"(threads), "r"(static_cast<uint32_t>(flag))
+      : "memory");
+  return any != 0;
 }
 
 template <int N>
@@ -468,7 +479,7 @@ template <int N, bool FIRST_INV, bool SHIFTED, bool UNIT_NORM>
 __global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlocks) cols_sweep_pipe(
     float2* __restrict__ scratch, int width, int nframes, int frame0, const float2* __restrict__ tw,
     const uint16_t* __restrict__ measured, float scale, float norm, float grad_scale, double inv_numel,
-    double* __restrict__ loss) {
+    double* __restrict__ loss, unsigned* __restrict__ err) {
   using S = RegShape<N>;
   using Cfg = ColPipeCfg<N>;
   constexpr int P = Cfg::kPairs;
@@ -502,8 +513,8 @@ __global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlo
   const int col_off = SHIFTED ? width / 2 : 0;
   const float2 gs = f2(grad_scale), nrm = f2(norm), sc_y = f2(scale);
   double acc = 0.0;
-  bool late = false;
-  for (int i = grp; i < n; i += PipeRing::kGroups) {
+  int i = grp;
+  for (; i < n; i += PipeRing::kGroups) {
     const long long tile = tile_at(i);
     const int f = static_cast<int>(tile / tiles), c0 = static_cast<int>(tile - (long long)f * tiles) * kTile;
     // the tile's counts, by rows of the spectrum; the previous tile's were read before a barrier
@@ -519,7 +530,7 @@ __global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlo
       cp_async_commit();
     }
     float4* rows = reinterpret_cast<float4*>(pipe_smem + PipeRing::buffer(i) * Cfg::kTileBytes) + p;
-    late |= !mbar_wait(full + PipeRing::barrier(i), PipeRing::parity(i));
+    const bool late = !mbar_wait(full + PipeRing::barrier(i), PipeRing::parity(i));
     CPair v[S::N1];
 #pragma unroll
     for (int j = 0; j < S::N1; ++j) {
@@ -527,7 +538,7 @@ __global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlo
       v[j] = {make_float2(q.x, q.z), make_float2(q.y, q.w)};
     }
     pipe_step1<N, FIRST_INV>(v, rows, t, tws);
-    group_sync(1 + grp, Cfg::kGroup);
+    if (group_sync_any(1 + grp, Cfg::kGroup, late)) break;
     pipe_load2<N>(v, rows, t);
     pipe_step2<N, FIRST_INV>(v);
     cp_async_wait_all();
@@ -567,8 +578,31 @@ __global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlo
       out[(t + S::T * m) * P] = make_float4(z.re.x, z.im.x, z.re.y, z.im.y);
     }
   }
-  // a copy that never came leaves no valid result: the loss says so
-  block_add_double(late ? __longlong_as_double(0x7ff8000000000000ll) : acc, inv_numel, loss);
+  // a copy that did not come: the tiles from there on are NaN, and so are the loss and gradients
+  const bool stopped = i < n;
+  if (__syncthreads_or(stopped)) {
+    const float nan = __int_as_float(0x7fc00000);
+    if (stopped) {
+      if (gt == 0 && err) atomicOr(err, kStatusTimeout);
+      cp_async_wait_all();
+      for (int k = i; k < n; k += PipeRing::kGroups) {
+        float4* out = reinterpret_cast<float4*>(scratch + tile_at(k) * N * kTile) + p;
+        for (int m = 0; m < S::N1; ++m) out[(t + S::T * m) * P] = make_float4(nan, nan, nan, nan);
+      }
+      acc = nan;
+    }
+    // the copies issued and not waited for: they write to this CTA's shared memory
+    int* next = reinterpret_cast<int*>(tws);
+    if (gt == 0) next[grp] = i;
+    __syncthreads();
+    if (tid == 0) {
+      for (int k = 0; k < n; ++k) {
+        if (PipeRing::left_open(k, next)) mbar_wait(full + PipeRing::barrier(k), PipeRing::parity(k));
+      }
+    }
+    __syncthreads();
+  }
+  block_add_double(acc, inv_numel, loss);
 }
 
 // Column lengths the pipeline is used for, and the frames it takes: whole pairs of tiles (the
@@ -588,13 +622,14 @@ int prepare_col_pipe() {
 }
 template <int N, bool FIRST_INV, bool SHIFTED, bool UNIT_NORM>
 void launch_col_pipe(float2* frames, int width, int nframes, int frame0, const float2* tw, const uint16_t* measured,
-                     float scale, float norm, float grad_scale, double inv_numel, double* loss, cudaStream_t s) {
+                     float scale, float norm, float grad_scale, double inv_numel, double* loss, unsigned* err,
+                     cudaStream_t s) {
   using C = ColPipeCfg<N>;
   auto kern = cols_sweep_pipe<N, FIRST_INV, SHIFTED, UNIT_NORM>;
   const int grid =
       persistent_grid((const void*)kern, 2 * C::kGroup, C::kSmemBytes, (long long)num_tiles(width) * nframes);
   launch_pdl(kern, grid, 2 * C::kGroup, C::kSmemBytes, s, frames, width, nframes, frame0, tw, measured, scale, norm,
-             grad_scale, inv_numel, loss);
+             grad_scale, inv_numel, loss, err);
 }
 
 }  // namespace ptx

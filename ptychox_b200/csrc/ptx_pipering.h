@@ -21,6 +21,11 @@ struct PipeRing {
   PTX_RING_HD static constexpr int buffer(int i) { return i % kBufs; }
   PTX_RING_HD static constexpr int barrier(int i) { return i % kBars; }
   PTX_RING_HD static constexpr unsigned parity(int i) { return (i / kBars) & 1; }
+  // whether tile i's copy has been issued and its group stopped before it: next[g] is the first tile
+  // that group g has not finished, and with tile k it issued tile k + kBufs
+  PTX_RING_HD static constexpr bool left_open(int i, const int* next) {
+    return i >= next[group(i)] && (i < kBufs || i - kBufs < next[group(i - kBufs)]);
+  }
 };
 
 }  // namespace ptx

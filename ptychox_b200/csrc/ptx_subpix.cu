@@ -75,7 +75,7 @@ __global__ void subpix_ramp_kernel(const double* __restrict__ pos, int nframes, 
     if (k == 0) {
       long long x0, y0;
       sp_corner(pos, f, x0, y0);
-      if (!sp_window_ok(x0, y0, ph, pw, H, W)) atomicOr(err, 1u);
+      if (!sp_window_ok(x0, y0, ph, pw, H, W)) atomicOr(err, kStatusWindow);
     }
   }
 }
@@ -471,7 +471,7 @@ int sp_launch_cols_sweep(const SpGeom& g, int frame0, int nf, const uint16_t* me
           if (st) return;
           prof_begin(kBaseCols, s);
           launch_col_pipe<N, false, true, true>(g.scratch, g.pw, nf, frame0, g.col.tw, measured, scale, 1.0f, grad_scale,
-                                                inv_numel, loss, s);
+                                                inv_numel, loss, g.err, s);
           prof_end(kBaseCols, s);
           return;
         }

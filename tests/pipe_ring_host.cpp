@@ -4,7 +4,9 @@
 // the barrier's open phase has parity P.  A group that has waited for its tile works on it and
 // then issues the copy of the tile that takes the buffer next.  Prints, per tile count: the
 // states reached, the waits that returned before their tile had come, the copies issued into a
-// buffer or on a barrier still in use, and the states from which nothing goes on before the end.
+// buffer or on a barrier still in use, the states from which nothing goes on before the end, and
+// those in which both groups wait and left_open names other copies than the issued ones they
+// have not waited for, or a wait for one of these would not hold just until it is done.
 #include <cstdio>
 #include <set>
 #include <tuple>
@@ -39,11 +41,16 @@ int main() {
     for (int i = 0; i < Ring::kBufs && i < n; ++i) first.issued |= 1u << i;
     std::set<State> seen{first};
     std::vector<State> todo{first};
-    int early = 0, in_use = 0, stuck = 0;
+    int early = 0, in_use = 0, stuck = 0, wrong_open = 0;
     while (!todo.empty()) {
       const State a = todo.back();
       todo.pop_back();
       bool moved = false;
+      for (int i = 0; i < n && !a.busy[0] && !a.busy[1]; ++i) {
+        const bool open = a.has(a.issued, i) && !a.waited(i);
+        const bool holds = (a.phases(Ring::barrier(i)) & 1u) == Ring::parity(i);
+        wrong_open += Ring::left_open(i, a.next) != open || (open && holds == a.has(a.done, i));
+      }
       auto go = [&](const State& b) {
         moved = true;
         if (seen.insert(b).second) todo.push_back(b);
@@ -78,7 +85,7 @@ int main() {
       }
       stuck += !moved && !(a.next[0] >= n && a.next[1] >= n && a.done == (1u << n) - 1);
     }
-    std::printf("%d %zu %d %d %d\n", n, seen.size(), early, in_use, stuck);
+    std::printf("%d %zu %d %d %d %d\n", n, seen.size(), early, in_use, stuck, wrong_open);
   }
   return 0;
 }
