@@ -834,8 +834,8 @@ int coded_check(int n, int ds, const void* a, const void* b, const void* t2, con
 
 // Shift ramps of every frame, tabulated in FP64 and rounded once: ramps[f][0][k] =
 // exp(2 pi i dx_f fk), ramps[f][1][k] = exp(2 pi i dy_f fk), fk the signed frequency of bin k
-// (numpy fftfreq * n, odd n too).  Part of the sweeps' first launch, which also zeroes what they
-// accumulate into.  Evaluating the two-dimensional ramp per element cost the column passes that apply it a
+// (numpy fftfreq * n, odd n too).  Part of the launch that zeroes what the sweeps accumulate
+// into.  Evaluating the two-dimensional ramp per element cost the column passes that apply it a
 // third of their instructions; the product of the two tables is also the more accurate (6e-8
 // against up to 2e-7 rad from the FP32 reduction of the summed argument).
 __global__ void __launch_bounds__(256) coded_prologue_kernel(float2* __restrict__ gospec, float2* __restrict__ grad_mask,
@@ -866,23 +866,22 @@ __global__ void __launch_bounds__(256) coded_prologue_kernel(float2* __restrict_
   }
 }
 
-// The ramp tables' place: grad_object, which nothing else writes before the last transform; null
-// where they do not fit (more frames than n / 2) or where the caller computes in place, and the
-// passes then evaluate the ramp themselves.
-float2* ramp_tables(int n, int batch, float* grad_object, const float* object, const float* coded_surface) {
-  const bool fits = 2 * (long long)batch <= n && grad_object != object && grad_object != coded_surface &&
-                    (reinterpret_cast<uintptr_t>(grad_object) & 15) == 0;
-  return fits ? reinterpret_cast<float2*>(grad_object) : nullptr;
-}
+// The ramp tables' place: the 2-D transforms' temporary, which holds nothing between the object's
+// transform and the last one; null where they do not fit (more frames than n / 2), and the passes
+// then evaluate the ramp themselves.
+float2* ramp_tables(const CodedGeom& g) { return 2 * (long long)g.batch <= g.n ? g.tmp : nullptr; }
 
-// The first launch of a sweep or adjoint.
-void launch_coded_prologue(const CodedGeom& g, float* grad_coded, double* loss, double* grad_shifts,
-                           const float* shifts, float2* ramps, cudaStream_t s) {
+// What a sweep or adjoint accumulates into is cleared and the ramp tables are written: after the
+// object's transform, which reads the object and uses the tables' place.  Returns the tables.
+const float2* launch_coded_prologue(const CodedGeom& g, float* grad_coded, double* loss, double* grad_shifts,
+                                    const float* shifts, cudaStream_t s) {
   const size_t field = g.field_bytes / sizeof(float2);
+  float2* ramps = ramp_tables(g);
   prof_begin(kMiscKernel, s);
   launch_pdl(coded_prologue_kernel, prologue_blocks(field, sm_count()), 256, 0, s, g.gospec,
              reinterpret_cast<float2*>(grad_coded), field, loss, grad_shifts, shifts, g.batch, g.n, ramps);
   prof_end(kMiscKernel, s);
+  return ramps;
 }
 
 const float2* ramps_at(const float2* ramps, int frame, int n) { return ramps ? ramps + 2 * (size_t)frame * n : nullptr; }
@@ -1102,11 +1101,8 @@ int coded_backward_impl(const float* grad_output, const float* x_forward, const 
   const float2* T1 = reinterpret_cast<const float2*>(transfer_1);
   const float2* T2 = reinterpret_cast<const float2*>(transfer_2);
   const float2* M = reinterpret_cast<const float2*>(coded_surface);
-  if (!prepared) {  // else the caller has launched the prologue
-    float2* tables = ramp_tables(n, batch, grad_object, nullptr, coded_surface);
-    launch_coded_prologue(g, grad_coded, nullptr, nullptr, shifts_xy, tables, s);
-    ramps = tables;
-  }
+  // a sweep's forward has launched the prologue
+  if (!prepared) ramps = launch_coded_prologue(g, grad_coded, nullptr, nullptr, shifts_xy, s);
   for (int b0 = 0; b0 < batch; b0 += g.chunk) {
     const int nf = std::min(g.chunk, batch - b0);
     launch_rows_pool<kCodedBackward>(g, b0, nf, nullptr, 0.f, 0.f, 0.0, nullptr,
@@ -1132,10 +1128,13 @@ size_t ptx_coded_workspace_bytes(int n, int batch) {
   return coded_fixed_bytes(n) + frames * per;
 }
 
+// The forward of a sweep clears what the sweep accumulates into (grad_coded and on: given) and hands on
+// its ramp tables.
 static int coded_forward_impl(const float* object, const float* coded_surface, const float* transfer_1,
                               const float* transfer_2, int n, const float* shifts_xy, int batch, int downsample,
                               float* x_forward, float* sensor, float* amplitude, void* workspace,
-                              size_t workspace_bytes, const float2* ramps, void* stream) {
+                              size_t workspace_bytes, void* stream, float* grad_coded = nullptr,
+                              double* loss = nullptr, double* grad_shifts = nullptr, const float2** tables = nullptr) {
   CodedGeom g;
   if (int st = coded_check(n, downsample, object, coded_surface, transfer_2, shifts_xy, batch, workspace,
                            workspace_bytes, false, &g)) {
@@ -1147,6 +1146,8 @@ static int coded_forward_impl(const float* object, const float* coded_surface, c
   const float2* T2 = reinterpret_cast<const float2*>(transfer_2);
   const float2* M = reinterpret_cast<const float2*>(coded_surface);
   launch_fft2<false>(g, reinterpret_cast<const float2*>(object), n, g.ospec, g.tmp, g.plan, T1, s);
+  const float2* ramps = nullptr;
+  if (tables) *tables = ramps = launch_coded_prologue(g, grad_coded, loss, grad_shifts, shifts_xy, s);
   for (int b0 = 0; b0 < batch; b0 += g.chunk) {
     const int nf = std::min(g.chunk, batch - b0);
     const float* sh = shifts_xy + 2 * (size_t)b0;
@@ -1163,7 +1164,7 @@ int ptx_coded_forward(const float* object, const float* coded_surface, const flo
                       int n, const float* shifts_xy, int batch, int downsample, float* x_forward, float* sensor,
                       float* amplitude, void* workspace, size_t workspace_bytes, void* stream) {
   return coded_forward_impl(object, coded_surface, transfer_1, transfer_2, n, shifts_xy, batch, downsample, x_forward,
-                            sensor, amplitude, workspace, workspace_bytes, nullptr, stream);
+                            sensor, amplitude, workspace, workspace_bytes, stream);
 }
 
 int ptx_coded_backward(const float* grad_output, const float* x_forward, const float* sensor, const float* amplitude,
@@ -1192,12 +1193,11 @@ static int coded_sweep_mse(const float* object, const float* coded_surface, cons
   const float2* T1 = reinterpret_cast<const float2*>(transfer_1);
   const float2* T2 = reinterpret_cast<const float2*>(transfer_2);
   const float2* M = reinterpret_cast<const float2*>(coded_surface);
-  float2* ramps = ramp_tables(n, batch, grad_object, object, coded_surface);
-  launch_coded_prologue(g, grad_coded, loss, grad_shifts, shifts_xy, ramps, s);
   const int lw = n / downsample;
   const double numel = (double)batch * lw * lw;
   const float grad_scale = static_cast<float>(2.0 / std::max(numel, 1.0));
   launch_fft2<false>(g, reinterpret_cast<const float2*>(object), n, g.ospec, g.tmp, g.plan, T1, s);
+  const float2* ramps = launch_coded_prologue(g, grad_coded, loss, grad_shifts, shifts_xy, s);
   for (int b0 = 0; b0 < batch; b0 += g.chunk) {
     const int nf = std::min(g.chunk, batch - b0);
     const float* sh = shifts_xy + 2 * (size_t)b0;
@@ -1267,16 +1267,11 @@ static int coded_sweep_fd(const float* object, const float* coded_surface, const
   p += up(b * pooled);
   const size_t inner = workspace_bytes - static_cast<size_t>(p - static_cast<char*>(workspace));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // the adjoint accumulates into its object-spectrum gradient in the frames' region; the shift
-  // gradient reads the object spectrum the forward leaves there
-  CodedGeom g;
-  if (int st = coded_check(n, downsample, object, coded_surface, transfer_2, shifts_xy, batch, p, inner, false, &g)) {
-    return st;
-  }
-  float2* ramps = ramp_tables(n, batch, grad_object, object, coded_surface);
-  launch_coded_prologue(g, grad_coded, loss, grad_shifts, shifts_xy, ramps, s);
+  // forward and adjoint share the frames' region: the object-spectrum gradient the forward clears,
+  // the object spectrum it leaves for the shift gradient, and its ramp tables
+  const float2* ramps = nullptr;
   if (int st = coded_forward_impl(object, coded_surface, transfer_1, transfer_2, n, shifts_xy, batch, downsample, xf,
-                                  sensor, amp, p, inner, ramps, stream)) {
+                                  sensor, amp, p, inner, stream, grad_coded, loss, grad_shifts, &ramps)) {
     return st;
   }
   const long long total = (long long)batch * h * h;
