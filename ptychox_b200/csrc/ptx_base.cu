@@ -610,7 +610,7 @@ template <int N, bool STAGE>
 __global__ void __launch_bounds__(256, 1) base_sweep_frame(
     const float2* __restrict__ sample, int H, int W, const float2* __restrict__ probe,
     const int64_t* __restrict__ pos, int nframes, const uint16_t* __restrict__ measured,
-    float scale, float grad_scale, double inv_numel, double* __restrict__ loss,
+    CountScale counts, float grad_scale, double inv_numel, double* __restrict__ loss,
     float2* __restrict__ grad_sample, float2* __restrict__ grad_probe, const float2* __restrict__ tw,
     unsigned* __restrict__ err) {
   pdl_wait();
@@ -669,10 +669,9 @@ __global__ void __launch_bounds__(256, 1) base_sweep_frame(
       for (int m = 0; m < S::N1; ++m) {
         const int kr = t + S::T * m;
         const int ir = (kr + N / 2) & (N - 1);
-        const float y = decode_amplitude(STAGE ? cnt_s[ir * Cfg::CP + ic] : cnt[ir * N + ic], scale);
         float a, inv;
         abs_and_inv(v[m], kEps, a, inv);
-        const float rr = a - y;
+        const float rr = minus_amplitude(a, STAGE ? cnt_s[ir * Cfg::CP + ic] : cnt[ir * N + ic], counts);
         part += static_cast<double>(rr * rr);
         v[m] = cscale(v[m], grad_scale * rr * inv);
       }

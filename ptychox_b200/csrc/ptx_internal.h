@@ -9,6 +9,7 @@
 #include <type_traits>
 
 #include "../../include/ptychox.h"
+#include "ptx_counts.cuh"
 #include "ptx_fft.cuh"
 
 namespace ptx {
@@ -186,7 +187,7 @@ struct MixColsArgs {
   const float2* twt;     // column-length twiddles
   const float2* twi;
   const uint16_t* measured;  // sweep: fftshifted counts
-  float scale;               // sweep: observed amplitude = sqrt(count scale)
+  CountScale counts;         // sweep: observed amplitude = sqrt(count scale)
   float grad_scale;
   double inv_numel;
   double* loss;
@@ -226,7 +227,7 @@ struct MixFpmColsArgs {
   const float2* twt;  // column-length (lh) twiddles
   const float2* twi;
   const uint16_t* measured;  // sweep: counts (not shifted)
-  float scale;
+  CountScale counts;
   float norm;                // 1 / (lh lw)
   float grad_scale;
   double inv_numel;

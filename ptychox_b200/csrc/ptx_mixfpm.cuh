@@ -299,10 +299,9 @@ __global__ void __launch_bounds__(ColCfg<N>::THREADS) mix_fpm_cols(MixFpmColsArg
         float2 out = make_float2(0.f, 0.f);
         if (col_ok) {
           const float2 im = cscale(z[k], a.norm);
-          const float yv = decode_amplitude(meas_s[kr * C + c], a.scale);
           float am, inv;
           abs_and_inv(im, kEps, am, inv);
-          const float rr = am - yv;
+          const float rr = minus_amplitude(am, meas_s[kr * C + c], a.counts);
           part = fmaf(rr, rr, part);
           out = cscale(im, a.grad_scale * rr * inv);
         }

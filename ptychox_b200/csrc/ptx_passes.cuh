@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <stdint.h>
 
+#include "ptx_counts.cuh"
 #include "ptx_internal.h"
 #include "ptx_pairfft.cuh"
 #include "ptx_pipering.h"
@@ -115,28 +116,6 @@ inline void launch_prologue(cudaStream_t s, float2* zero_a, size_t n_a, float2* 
 __device__ __forceinline__ float rsqrt_nr(float s) {
   const float y = rsqrtf(s);
   return y * fmaf(-0.5f * s, y * y, 1.5f);
-}
-
-// sqrt(count scale), the amplitude observed at a detector pixel: a reciprocal square root refined
-// by one step of g + (x - g^2) h, h ~ 1 / (2 sqrt x) (P. Markstein, IBM J. Res. Dev. 34, 111
-// (1990)), which rounds to nearest; 0 for no counts.  A table of all 65536 counts read by the
-// epilogues instead cost their warps the loads' latency (Fourier columns of 225 x 256^2: 65.9
-// against 59.3 us) and each sweep its making.
-__device__ __forceinline__ float rsqrt_floor(float x) {  // 1 / sqrt(max(x, the least normal number))
-  float y;
-  asm("rsqrt.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(fmaxf(x, 1.1754944e-38f)));
-  return y;
-}
-__device__ __forceinline__ float decode_amplitude(uint32_t count, float scale) {
-  const float x = static_cast<float>(count) * scale;
-  const float y = rsqrt_floor(x), g = x * y;
-  return fmaf(fmaf(-g, g, x), 0.5f * y, g);
-}
-// of the two counts of a 32-bit word
-__device__ __forceinline__ float2 decode_amplitudes(uint32_t counts, float2 scale) {
-  const float2 x = mul2(make_float2(static_cast<float>(counts & 0xffffu), static_cast<float>(counts >> 16)), scale);
-  const float2 y = make_float2(rsqrt_floor(x.x), rsqrt_floor(x.y)), g = mul2(x, y);
-  return fma2(fma2(neg2(g), g, x), mul2(f2(0.5f), y), g);
 }
 
 // |z| and 1 / max(|z|, eps) from one reciprocal square root.
@@ -251,7 +230,7 @@ __global__ void __launch_bounds__(256, 2) fft2_cols_kernel(const float2* __restr
 // one packed instruction for two columns.  A column pair is one 16-byte load / store per
 // row (a warp covers four whole 128-byte tile rows).  The sequence per column: DFT in the
 // FIRST_INV direction, scale by `norm`, amplitude-loss epilogue against the counts
-// (decoded with `scale`; SHIFTED: the counts are stored fftshifted in both axes), the
+// (decoded with their scale; SHIFTED: the counts are stored fftshifted in both axes), the
 // DFT in the other direction, store in place.  The tile's counts arrive by cp.async while
 // the first transform runs; the twiddle table sits in shared memory as broadcast pairs.
 template <int N>
@@ -277,7 +256,7 @@ constexpr int col_pair_min_blocks() {
 template <int N, bool FIRST_INV, bool SHIFTED, bool UNIT_NORM = false, bool FULL = false>
 __global__ void __launch_bounds__(ColPairCfg<N>::kThreads, col_pair_min_blocks<N>()) cols_sweep_pair(
     float2* __restrict__ scratch, int width, int frame0, const float2* __restrict__ tw,
-    const uint16_t* __restrict__ measured, float scale, float norm, float grad_scale, double inv_numel,
+    const uint16_t* __restrict__ measured, CountScale counts, float norm, float grad_scale, double inv_numel,
     double* __restrict__ loss) {
   pdl_wait();
   using S = RegShape<N>;
@@ -337,7 +316,7 @@ __global__ void __launch_bounds__(ColPairCfg<N>::kThreads, col_pair_min_blocks<N
   cp_async_wait_all();
   __syncthreads();
   float2 part = make_float2(0.f, 0.f);  // squared residuals of the two columns
-  const float2 gs = f2(grad_scale), nrm = f2(norm), sc_y = f2(scale);
+  const float2 gs = f2(grad_scale), nrm = f2(norm);
 #pragma unroll
   for (int m = 0; m < S::N1; ++m) {
     const int kr = t + S::T * m;
@@ -350,7 +329,7 @@ __global__ void __launch_bounds__(ColPairCfg<N>::kThreads, col_pair_min_blocks<N
     const float2 a = mul2(s2, r);
     const float2 inv =
         make_float2(a.x >= kEpsF32 ? r.x : 1.0f / kEpsF32, a.y >= kEpsF32 ? r.y : 1.0f / kEpsF32);
-    float2 rr = sub2(a, decode_amplitudes(*reinterpret_cast<const uint32_t*>(meas_s + kr * kTile + 2 * p), sc_y));
+    float2 rr = minus_amplitudes(a, *reinterpret_cast<const uint32_t*>(meas_s + kr * kTile + 2 * p), counts);
     rr = make_float2(okA ? rr.x : 0.f, okB ? rr.y : 0.f);
     part = fma2(rr, rr, part);
     const float2 sc = mul2(mul2(gs, rr), inv);
@@ -478,7 +457,7 @@ __device__ __forceinline__ constexpr int pipe_index(int m) {
 template <int N, bool FIRST_INV, bool SHIFTED, bool UNIT_NORM>
 __global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlocks) cols_sweep_pipe(
     float2* __restrict__ scratch, int width, int nframes, int frame0, const float2* __restrict__ tw,
-    const uint16_t* __restrict__ measured, float scale, float norm, float grad_scale, double inv_numel,
+    const uint16_t* __restrict__ measured, CountScale counts, float norm, float grad_scale, double inv_numel,
     double* __restrict__ loss, unsigned* __restrict__ err) {
   using S = RegShape<N>;
   using Cfg = ColPipeCfg<N>;
@@ -511,7 +490,7 @@ __global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlo
   }
   constexpr int kRowOff = SHIFTED ? N / 2 : 0;
   const int col_off = SHIFTED ? width / 2 : 0;
-  const float2 gs = f2(grad_scale), nrm = f2(norm), sc_y = f2(scale);
+  const float2 gs = f2(grad_scale), nrm = f2(norm);
   double acc = 0.0;
   int i = grp;
   for (; i < n; i += PipeRing::kGroups) {
@@ -558,7 +537,7 @@ __global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlo
       const float2 a = mul2(s2, r);
       const float2 inv =
           make_float2(a.x >= kEpsF32 ? r.x : 1.0f / kEpsF32, a.y >= kEpsF32 ? r.y : 1.0f / kEpsF32);
-      const float2 rr = sub2(a, decode_amplitudes(*reinterpret_cast<const uint32_t*>(meas_s + kr * kTile + 2 * p), sc_y));
+      const float2 rr = minus_amplitudes(a, *reinterpret_cast<const uint32_t*>(meas_s + kr * kTile + 2 * p), counts);
       part = fma2(rr, rr, part);
       const float2 sc = mul2(mul2(gs, rr), inv);
       g[m] = {mul2(F.re, sc), mul2(F.im, sc)};
