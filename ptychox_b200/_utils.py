@@ -11,6 +11,7 @@ from __future__ import annotations
 import contextlib
 
 import torch
+from torch.autograd import forward_ad
 
 from . import _abi
 
@@ -170,23 +171,30 @@ def as_u16(measured: torch.Tensor, device: torch.device) -> torch.Tensor:
     return measured.to(device=device).contiguous()
 
 
+def readable(t: torch.Tensor) -> bool:
+    """Whether a kernel may read ``t`` through its pointer: storage of its own (not a batched
+    tensor of vmap) that holds its values (no conjugate or negative view), and no tangent that
+    only torch's operators carry on."""
+    try:
+        stored = t.data_ptr() != 0
+    except RuntimeError:
+        return False
+    return stored and not t.is_conj() and not t.is_neg() and forward_ad.unpack_dual(t).tangent is None
+
+
 def scaled_gradients(grad_loss: torch.Tensor, first: torch.Tensor, second: torch.Tensor):
     """``(first * g, second * g)`` for saved unit-loss gradients and the FP64 scalar gradient
     ``g`` of the loss: one launch, or torch's products where those are needed themselves (a
-    backward that is to be differentiated) or hold what the kernel cannot read (batched or
-    moved saved tensors)."""
-    if not torch.is_grad_enabled():
+    backward that is to be differentiated, a tangent of ``g``) or hold what the kernel cannot
+    read (batched or moved saved tensors, conjugate or negative views)."""
+    if not torch.is_grad_enabled() and readable(grad_loss) and readable(first) and readable(second):
         dev = first.device
-        try:
-            args = grad_loss.data_ptr(), first.data_ptr(), second.data_ptr()
-        except RuntimeError:  # a tensor without storage of its own (vmap)
-            args = (0,)
-        if all(args) and dev.type == "cuda" and grad_loss.device == dev == second.device \
+        if dev.type == "cuda" and grad_loss.device == dev == second.device \
                 and grad_loss.dtype == torch.float64 and grad_loss.numel() == 1 \
                 and first.dtype == second.dtype == torch.complex64 and first.is_contiguous() and second.is_contiguous():
             out = torch.empty_like(first), torch.empty_like(second)
-            call_on(dev, "ptx_scale_gradients", args[0], args[1], out[0].data_ptr(), first.numel(), args[2],
-                    out[1].data_ptr(), second.numel())
+            call_on(dev, "ptx_scale_gradients", ptr(grad_loss), ptr(first), ptr(out[0]), first.numel(), ptr(second),
+                    ptr(out[1]), second.numel())
             return out
     g = grad_loss.to(torch.float32)
     return first * g, second * g

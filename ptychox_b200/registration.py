@@ -25,10 +25,9 @@ from __future__ import annotations
 import math
 
 import torch
-from torch.autograd import forward_ad
 
 from . import _abi
-from ._utils import ptr, stream_handle, workspace
+from ._utils import ptr, readable, stream_handle, workspace
 
 __all__ = ["dftregistration", "track_position", "refine_position"]
 
@@ -104,14 +103,8 @@ def _in_memory(t: torch.Tensor) -> torch.Tensor:
 
 
 def _plain(t: torch.Tensor) -> bool:
-    """Whether the library may read ``t`` directly: it has storage of its own (not a batched
-    tensor of vmap) and carries no derivative."""
-    try:
-        stored = t.data_ptr() != 0
-    except RuntimeError:
-        stored = False
-    return (stored and not (t.requires_grad and torch.is_grad_enabled())
-            and forward_ad.unpack_dual(t).tangent is None)
+    """Whether the library may read ``t`` directly, and no derivative is wanted of it."""
+    return readable(t) and not (t.requires_grad and torch.is_grad_enabled())
 
 
 def _energy(spec: torch.Tensor) -> torch.Tensor:
@@ -220,9 +213,11 @@ def _spectra(images: torch.Tensor) -> torch.Tensor:
     """``fft2`` of real images ``[..., h, w]``, complex64."""
     h, w = images.shape[-2:]
     own = _prime_fft_bytes(images.numel() // max(1, h * w), h, w)
+    if own:
+        images = images.resolve_neg()
     if not own or images.dtype != torch.float32 or not _plain(images):
         return torch.fft.fft2(images.to(torch.complex64))
-    x = images.reshape(-1, h, w).resolve_neg()
+    x = images.reshape(-1, h, w)
     if x.stride(2) != 1:
         x = x.contiguous()
     half = torch.empty(x.shape[0], w, h, dtype=torch.complex64, device=x.device)
