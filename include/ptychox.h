@@ -479,7 +479,9 @@ int ptx_reg_upsampled_peak(const float* cross_power, int batch, int rows, int co
  *                          (int32 [batch][2], signed half pixels), the centres round(shift usfac)
  *                          for ptx_reg_upsampled_peak (int32 [batch] each), and the correlation
  *                          there (interleaved complex128 [batch])
- *   ptx_reg_energy         sum |spec|^2 of each image in FP64 */
+ *   ptx_reg_energy         sum |spec|^2 of each image in FP64
+ *   ptx_reg_partial_energy the same over `parts` pieces of each image, `energy` [batch][parts], for
+ *                          few and large images; ptx_reg_energy_parts is the number that fills the GPU */
 int ptx_reg_cross_power(const float* spec1, int batch1, const float* spec2, int batch, int rows, int cols,
                         float* padded, float* cross_power, void* stream);
 int ptx_reg_pad_transpose(const float* in, int batch, int rows, int cols, float* out, void* stream);
@@ -501,6 +503,8 @@ int ptx_reg_prime_fft2(const float* images, long long image_stride, long long ro
 int ptx_reg_prime_correlation(const float* cross_power, int batch, int rows, int cols, float* half,
                               float* correlation, void* workspace, size_t workspace_bytes, void* stream);
 int ptx_reg_energy(const float* spec, int batch, int rows, int cols, double* energy, void* stream);
+int ptx_reg_energy_parts(int batch, int rows, int cols);
+int ptx_reg_partial_energy(const float* spec, int batch, int rows, int cols, int parts, double* energy, void* stream);
 
 #ifdef __cplusplus
 }  /* extern "C" */

@@ -90,6 +90,8 @@ SIGNATURES: dict[str, tuple] = {
     "ptx_reg_prime_fft2": (_i, [_p, C.c_longlong, C.c_longlong, _i, _i, _i, _p, _p, _p, _sz, _p]),
     "ptx_reg_prime_correlation": (_i, [_p, _i, _i, _i, _p, _p, _p, _sz, _p]),
     "ptx_reg_energy": (_i, [_p, _i, _i, _i, _p, _p]),
+    "ptx_reg_energy_parts": (_i, [_i, _i, _i]),
+    "ptx_reg_partial_energy": (_i, [_p, _i, _i, _i, _i, _p, _p]),
     "ptx_server_create": (_i, [_i, _sz, _i, _p]),
     "ptx_server_submit": (_i, [_p, _p, _p]),
     "ptx_server_poll": (_i, [_p, C.c_longlong, _p, _p, _p, _p, _p]),

@@ -513,23 +513,29 @@ __global__ void __launch_bounds__(32) reg_estimate_kernel(const PeakCand* __rest
   }
 }
 
-// sum |spec[b]|^2 in FP64, one CTA per image (the same order of summation on every call)
-__global__ void __launch_bounds__(1024) reg_energy_kernel(const float2* __restrict__ spec, long long count,
+// sum |spec[b]|^2 in FP64 over `parts` pieces of each image, one CTA per piece (the same order of
+// summation on every call).  A CTA alone reads 60 GB/s, bound by the latency of its loads, so that few
+// and large images are shared out (us, with the sum over the pieces, in one piece -> as
+// ptx_reg_energy_parts has it): one of 4096^2 2290 -> 31 (4.3 TB/s), one of 512^2 27 -> 10, 64 of
+// 512^2 48 -> 29; 200 of 472^2 keep one piece (60; 68 in three).
+__global__ void __launch_bounds__(1024) reg_energy_kernel(const float2* __restrict__ spec, long long count, int parts,
                                                           double* __restrict__ out) {
-  __shared__ double part[32];
-  const float2* sb = spec + (size_t)blockIdx.x * count;
+  __shared__ double sums[32];
+  const long long image = blockIdx.x / parts, p = blockIdx.x - image * parts;
+  const float2* sb = spec + image * count;
+  const long long end = count * (p + 1) / parts;
   double s = 0.0;
 #pragma unroll 4
-  for (long long i = threadIdx.x; i < count; i += 1024) {
+  for (long long i = count * p / parts + threadIdx.x; i < end; i += 1024) {
     const double x = sb[i].x, y = sb[i].y;
     s = fma(x, x, fma(y, y, s));
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+  if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = s;
   __syncthreads();
   if (threadIdx.x < 32) {
-    s = part[threadIdx.x];
+    s = sums[threadIdx.x];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (threadIdx.x == 0) out[blockIdx.x] = s;
@@ -724,15 +730,29 @@ int ptx_reg_estimate(const float* correlation, int batch, int rows, int cols, in
   return cuda_status(cudaGetLastError(), "ptx_reg_estimate launch");
 }
 
-int ptx_reg_energy(const float* spec, int batch, int rows, int cols, double* energy, void* stream) {
+int ptx_reg_energy_parts(int batch, int rows, int cols) {
+  if (batch <= 0 || rows <= 0 || cols <= 0) return 1;
+  // at most one wave of CTAs (two of 1024 threads per SM), of at least 2^15 values each: below that
+  // the sum over the pieces costs what they gain
+  const long long resident = 2LL * sm_count() / batch, most = (long long)rows * cols >> 15;
+  return static_cast<int>(std::max(1LL, std::min(resident, most)));
+}
+
+int ptx_reg_partial_energy(const float* spec, int batch, int rows, int cols, int parts, double* energy, void* stream) {
   if (int st = reg_check_stack(batch, rows, cols)) return st;
+  if (parts < 1 || (long long)parts * batch > 0x7fffffff) return set_error(PTX_ERR_INVALID_ARGUMENT, "parts out of range");
   if (batch == 0) return PTX_OK;
   if (!spec || !energy) return set_error(PTX_ERR_INVALID_ARGUMENT, "null pointer argument");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   prof_begin(kMiscKernel, s);
-  reg_energy_kernel<<<batch, 1024, 0, s>>>(reinterpret_cast<const float2*>(spec), (long long)rows * cols, energy);
+  reg_energy_kernel<<<batch * parts, 1024, 0, s>>>(reinterpret_cast<const float2*>(spec), (long long)rows * cols, parts,
+                                                   energy);
   prof_end(kMiscKernel, s);
   return cuda_status(cudaGetLastError(), "ptx_reg_energy launch");
+}
+
+int ptx_reg_energy(const float* spec, int batch, int rows, int cols, double* energy, void* stream) {
+  return ptx_reg_partial_energy(spec, batch, rows, cols, 1, energy, stream);
 }
 
 }  // extern "C"

@@ -111,10 +111,11 @@ def _energy(spec: torch.Tensor) -> torch.Tensor:
     """``sum |spec|^2`` of each image in FP64."""
     if spec.numel() and not _plain(spec):
         return (spec.abs().double() ** 2).sum(dim=(-2, -1))
-    out = torch.empty(spec.shape[0], dtype=torch.float64, device=spec.device)
     with torch.cuda.device(spec.device):
-        _abi.call("ptx_reg_energy", ptr(spec), *spec.shape, ptr(out), stream_handle(spec.device))
-    return out
+        parts = _abi.query("ptx_reg_energy_parts", *spec.shape)
+        out = torch.empty(spec.shape[0], parts, dtype=torch.float64, device=spec.device)
+        _abi.call("ptx_reg_partial_energy", ptr(spec), *spec.shape, parts, ptr(out), stream_handle(spec.device))
+    return out.sum(dim=1) if parts > 1 else out[:, 0]
 
 
 def _refine(q: torch.Tensor, usfac: int, rc: torch.Tensor, cc: torch.Tensor):

@@ -62,3 +62,23 @@ def test_spectra_on_two_devices_are_refused():
     for usfac in (0, 1, 2, 100):
         with pytest.raises(ValueError, match="same device"):
             dftregistration(a, b, usfac)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch, rows, cols", [(1, 1, 1), (1, 255, 257), (1, 256, 256), (1, 1500, 1777), (3, 700, 701), (40, 181, 182),
+                                               (700, 130, 129), (2, 1, 40000)])
+def test_energies_of_few_and_many_images(batch, rows, cols):
+    """One piece per image, several, and more than divide it evenly: within the rounding of an FP64 sum
+    in any order, and the same on every call."""
+    from ptychox_b200 import _abi
+    from ptychox_b200.registration import _energy
+
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    spec = torch.randn(batch, rows, cols, dtype=torch.complex64, generator=gen, device="cuda")
+    parts = _abi.query("ptx_reg_energy_parts", batch, rows, cols)
+    assert 1 <= parts <= max(1, rows * cols // 2**15)
+    want = torch.view_as_real(spec).double().square().sum(dim=(1, 2, 3))
+    got = _energy(spec)
+    eps = torch.finfo(torch.float64).eps
+    assert ((got - want).abs() <= 4 * rows * cols * eps * want).all()
+    assert torch.equal(got, _energy(spec))
