@@ -834,7 +834,7 @@ int coded_check(int n, int ds, const void* a, const void* b, const void* t2, con
 
 // Shift ramps of every frame, tabulated in FP64 and rounded once: ramps[f][0][k] =
 // exp(2 pi i dx_f fk), ramps[f][1][k] = exp(2 pi i dy_f fk), fk the signed frequency of bin k
-// (numpy fftfreq * n, odd n too).  Part of the launch that zeroes what the sweeps accumulate
+// (numpy fftfreq * n).  Part of the launch that zeroes what the sweeps accumulate
 // into.  Evaluating the two-dimensional ramp per element cost the column passes that apply it a
 // third of their instructions; the product of the two tables is also the more accurate (6e-8
 // against up to 2e-7 rad from the FP32 reduction of the summed argument).
@@ -868,8 +868,8 @@ __global__ void __launch_bounds__(256) coded_prologue_kernel(float2* __restrict_
 
 // The ramp tables' place: the 2-D transforms' temporary, which holds nothing between the object's
 // transform and the last one; null where they do not fit (more frames than n / 2), and the passes
-// then evaluate the ramp themselves.
-float2* ramp_tables(const CodedGeom& g) { return 2 * (long long)g.batch <= g.n ? g.tmp : nullptr; }
+// then evaluate the ramp themselves, as the mixed-radix ones do.
+float2* ramp_tables(const CodedGeom& g) { return !g.mix && 2 * (long long)g.batch <= g.n ? g.tmp : nullptr; }
 
 // What a sweep or adjoint accumulates into is cleared and the ramp tables are written: after the
 // object's transform, which reads the object and uses the tables' place.  Returns the tables.
@@ -936,7 +936,6 @@ void launch_cols(const CodedGeom& g, int nf, const float2* t2, const float* shif
     MixCodedArgs a = mix_args(g, nf, inv_n);
     a.t2 = t2;
     a.shifts = shifts;
-    a.ramps = ramps;
     a.grad_shifts = STAGE == 7 ? grad_shifts : nullptr;
     g.mix->cols(STAGE, CONJ, a, s);
     prof_end(kCodedCols, s);

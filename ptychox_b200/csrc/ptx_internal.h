@@ -259,7 +259,6 @@ struct MixCodedArgs {
   const float2* ospec;      // O^ T1 = fft2(O) T1 (near-field: fft2(O))
   const float2* t2;
   const float* shifts;      // (dx, dy) per frame of this chunk
-  const float2* ramps;      // their ramps [frame][x, y][n], or null (evaluated)
   float inv_n;              // 1 / n^2
   float2* grad_ospec;
   const float2* twt;        // line twiddles of n (LinePlan::mix_twt / mix_twi)

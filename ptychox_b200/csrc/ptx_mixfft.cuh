@@ -295,9 +295,7 @@ struct Shape {
 // RS = P, CS = 1 for lines stored one after another; RS = B * C, CS = C for C lines interleaved
 // element by element (the column kernels, whose neighbouring threads own neighbouring lines).
 // Twiddle tables, both of N entries: twt[u * B + t] = twi[t * A + u] = exp(-2 pi i t u / N)
-// (one per layout, so each step reads consecutive entries from consecutive threads).  With
-// TP > 0 both steps take one table instead, tw[u * TP + t], for shared memory: an odd pitch TP
-// serves either order of the threads without bank conflicts.
+// (one per layout, so each step reads consecutive entries from consecutive threads).
 
 // The steps below take the sign of the transform as PLUS: exp(-2 pi i ...) for PLUS = false
 // (the forward DFT), exp(+2 pi i ...) for PLUS = true (the unnormalised inverse).  "fwd" steps
@@ -307,14 +305,14 @@ struct Shape {
 
 // Space -> frequency, step 1, thread t < B: DFT-A of x[t + B j] (in y, j < A), twiddle,
 // store row u.
-template <int N, int RS, int CS, bool PLUS = false, int TP = 0>
+template <int N, int RS, int CS, bool PLUS = false>
 PTX_MIX_HD void fwd_step1(float2 (&y)[Shape<N>::A], float2* buf, int t, const float2* twt) {
   using S = Shape<N>;
   Dft<S::A, PLUS>::run(y);
   buf[t * CS] = y[0];
 #pragma unroll
   for (int u = 1; u < S::A; ++u) {
-    const float2 w = twt[u * (TP > 0 ? TP : S::B) + t];
+    const float2 w = twt[u * S::B + t];
     buf[u * RS + t * CS] = PLUS ? mulc(y[u], w) : mul(y[u], w);
   }
 }
@@ -329,14 +327,14 @@ PTX_MIX_HD void fwd_step2(float2 (&z)[Shape<N>::B], const float2* buf, int u) {
 }
 
 // Frequency -> space, step 1, thread u < A: DFT-B of X[u + A k] (in z), twiddle, store row u.
-template <int N, int RS, int CS, bool PLUS = true, int TP = 0>
+template <int N, int RS, int CS, bool PLUS = true>
 PTX_MIX_HD void inv_step1(float2 (&z)[Shape<N>::B], float2* buf, int u, const float2* twi) {
   using S = Shape<N>;
   Dft<S::B, PLUS>::run(z);
   buf[u * RS] = z[0];
 #pragma unroll
   for (int t = 1; t < S::B; ++t) {
-    const float2 w = TP > 0 ? twi[u * TP + t] : twi[t * S::A + u];
+    const float2 w = twi[t * S::A + u];
     buf[u * RS + t * CS] = PLUS ? mulc(z[t], w) : mul(z[t], w);
   }
 }
