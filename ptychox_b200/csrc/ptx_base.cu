@@ -881,7 +881,7 @@ void launch_cols(const BaseGeom& g, int frame0, int nframes, const uint16_t* mea
         // column DFT, amplitude-loss epilogue and inverse column DFT; counts fftshifted
         dim3 grid(num_tiles(g.pw), nframes);
         if constexpr (col_pipe_length<N>()) {
-          if (col_pipe_takes(g.pw, measured)) {
+          if (col_pipe_takes(g.pw, nframes, measured)) {
             launch_col_pipe<N, false, true, true>(g.scratch, g.pw, nframes, frame0, g.col.tw, measured, scale, 1.0f,
                                                   grad_scale, inv_numel, loss, g.err, s);
             return;

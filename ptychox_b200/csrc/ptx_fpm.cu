@@ -474,7 +474,7 @@ void launch_cols(const FpmGeom& g, int frame0, int nf, const uint16_t* measured,
       // inverse column DFT, 1/(h w), amplitude-loss epilogue, forward column DFT
       dim3 grid(num_tiles(g.lw), nf);
       if constexpr (col_pipe_length<N>()) {
-        if (col_pipe_takes(g.lw, measured)) {
+        if (col_pipe_takes(g.lw, nf, measured)) {
           launch_col_pipe<N, true, false, false>(g.frames, g.lw, nf, frame0, g.p_lh.tw, measured, scale, norm,
                                                  grad_scale, inv_numel, loss, g.err, s);
           return;

@@ -585,15 +585,19 @@ __global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlo
 }
 
 // Column lengths the pipeline is used for, and the frames it takes: whole pairs of tiles (the
-// counts' 16-byte pieces stay inside a tile), counts on a 16-byte boundary.  At 512 points a CTA of
-// cols_sweep_pair leaves no room for the next tile's loads beside it (1135 us against 1023 here);
-// at 256 several of its CTAs share an SM and it is the faster one (225 frames: 60.5 us against 69.8).
+// counts' 16-byte pieces stay inside a tile), counts on a 16-byte boundary, and five tiles or more per
+// CTA.  At 512 points a CTA of cols_sweep_pair leaves no room for the next tile's loads beside it
+// (14400 tiles 1135 us against 1023 here); at 256 several of its CTAs share an SM and it is the faster
+// one (225 frames: 60.5 us against 69.8).  With few tiles per CTA the pipeline's start and end
+// weigh more (whole sweeps, us, pipeline and pair: 180 tiles of 512 x 96 33.3 and 32.5, 600 tiles 81.6 and
+// 79.5, 640 tiles of 512^2 75.1 and 73.2; equal within 1% from 740 to 1200 tiles).
 template <int N>
 constexpr bool col_pipe_length() {
   return N == 512;
 }
-inline bool col_pipe_takes(int width, const uint16_t* measured) {
-  return width % (2 * kTile) == 0 && (reinterpret_cast<uintptr_t>(measured) & 15) == 0;
+inline bool col_pipe_takes(int width, int nframes, const uint16_t* measured) {
+  return width % (2 * kTile) == 0 && (reinterpret_cast<uintptr_t>(measured) & 15) == 0 &&
+         (long long)(width / kTile) * nframes >= 5LL * sm_count();
 }
 template <int N, bool FIRST_INV, bool SHIFTED, bool UNIT_NORM>
 int prepare_col_pipe() {

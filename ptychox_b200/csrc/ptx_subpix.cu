@@ -466,7 +466,7 @@ int sp_launch_cols_sweep(const SpGeom& g, int frame0, int nf, const uint16_t* me
     constexpr int N = decltype(NT)::value;
     if constexpr (N >= 16) {
       if constexpr (col_pipe_length<N>()) {
-        if (col_pipe_takes(g.pw, measured)) {
+        if (col_pipe_takes(g.pw, nf, measured)) {
           st = prepare_col_pipe<N, false, true, true>();
           if (st) return;
           prof_begin(kBaseCols, s);
