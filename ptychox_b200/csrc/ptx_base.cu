@@ -787,11 +787,7 @@ int check_common(const void* sample, int H, int W, const void* probe, int ph, in
     constexpr int N = decltype(NT)::value;
     if constexpr (N > 0) {
       const int sm = RegLaunch<N>::col_smem();
-      if (!st) st = ensure_smem((const void*)cols_sweep_pair<N, false, true>, ColPairCfg<N>::kSmemBytes);
-      if (!st) st = ensure_smem((const void*)cols_sweep_pair<N, false, true, true, true>, ColPairCfg<N>::kSmemBytes);
-      if constexpr (col_pipe_length<N>()) {
-        if (!st) st = prepare_col_pipe<N, false, true, true>();
-      }
+      if (!st) st = prepare_cols_sweep<N, false, true, true>();
       if (!st) st = ensure_smem((const void*)base_cols_reg<kColForward, N>, sm);
       if (!st) st = ensure_smem((const void*)base_cols_reg<kColBackward, N>, sm);
     } else if (const MixOps* mo = mix_ops(ph)) {
@@ -879,21 +875,8 @@ void launch_cols(const BaseGeom& g, int frame0, int nframes, const uint16_t* mea
       using L = RegLaunch<N>;
       if constexpr (MODE == kColSweep) {
         // column DFT, amplitude-loss epilogue and inverse column DFT; counts fftshifted
-        dim3 grid(num_tiles(g.pw), nframes);
-        if constexpr (col_pipe_length<N>()) {
-          if (col_pipe_takes(g.pw, nframes, measured)) {
-            launch_col_pipe<N, false, true, true>(g.scratch, g.pw, nframes, frame0, g.col.tw, measured, scale, 1.0f,
-                                                  grad_scale, inv_numel, loss, g.err, s);
-            return;
-          }
-        }
-        if (g.pw % kTile == 0) {
-          launch_pdl(cols_sweep_pair<N, false, true, true, true>, grid, ColPairCfg<N>::kThreads, ColPairCfg<N>::kSmemBytes, s,
-              g.scratch, g.pw, frame0, g.col.tw, measured, scale, 1.0f, grad_scale, inv_numel, loss);
-        } else {
-          launch_pdl(cols_sweep_pair<N, false, true>, grid, ColPairCfg<N>::kThreads, ColPairCfg<N>::kSmemBytes, s,
-              g.scratch, g.pw, frame0, g.col.tw, measured, scale, 1.0f, grad_scale, inv_numel, loss);
-        }
+        launch_cols_sweep<N, false, true, true>(g.scratch, g.pw, nframes, frame0, g.col.tw, measured, scale, 1.0f,
+                                                grad_scale, inv_numel, loss, g.err, s);
       } else {
         dim3 grid(num_tiles(g.pw) * (kTile / kColsReg), nframes);
         launch_pdl(base_cols_reg<MODE, N>, grid, L::col_threads(), L::col_smem(), s, g.scratch, g.pw, frame0, g.col.tw,

@@ -389,11 +389,7 @@ int fpm_check(const void* object, int oh, int ow, const void* pupil, int lh, int
   });
   dispatch_pow2(lh, [&](auto NT) {
     constexpr int N = decltype(NT)::value;
-    if constexpr (col_pipe_length<N>()) {
-      if (!st) st = prepare_col_pipe<N, true, false, false>();
-    }
-    if (!st) st = ensure_smem((const void*)cols_sweep_pair<N, true, false>, ColPairCfg<N>::kSmemBytes);
-    if (!st) st = ensure_smem((const void*)cols_sweep_pair<N, true, false, false, true>, ColPairCfg<N>::kSmemBytes);
+    if (!st) st = prepare_cols_sweep<N, true, false, false>();
     if (!st) st = ensure_smem((const void*)fpm_cols<kFpmForward, N>, ColPass<N>::kSmemBytes);
     if (!st) st = ensure_smem((const void*)fpm_cols<kFpmBackward, N>, ColPass<N>::kSmemBytes);
   });
@@ -472,21 +468,8 @@ void launch_cols(const FpmGeom& g, int frame0, int nf, const uint16_t* measured,
     constexpr int N = decltype(NT)::value;
     if constexpr (MODE == kFpmSweep) {
       // inverse column DFT, 1/(h w), amplitude-loss epilogue, forward column DFT
-      dim3 grid(num_tiles(g.lw), nf);
-      if constexpr (col_pipe_length<N>()) {
-        if (col_pipe_takes(g.lw, nf, measured)) {
-          launch_col_pipe<N, true, false, false>(g.frames, g.lw, nf, frame0, g.p_lh.tw, measured, scale, norm,
-                                                 grad_scale, inv_numel, loss, g.err, s);
-          return;
-        }
-      }
-      if (g.lw % kTile == 0) {
-        launch_pdl(cols_sweep_pair<N, true, false, false, true>, grid, ColPairCfg<N>::kThreads, ColPairCfg<N>::kSmemBytes, s,
-            g.frames, g.lw, frame0, g.p_lh.tw, measured, scale, norm, grad_scale, inv_numel, loss);
-      } else {
-        launch_pdl(cols_sweep_pair<N, true, false>, grid, ColPairCfg<N>::kThreads, ColPairCfg<N>::kSmemBytes, s,
-            g.frames, g.lw, frame0, g.p_lh.tw, measured, scale, norm, grad_scale, inv_numel, loss);
-      }
+      launch_cols_sweep<N, true, false, false>(g.frames, g.lw, nf, frame0, g.p_lh.tw, measured, scale, norm, grad_scale,
+                                               inv_numel, loss, g.err, s);
     } else {
       dim3 grid(num_tiles(g.lw) * (kTile / kColsPerCta), nf);
       launch_pdl(fpm_cols<MODE, N>, grid, ColPass<N>::kThreads, ColPass<N>::kSmemBytes, s,

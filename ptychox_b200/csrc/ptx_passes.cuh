@@ -253,10 +253,10 @@ constexpr int col_pair_min_blocks() {
   return ColPairCfg<N>::kThreads > 128 ? 1 : (N <= 256 ? 4 : 2);
 }
 
-template <int N, bool FIRST_INV, bool SHIFTED, bool UNIT_NORM = false, bool FULL = false>
+template <int N, bool FIRST_INV, bool SHIFTED, bool UNIT_NORM, bool FULL, bool PLAIN>
 __global__ void __launch_bounds__(ColPairCfg<N>::kThreads, col_pair_min_blocks<N>()) cols_sweep_pair(
     float2* __restrict__ scratch, int width, int frame0, const float2* __restrict__ tw,
-    const uint16_t* __restrict__ measured, CountScale counts, float norm, float grad_scale, double inv_numel,
+    const uint16_t* __restrict__ measured, float scale, float norm, float grad_scale, double inv_numel,
     double* __restrict__ loss) {
   pdl_wait();
   using S = RegShape<N>;
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(ColPairCfg<N>::kThreads, col_pair_min_blocks<N
     const float2 a = mul2(s2, r);
     const float2 inv =
         make_float2(a.x >= kEpsF32 ? r.x : 1.0f / kEpsF32, a.y >= kEpsF32 ? r.y : 1.0f / kEpsF32);
-    float2 rr = minus_amplitudes(a, *reinterpret_cast<const uint32_t*>(meas_s + kr * kTile + 2 * p), counts);
+    float2 rr = minus_amplitudes<PLAIN>(a, *reinterpret_cast<const uint32_t*>(meas_s + kr * kTile + 2 * p), scale);
     rr = make_float2(okA ? rr.x : 0.f, okB ? rr.y : 0.f);
     part = fma2(rr, rr, part);
     const float2 sc = mul2(mul2(gs, rr), inv);
@@ -457,7 +457,7 @@ __device__ __forceinline__ constexpr int pipe_index(int m) {
 template <int N, bool FIRST_INV, bool SHIFTED, bool UNIT_NORM>
 __global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlocks) cols_sweep_pipe(
     float2* __restrict__ scratch, int width, int nframes, int frame0, const float2* __restrict__ tw,
-    const uint16_t* __restrict__ measured, CountScale counts, float norm, float grad_scale, double inv_numel,
+    const uint16_t* __restrict__ measured, float scale, float norm, float grad_scale, double inv_numel,
     double* __restrict__ loss, unsigned* __restrict__ err) {
   using S = RegShape<N>;
   using Cfg = ColPipeCfg<N>;
@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlo
       const float2 a = mul2(s2, r);
       const float2 inv =
           make_float2(a.x >= kEpsF32 ? r.x : 1.0f / kEpsF32, a.y >= kEpsF32 ? r.y : 1.0f / kEpsF32);
-      const float2 rr = minus_amplitudes(a, *reinterpret_cast<const uint32_t*>(meas_s + kr * kTile + 2 * p), counts);
+      const float2 rr = minus_amplitudes<true>(a, *reinterpret_cast<const uint32_t*>(meas_s + kr * kTile + 2 * p), scale);
       part = fma2(rr, rr, part);
       const float2 sc = mul2(mul2(gs, rr), inv);
       g[m] = {mul2(F.re, sc), mul2(F.im, sc)};
@@ -585,8 +585,8 @@ __global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlo
 }
 
 // Column lengths the pipeline is used for, and the frames it takes: whole pairs of tiles (the
-// counts' 16-byte pieces stay inside a tile), counts on a 16-byte boundary, and five tiles or more per
-// CTA.  At 512 points a CTA of cols_sweep_pair leaves no room for the next tile's loads beside it
+// counts' 16-byte pieces stay inside a tile), counts on a 16-byte boundary and of a plain scale, and
+// five tiles or more per CTA.  At 512 points a CTA of cols_sweep_pair leaves no room for the next tile's loads beside it
 // (14400 tiles 1135 us against 1023 here); at 256 several of its CTAs share an SM and it is the faster
 // one (225 frames: 60.5 us against 69.8).  With few tiles per CTA the pipeline's start and end
 // weigh more (whole sweeps, us, pipeline and pair: 180 tiles of 512 x 96 33.3 and 32.5, 600 tiles 81.6 and
@@ -595,24 +595,56 @@ template <int N>
 constexpr bool col_pipe_length() {
   return N == 512;
 }
-inline bool col_pipe_takes(int width, int nframes, const uint16_t* measured) {
-  return width % (2 * kTile) == 0 && (reinterpret_cast<uintptr_t>(measured) & 15) == 0 &&
+inline bool col_pipe_takes(int width, int nframes, const uint16_t* measured, float scale) {
+  return width % (2 * kTile) == 0 && (reinterpret_cast<uintptr_t>(measured) & 15) == 0 && plain_scale(scale) &&
          (long long)(width / kTile) * nframes >= 5LL * sm_count();
 }
+
+// The column pass of a sweep (every power-of-two length), once prepared: the pipeline, or the paired
+// pass in the compilation for whole tiles (UNIT_NORM: a `norm` of 1 is then not applied) or any width,
+// and for the scale.
 template <int N, bool FIRST_INV, bool SHIFTED, bool UNIT_NORM>
-int prepare_col_pipe() {
-  return ensure_smem((const void*)cols_sweep_pipe<N, FIRST_INV, SHIFTED, UNIT_NORM>, ColPipeCfg<N>::kSmemBytes);
+int prepare_cols_sweep() {
+  int st = PTX_OK;
+  if constexpr (col_pipe_length<N>()) {
+    st = ensure_smem((const void*)cols_sweep_pipe<N, FIRST_INV, SHIFTED, UNIT_NORM>, ColPipeCfg<N>::kSmemBytes);
+  }
+  auto pair = [&](auto kern) {
+    if (!st) st = ensure_smem((const void*)kern, ColPairCfg<N>::kSmemBytes);
+  };
+  pair(cols_sweep_pair<N, FIRST_INV, SHIFTED, UNIT_NORM, true, true>);
+  pair(cols_sweep_pair<N, FIRST_INV, SHIFTED, UNIT_NORM, true, false>);
+  pair(cols_sweep_pair<N, FIRST_INV, SHIFTED, false, false, true>);
+  pair(cols_sweep_pair<N, FIRST_INV, SHIFTED, false, false, false>);
+  return st;
 }
 template <int N, bool FIRST_INV, bool SHIFTED, bool UNIT_NORM>
-void launch_col_pipe(float2* frames, int width, int nframes, int frame0, const float2* tw, const uint16_t* measured,
-                     float scale, float norm, float grad_scale, double inv_numel, double* loss, unsigned* err,
-                     cudaStream_t s) {
-  using C = ColPipeCfg<N>;
-  auto kern = cols_sweep_pipe<N, FIRST_INV, SHIFTED, UNIT_NORM>;
-  const int grid =
-      persistent_grid((const void*)kern, 2 * C::kGroup, C::kSmemBytes, (long long)num_tiles(width) * nframes);
-  launch_pdl(kern, grid, 2 * C::kGroup, C::kSmemBytes, s, frames, width, nframes, frame0, tw, measured, scale, norm,
-             grad_scale, inv_numel, loss, err);
+void launch_cols_sweep(float2* frames, int width, int nframes, int frame0, const float2* tw, const uint16_t* measured,
+                       float scale, float norm, float grad_scale, double inv_numel, double* loss, unsigned* err,
+                       cudaStream_t s) {
+  if constexpr (col_pipe_length<N>()) {
+    if (col_pipe_takes(width, nframes, measured, scale)) {
+      using C = ColPipeCfg<N>;
+      auto kern = cols_sweep_pipe<N, FIRST_INV, SHIFTED, UNIT_NORM>;
+      const int grid =
+          persistent_grid((const void*)kern, 2 * C::kGroup, C::kSmemBytes, (long long)num_tiles(width) * nframes);
+      launch_pdl(kern, grid, 2 * C::kGroup, C::kSmemBytes, s, frames, width, nframes, frame0, tw, measured, scale, norm,
+                 grad_scale, inv_numel, loss, err);
+      return;
+    }
+  }
+  auto pair = [&](auto kern) {
+    launch_pdl(kern, dim3(num_tiles(width), nframes), ColPairCfg<N>::kThreads, ColPairCfg<N>::kSmemBytes, s, frames,
+               width, frame0, tw, measured, scale, norm, grad_scale, inv_numel, loss);
+  };
+  const bool full = width % kTile == 0;
+  if (plain_scale(scale)) {
+    full ? pair(cols_sweep_pair<N, FIRST_INV, SHIFTED, UNIT_NORM, true, true>)
+         : pair(cols_sweep_pair<N, FIRST_INV, SHIFTED, false, false, true>);
+  } else {
+    full ? pair(cols_sweep_pair<N, FIRST_INV, SHIFTED, UNIT_NORM, true, false>)
+         : pair(cols_sweep_pair<N, FIRST_INV, SHIFTED, false, false, false>);
+  }
 }
 
 }  // namespace ptx

@@ -465,25 +465,11 @@ int sp_launch_cols_sweep(const SpGeom& g, int frame0, int nf, const uint16_t* me
   dispatch_pow2(g.ph, [&](auto NT) {
     constexpr int N = decltype(NT)::value;
     if constexpr (N >= 16) {
-      if constexpr (col_pipe_length<N>()) {
-        if (col_pipe_takes(g.pw, nf, measured)) {
-          st = prepare_col_pipe<N, false, true, true>();
-          if (st) return;
-          prof_begin(kBaseCols, s);
-          launch_col_pipe<N, false, true, true>(g.scratch, g.pw, nf, frame0, g.col.tw, measured, scale, 1.0f, grad_scale,
-                                                inv_numel, loss, g.err, s);
-          prof_end(kBaseCols, s);
-          return;
-        }
-      }
-      // the full-tile variant needs whole 16-column tiles
-      auto kern = (g.pw % kTile == 0) ? cols_sweep_pair<N, false, true, true, true> : cols_sweep_pair<N, false, true, true>;
-      st = ensure_smem((const void*)kern, ColPairCfg<N>::kSmemBytes);
+      st = prepare_cols_sweep<N, false, true, true>();
       if (st) return;
-      dim3 grid(num_tiles(g.pw), nf);
       prof_begin(kBaseCols, s);
-      launch_pdl(kern, grid, ColPairCfg<N>::kThreads, ColPairCfg<N>::kSmemBytes, s, g.scratch, g.pw, frame0,
-                 g.col.tw, measured, scale, 1.0f, grad_scale, inv_numel, loss);
+      launch_cols_sweep<N, false, true, true>(g.scratch, g.pw, nf, frame0, g.col.tw, measured, scale, 1.0f, grad_scale,
+                                              inv_numel, loss, g.err, s);
       prof_end(kBaseCols, s);
     }
   });

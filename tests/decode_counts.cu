@@ -13,7 +13,7 @@ __global__ void all_mantissas(unsigned long long* bad) {
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;  // 2^24 threads
   const float x = __uint_as_float(0x3f800000u + i);
   const ptx::CountScale s(x);
-  const float2 both = ptx::minus_amplitudes(make_float2(0.f, 0.f), 0x10001u, s);
+  const float2 both = ptx::minus_amplitudes<true>(make_float2(0.f, 0.f), 0x10001u, x);
   const float want = sqrtf(x);
   if (!same(-ptx::minus_amplitude(0.f, 1u, s), want) || !same(-both.x, want) || !same(-both.y, want)) atomicAdd(bad, 1ull);
 }
@@ -23,7 +23,9 @@ __global__ void all_counts(const float* scales, unsigned long long* bad) {
   const float scale = scales[blockIdx.y];
   const ptx::CountScale s(scale);
   const unsigned other = 65535u - c;
-  const float2 both = ptx::minus_amplitudes(make_float2(0.f, 0.f), c | other << 16, s);
+  const float2 zero = make_float2(0.f, 0.f);
+  const float2 both = ptx::plain_scale(scale) ? ptx::minus_amplitudes<true>(zero, c | other << 16, scale)
+                                              : ptx::minus_amplitudes<false>(zero, c | other << 16, scale);
   const float want = sqrtf(static_cast<float>(c) * scale), want2 = sqrtf(static_cast<float>(other) * scale);
   if (!same(-ptx::minus_amplitude(0.f, c, s), want) || !same(-both.x, want) || !same(-both.y, want2)) atomicAdd(bad, 1ull);
   // the difference is rounded once
