@@ -178,7 +178,8 @@ int ptx_base_sweep_small(const float* sample, int sample_h, int sample_w,
  * past the far edge).  This call copies the 4-byte word in stream order on `stream` to
  * `status` (device memory or page-locked host memory: no host synchronisation), so a caller
  * with device-resident positions learns of a bad window without copying the positions to
- * the host.  Read it after the stream has reached the copy and map it with ptx_status_code. */
+ * the host.  Read it after the stream has reached the copy and map it with ptx_status_code.
+ * Bit 1 of the word (base, sub-pixel and Fourier sweeps) is explained at ptx_status_code. */
 int ptx_workspace_status(const void* workspace, unsigned* status, void* stream);
 
 /* The same check deferred and without a host synchronisation: ptx_status_track copies the status

@@ -14,6 +14,9 @@ device tensor of positions every step (``train_ptychography.py:549``) -- three m
 * ``"host"``: the positions are copied to the host and checked before the launch (one
   device-to-host synchronisation per call).
 
+The same word tells of a device wait of the sweep that gave up (bit 1: its loss and gradients are
+NaN), which is raised as ``PtychoXError`` where the call is retired.
+
 Calls made while a stream is being captured into a CUDA graph are not tracked.
 """
 

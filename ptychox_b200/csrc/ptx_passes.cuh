@@ -351,8 +351,9 @@ __global__ void __launch_bounds__(ColPairCfg<N>::kThreads, col_pair_min_blocks<N
 // over three tile buffers.  A whole tile is one contiguous block, so it arrives by one bulk copy
 // (cp.async.bulk, no registers, no load instructions) while both groups transform earlier tiles;
 // the exchanges of a tile's two transforms happen in the same buffer: thread (c, t) of column c
-// writes exactly where it has read (rows t + T j), and a half-warp always covers one 128-byte row.  The buffer takes the next tile as soon as the second exchange has been
-// read, before that transform's last step and the stores.
+// writes exactly where it has read (rows t + T j), and a half-warp always covers one 128-byte row.
+// The buffer takes the next tile as soon as the second exchange has been read, before that
+// transform's last step and the stores.
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
@@ -451,9 +452,10 @@ __device__ __forceinline__ constexpr int pipe_index(int m) {
   return (m % RegShape<N>::C) * RegShape<N>::T + m / RegShape<N>::C;
 }
 
-// Whole tiles only (`width` a multiple of 2 kTile) and counts on a 16-byte boundary.  Bound: the
-// latency of the exchanges and the epilogue at 8 to 16 warps per SM (900 frames of 512^2: 1023 us,
-// of cols_sweep_pair 1135; 825 without the DFT arithmetic, 780 with the frames in L2 as well).
+// Whole tiles only (`width` a multiple of 2 kTile) and counts on a 16-byte boundary.  Bound: at 8
+// warps per SM the transforms, the exchanges and the epilogue overlap only in part, no pipe is above
+// 47% (900 frames of 512^2: 1023 us, cols_sweep_pair 1135; 825 without the DFT arithmetic, 780 with
+// the frames in L2 as well).
 template <int N, bool FIRST_INV, bool SHIFTED, bool UNIT_NORM>
 __global__ void __launch_bounds__(2 * ColPipeCfg<N>::kGroup, ColPipeCfg<N>::kBlocks) cols_sweep_pipe(
     float2* __restrict__ scratch, int width, int nframes, int frame0, const float2* __restrict__ tw,

@@ -405,7 +405,8 @@ __device__ __forceinline__ int unpadded_bin(int c, int n) {
 }
 
 // One pass from the two spectra to the product spec1 conj(spec2), rows zero-padded to 2 cols
-// (what a library's row transform reads; null where the padding is the transform's own), and the cross-power conj(spec1) spec2 the refinement reads.
+// (what a library's row transform reads; null where the padding is the transform's own), and the
+// cross-power conj(spec1) spec2 the refinement reads.
 // HBM-bound: 8 B read (spec1 of a tracked stack is one image, resident in L2), 24 B written.
 __global__ void __launch_bounds__(256) reg_cross_power_kernel(const float2* __restrict__ s1, bool one,
                                                               const float2* __restrict__ s2, int rows, int cols,
